@@ -453,7 +453,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t otc0 = want_tc[0] ? bp.take(tc_tile_bytes(n)) : 0;
         const size_t otc1 = want_tc[1] ? bp.take(tc_tile_bytes(n)) : 0;
         const size_t ow32 = bp.take((size_t)n * sizeof(float));
-        const size_t oaux = bp.take((2 + 2 * (size_t)n) * sizeof(double)); // moments + factorisation scratch
+        const size_t oaux = bp.take(cholesky_aux_len(n) * sizeof(double)); // moments + factorisation scratch
         const size_t oinfo = bp.take(sizeof(int));
         RG_CUDA_TRY(cudaMalloc(&p->d_block, bp.total));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
@@ -498,6 +498,10 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     cudaEventElapsedTime(&p->ms_chol, e0, e1);
     if (info == -1) {
         st = set_error(RG_ERR_INVALID, "mu, weights or Sigma hold a NaN or Inf");
+        goto fail;
+    }
+    if (info == -2) {
+        st = set_error(RG_ERR_TIMEOUT, "the factorisation gave up a bounded wait");
         goto fail;
     }
     if (info != 0) {

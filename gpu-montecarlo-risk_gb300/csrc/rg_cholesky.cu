@@ -5,31 +5,47 @@
 // its flatten step (:96-108, lower triangle kept, upper zeroed).  FP64 is
 // kept for this one step: it is the step whose stability needs it.
 //
-// One CTA factors the matrix left-looking, column by column, in place in
-// the row-major output:
-//   L_jj = sqrt(A_jj - sum_{k<j} L_jk^2)
-//   L_ij = (A_ij - sum_{k<j} L_ik L_jk) / L_jj,   i > j
-// Row j (final once column j-1 is done) is staged in shared memory and read
-// by every thread; thread t owns rows i = j+1+t, j+1+t+blockDim, ...
+// The FP64 pipe of this part takes 64 cycles for a warp instruction on one
+// SM sub-partition (76 with all four busy), whether 32 lanes are active or
+// one, so every form below spreads its FP64 warp instructions over warps and
+// SMs and keeps the chain from one pivot to the next short.
+//
+// N <= 64 (chol_small_kernel): one CTA, right-looking, column by column: one
+//   warp carries the chain from pivot to pivot, six apply the finished columns
+//   to theirs (chol_factor_cta).
+// Above (launch_cholesky_blocked): right-looking over 32-column blocks, two
+//   launches a block:
+//   chol_step   CTA 0 subtracts the previous panel from the next 32 x 32
+//               diagonal block and factors it (the same scheme); the other
+//               CTAs subtract the panel from the rest of the trailing lower
+//               triangle, a 16 x 16 tile each, at the same time;
+//   chol_panel  one warp per row below the block solves x L_kk^T = a with a
+//               lane per column: 32 steps of one shuffle and one FMA, on the
+//               rows of L_kk divided by their pivots.
+//   A 32 x 32 x 32 update is 19.5k cycles of one SM's FP64 pipe, hence the
+//   16 x 16 tiles (N = 600: 663 in the first step), and a row per warp in the
+//   panel (a row per lane put all 32 rows of a CTA on one sub-partition: 28 us
+//   a panel at N = 600, now 9, both under ncu).  The launches overlap their
+//   start-up with the previous kernel's end (programmatic dependent launch).
+//   chol_prep (finite checks, lower(A), w32, per-row moment terms) runs
+//   first, chol_finish (packed FP32 rows, moment sums in a fixed order, so
+//   the result does not depend on scheduling) last.
+// Device time of the factorisation, microseconds, before (the left-looking
+// one-CTA form up to N = 64; above, one warp per diagonal block, a row per
+// lane in the panel, 32 x 32 update tiles) and now:
+//   N        9    20    50    64    65   200   333   600   1000   2000
+//   before  34    65   178   249   188   538   924  1578   2810   7246
+//   now     12    20    49    58    81   223   364   673   1237   3706
+// Both forms cross at N = 64, the widest block whose columns stay in
+// registers (58 us against about 75 us blocked).
+// RG_CHOLESKY=single forces cholesky_kernel, one CTA left-looking column by
+// column in place in the row-major output, above N = 64 too (a second
+// implementation that the tests compare).
+//
 // A pivot that is not > 0 (or not finite) stops the factorisation and
-// records info = j + 1; the host turns that into RG_ERR_NOT_PD.  A
-// non-finite input records info = -1 (RG_ERR_INVALID).
-//
-// The same launch then writes the packed FP32 rows used by the fused
-// counting kernel and the portfolio moments w^T Sigma w and w.mu (FP64).
-//
-// Above kCholSingleMaxN a blocked right-looking form spreads the work over
-// the SMs (one SM's FP64 rate is a small fraction of the part's): for each
-// 32-column block k,
-//   chol_diag    one warp factors the diagonal block in registers,
-//   chol_panel   one thread per row solves L_ik L_kk^T = A_ik below it,
-//   chol_update  one CTA per 32 x 32 tile of the trailing lower triangle
-//                subtracts L_ik L_jk^T,
-// between chol_prep (finite checks, lower(A), w32, per-row moment terms)
-// and chol_finish (packed FP32 rows, moment sums in a fixed order, so the
-// result does not depend on scheduling).  The first pivot that is not > 0
-// (or not finite) records info = column + 1 and every later kernel returns
-// at once.
+// records info = column + 1 (every later kernel returns at once); the host
+// turns that into RG_ERR_NOT_PD.  A non-finite input records info = -1
+// (RG_ERR_INVALID).
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -157,13 +173,298 @@ __global__ void __launch_bounds__(kCholThreads) cholesky_kernel(
     }
 }
 
+static constexpr int kCholNb = 32;          // block size of the blocked form
+static constexpr int kCholSmallMaxN = 64;   // the one-CTA form up to here
+static constexpr int kCholCta = 256;        // threads of the factoring CTA and of chol_step's others
+static constexpr int kCholTimeout = -2;     // info: a bounded wait ran out
+static constexpr int kCholTile = 16;        // trailing-update tile
+static constexpr size_t kCholAlone = 96 * 1024; // dynamic shared memory that, with the static, leaves one CTA an SM
+
+// A positive finite pivot, tested on the bits (no FP64-pipe instruction).
+__device__ __forceinline__ bool good_pivot(double d)
+{
+    const long long b = __double_as_longlong(d);
+    return b > 0ll && b < 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool finite_bits(double v)
+{
+    return (__double_as_longlong(v) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
+}
+
+// 1 / sqrt(d) of a positive finite d: the hardware's approximation y (about
+// 20 bits) and the binomial series of (1 - e)^(-1/2) to its second term with
+// e = 1 - d y^2; the rest, 5/16 e^3, is below FP64's rounding.  Five FP64
+// instructions, four deep, on the chain from pivot to pivot.
+__device__ __forceinline__ double pivot_rsqrt(double d)
+{
+    const int ex = __double2hiint(d) >> 20; // biased exponent
+    if (ex < 64 || ex > 1983) return rsqrt(d); // out of the approximation's range
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-(d * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// The warps that factor a block: the chain warp (0) and six bulk warps (1-3,
+// 5-7).  Warp 4 would share the chain warp's SM sub-partition, and its FP64
+// instructions would queue ahead of the chain's: it does not take part.
+static constexpr int kCholBulk = 6;
+__device__ __forceinline__ bool chol_takes_part() { return (threadIdx.x >> 5) != 4; }
+
+// Hand-over of columns between the warps of the factoring CTA: one mbarrier
+// a column and direction, each used once.
+struct CholFlags {
+    unsigned long long fin[64]; // column final (chain -> bulk)
+    unsigned long long pre[64]; // column up to date but for the one before it (bulk -> chain)
+};
+__device__ __forceinline__ unsigned chol_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void chol_flags_init(CholFlags &f)
+{
+    for (int i = threadIdx.x; i < 64; i += blockDim.x) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(chol_smem(&f.fin[i])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(chol_smem(&f.pre[i])) : "memory");
+    }
+}
+// The whole warp's writes before it are visible to the waiters.
+__device__ __forceinline__ void chol_arrive(unsigned long long *bar)
+{
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(chol_smem(bar)) : "memory");
+}
+// Bounded: false after about a second (the other warps of the CTA are
+// resident, so a wait ends within microseconds unless something is broken).
+__device__ __forceinline__ bool chol_wait(unsigned long long *bar)
+{
+    for (int i = 0; i < (1 << 20); i++) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(chol_smem(bar))
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// Factor an n x n block (n <= NC) in place: col[c NR + row], NR = NC rounded
+// up to 32, lower triangle, zeros above the diagonal; the reciprocal pivots
+// are left in inv[].  Called by the seven warps of a 256-thread CTA that take
+// part, after a barrier that made col and the initialised flags visible and
+// *s_fail zero; another CTA barrier must follow.  *s_fail is then 0, 1 + the
+// first failing column, or -1 (a bounded wait ran out).
+//
+// Right-looking.  The chain warp, once column c - 1 is final and column c has
+// had every column before c - 1 applied, applies column c - 1, forms the pivot
+// and leaves column c final: one FMA, the reciprocal square root and one
+// multiply a column.  The bulk warps (column j in the registers of bulk warp
+// j mod 6, lane = row, two rows a lane for NC > 32) apply each final column c
+// to theirs; the one that owns column c + 2 does that one first, writes it
+// back for the chain warp and catches up with its other columns later
+// (`done`: columns applied so far).  Hand-over by column instead of a CTA
+// barrier a column lets a bulk warp fall behind while the chain goes on.
+template <int NC>
+__device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv, CholFlags &f, int *s_fail)
+{
+    constexpr int SL = (NC + kCholBulk - 1) / kCholBulk, G = (NC + 31) / 32, NR = 32 * G;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int *failed = s_fail;
+    if (warp == 0) {
+        double p[G]; // the previous column
+#pragma unroll
+        for (int g = 0; g < G; g++) p[g] = 0.0;
+        int c = 0;
+        for (; c < n; c++) {
+            if (c >= 2 && !chol_wait(&f.pre[c])) {
+                if (lane == 0) *failed = -1;
+                break;
+            }
+            double v[G];
+            const double l = c > 0 ? -col[(c - 1) * NR + c] : 0.0;
+#pragma unroll
+            for (int g = 0; g < G; g++) v[g] = fma(p[g], l, col[c * NR + 32 * g + lane]);
+            const double d = __shfl_sync(0xffffffffu, c >= 32 ? v[G - 1] : v[0], c & 31);
+            if (!good_pivot(d)) { // the same value in every lane
+                if (lane == 0) *failed = c + 1;
+                break;
+            }
+            const double rs = pivot_rsqrt(d);
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                p[g] = 32 * g + lane >= c ? v[g] * rs : 0.0; // on the diagonal d / sqrt(d)
+                col[c * NR + 32 * g + lane] = p[g];
+            }
+            if (lane == 0) inv[c] = rs;
+            chol_arrive(&f.fin[c]);
+        }
+        // after a failure: release the bulk warps from the columns not
+        // published (each flag is arrived on once)
+        for (; c < n; c++) chol_arrive(&f.fin[c]);
+        return;
+    }
+    const int b = warp < 4 ? warp - 1 : warp - 2; // bulk index
+    double a[SL][G];
+#pragma unroll
+    for (int s = 0; s < SL; s++)
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            const int j = s * kCholBulk + b;
+            a[s][g] = j < n ? col[j * NR + 32 * g + lane] : 0.0;
+        }
+    int done = 0;
+    // Unrolled over the slots so that finished columns cost nothing: an FP64
+    // instruction whose predicate is false still takes its 64 cycles.
+#pragma unroll
+    for (int s0 = 0; s0 < SL; s0++) {
+        for (int c = s0 * kCholBulk; c < (s0 + 1) * kCholBulk && c + 2 < n; c++) {
+            if (!chol_wait(&f.fin[c])) {
+                if (lane == 0) *failed = -1;
+                return;
+            }
+            if (*failed != 0) return;
+            if (b == (c + 2) % kCholBulk) {
+                // the owned column by masks: an index known only at run time
+                // would move the array to local memory
+                double v[G];
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    long long bits = 0;
+#pragma unroll
+                    for (int s = s0; s < SL; s++)
+                        bits |= __double_as_longlong(a[s][g]) & -(long long)(s == (c + 2) / kCholBulk);
+                    v[g] = __longlong_as_double(bits);
+                }
+                for (int k = done; k <= c; k++) {
+                    const double l = -col[k * NR + c + 2];
+#pragma unroll
+                    for (int g = 0; g < G; g++) v[g] = fma(col[k * NR + 32 * g + lane], l, v[g]);
+                }
+#pragma unroll
+                for (int g = 0; g < G; g++) col[(c + 2) * NR + 32 * g + lane] = v[g];
+                chol_arrive(&f.pre[c + 2]);
+                continue;
+            }
+            for (int k = done; k <= c; k++) {
+                const double *ck = col + k * NR;
+                double lr[G];
+#pragma unroll
+                for (int g = 0; g < G; g++) lr[g] = ck[32 * g + lane];
+#pragma unroll
+                for (int s = s0; s < SL; s++) {
+                    const int j = s * kCholBulk + b;
+                    const double l = -ck[j < NR ? j : 0];
+                    // rows above the column's own 32-row group hold nothing
+#pragma unroll
+                    for (int g = 0; g < G; g++)
+                        if (g >= s * kCholBulk / 32) a[s][g] = fma(lr[g], l, a[s][g]);
+                }
+            }
+            done = c + 1;
+        }
+    }
+}
+
+// N <= 64: everything in one CTA (NC = 32 or 64).
+template <int NC>
+__global__ void __launch_bounds__(kCholCta, 1) chol_small_kernel(
+    const double *__restrict__ A, long long lda, int n, const double *__restrict__ w,
+    const double *__restrict__ mu, double *__restrict__ L, float *__restrict__ Lp,
+    float *__restrict__ w32, double *__restrict__ aux, int *__restrict__ info)
+{
+    constexpr int G = (NC + 31) / 32, NR = 32 * G, kW = kCholCta / 32, SEG = kW / G;
+    __shared__ double col[NC * NR];
+    __shared__ double sw[NR], smu[NR], inv[NC], part[SEG][NR];
+    __shared__ CholFlags flags;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, bs = blockDim.x, warp = tid >> 5, lane = tid & 31;
+
+    int bad = 0;
+    for (int idx = tid; idx < NR * NC; idx += bs) {
+        const int i = idx / NC, j = idx % NC;
+        const double v = (i < n && j <= i) ? A[(long long)i * lda + j] : 0.0;
+        if (!finite_bits(v)) bad = 1;
+        col[j * NR + i] = v;
+    }
+    chol_flags_init(flags);
+    if (tid == 0) s_fail = 0;
+    for (int i = tid; i < NR; i += bs) {
+        const double wi = (w != nullptr && i < n) ? w[i] : 0.0, mi = i < n ? mu[i] : 0.0;
+        if (!finite_bits(wi) || !finite_bits(mi)) bad = 1;
+        sw[i] = wi;
+        smu[i] = mi;
+        if (i < n) w32[i] = (float)wi;
+    }
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) *info = -1;
+        return;
+    }
+    if (chol_takes_part()) chol_factor_cta<NC>(n, col, inv, flags, &s_fail);
+    __syncthreads();
+    if (tid == 0) *info = s_fail < 0 ? kCholTimeout : s_fail;
+    if (s_fail) return;
+
+    // L (zero upper) and the packed FP32 rows
+    for (int idx = tid; idx < n * n; idx += bs) {
+        const int i = idx / n, j = idx % n;
+        L[idx] = j <= i ? col[j * NR + i] : 0.0;
+    }
+    for (int i = warp; i < n; i += kW) {
+        const int off = packed_row_offset(i), len = 4 * (i / 4 + 1);
+        for (int j = lane; j < len; j += 32) Lp[off + j] = j <= i ? (float)col[j * NR + i] : 0.f;
+    }
+    // w^T Sigma w (the strict lower triangle counts twice) and w.mu: lane =
+    // row, a segment of its columns per warp
+    if (w != nullptr) {
+        constexpr int W = NR / SEG;
+        const int i = 32 * (warp % G) + lane, seg = warp / G;
+        double t = 0.0;
+        for (int j = seg * W; j < (seg + 1) * W && j < n; j++)
+            t = fma((i < n && j < i) ? A[(long long)i * lda + j] : 0.0, sw[j], t);
+        part[seg][i] = 2.0 * t;
+        __syncthreads();
+        if (warp == 0) {
+            double x = 0.0, y = 0.0;
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                const int r = 32 * g + lane;
+                double u = r < n ? A[(long long)r * lda + r] * sw[r] : 0.0;
+#pragma unroll
+                for (int q = 0; q < SEG; q++) u += part[q][r];
+                x = fma(sw[r], u, x);
+                y = fma(sw[r], smu[r], y);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                x += __shfl_xor_sync(0xffffffffu, x, o);
+                y += __shfl_xor_sync(0xffffffffu, y, o);
+            }
+            if (lane == 0) {
+                aux[0] = x;
+                aux[1] = y;
+            }
+        }
+    } else if (tid == 0) {
+        aux[0] = 0.0;
+        aux[1] = 0.0;
+    }
+}
+
 // ------------------------------------------------------------ blocked form
-static constexpr int kCholNb = 32;          // block size (one warp per diagonal block)
-static constexpr int kCholSingleMaxN = 64;  // the single-CTA form up to here
+// Start of a kernel launched programmatically behind the previous one: let
+// the next one be scheduled, then wait until the previous one's writes are
+// visible.
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Checks, L <- lower(A) (upper zeroed), w32, and the per-row moment terms
-// aux[2 + i] = w_i sum_j Sigma_ij w_j, aux[2 + n + i] = w_i mu_i.  One warp
-// per row.
+// aux[2 + i] = w_i (2 sum_{j<i} Sigma_ij w_j + Sigma_ii w_i),
+// aux[2 + n + i] = w_i mu_i.  One warp per row (only the lower triangle is
+// read: coalesced).
 __global__ void chol_prep_kernel(const double *__restrict__ A, long long lda, int n, const double *__restrict__ w,
                                  const double *__restrict__ mu, double *__restrict__ L, float *__restrict__ w32,
                                  double *__restrict__ aux, int *__restrict__ info)
@@ -174,130 +475,154 @@ __global__ void chol_prep_kernel(const double *__restrict__ A, long long lda, in
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
         const double *ai = A + (long long)i * lda;
         double part = 0.0;
-        for (int j = lane; j < n; j += 32) {
-            const double a = (j <= i) ? ai[j] : A[(long long)j * lda + i];
-            if (j <= i && !isfinite(a)) bad = 1;
-            L[(long long)i * n + j] = (j <= i) ? a : 0.0;
-            if (w != nullptr) part += a * w[j];
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const int j = j0 + lane;
+            const double a = j <= i ? ai[j] : 0.0;
+            if (!finite_bits(a)) bad = 1;
+            if (j < n) L[(long long)i * n + j] = a;
+            if (w != nullptr && j0 <= i) part = fma(a, j < i ? w[j] : 0.0, part);
         }
+        double wi = 0.0, mi = 0.0;
+        if (w != nullptr) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+            wi = w[i];
+        }
+        mi = mu[i];
+        if (!finite_bits(wi) || !finite_bits(mi)) bad = 1;
         if (lane == 0) {
-            if (!isfinite(mu[i]) || (w != nullptr && !isfinite(w[i]))) bad = 1;
-            w32[i] = (w != nullptr) ? (float)w[i] : 0.f;
-            aux[2 + i] = (w != nullptr) ? w[i] * part : 0.0;
-            aux[2 + n + i] = (w != nullptr) ? w[i] * mu[i] : 0.0;
+            w32[i] = (float)wi;
+            aux[2 + i] = (w != nullptr) ? wi * fma(2.0, part, ai[i] * wi) : 0.0;
+            aux[2 + n + i] = (w != nullptr) ? wi * mi : 0.0;
         }
     }
     if (bad) atomicExch(info, -1);
 }
 
-// Factor the diagonal block at k0 (kb <= 32 columns) with one warp; lane r
-// holds row r of the block in registers (fully unrolled), and column values
-// move between lanes by shuffles.  Right-looking: after column c is scaled,
-// lane r subtracts L_rc L_jc from its entries j in (c, r].
-__global__ void chol_diag_kernel(double *__restrict__ L, int n, int k0, int kb, int *__restrict__ info)
+// The previous panel (columns k0 .. k0 + kb - 1, kb = 0 before the first
+// block) applied to the trailing lower triangle, whose first row is
+// r0 = k0 + kb; CTA 0 then factors the 32 x 32 diagonal block at r0 and
+// leaves its reciprocal pivots in dinv.
+__global__ void __launch_bounds__(kCholCta) chol_step_kernel(double *__restrict__ L, int n, int k0, int kb,
+                                                                    double *__restrict__ dinv, int *__restrict__ info)
 {
-    if (*info != 0) return;
-    const int r = threadIdx.x;
-    double a[kCholNb];
-#pragma unroll
-    for (int c = 0; c < kCholNb; c++) a[c] = (r < kb && c <= r) ? L[(long long)(k0 + r) * n + k0 + c] : 0.0;
-#pragma unroll
-    for (int c = 0; c < kCholNb; c++) {
-        if (c < kb) {
-            const double d = __shfl_sync(0xffffffffu, a[c], c); // the same value in every lane: uniform branch
-            if (!(d > 0.0) || !isfinite(d)) {
-                if (r == 0) *info = k0 + c + 1;
-                return;
-            }
-            // one FP64 reciprocal square root per column instead of a square
-            // root and a division: both are long FP64 sequences on this part
-            const double rs = rsqrt(d);
-            if (r == c) a[c] = d * rs;
-            if (r > c) a[c] = a[c] * rs;
-#pragma unroll
-            for (int j = c + 1; j < kCholNb; j++) {
-                const double ljc = __shfl_sync(0xffffffffu, a[c], j);
-                if (r >= j) a[j] = fma(-a[c], ljc, a[j]);
-            }
-        }
-    }
-    if (r < kb) {
-#pragma unroll
-        for (int c = 0; c < kCholNb; c++)
-            if (c <= r) L[(long long)(k0 + r) * n + k0 + c] = a[c];
-    }
-}
-
-// Rows below the diagonal block: x L_kk^T = a, one thread per row (32 per
-// CTA).  The dot products use four partial sums, so the dependent chain is a
-// quarter as long.
-__global__ void chol_panel_kernel(double *__restrict__ L, int n, int k0, int kb, const int *__restrict__ info)
-{
-    if (*info != 0) return;
-    __shared__ double lkk[kCholNb][kCholNb + 1];
+    __shared__ double P[kCholNb][kCholNb + 1];
+    __shared__ double col[kCholNb * kCholNb];
+    __shared__ double T[kCholTile][kCholNb + 1];
     __shared__ double inv[kCholNb];
-    const int t = threadIdx.x;
-    for (int c = 0; c < kCholNb; c++)
-        lkk[t][c] = (t < kb && c <= t) ? L[(long long)(k0 + t) * n + k0 + c] : 0.0;
-    inv[t] = (t < kb) ? 1.0 / L[(long long)(k0 + t) * n + k0 + t] : 0.0; // one division per CTA lane
-    __syncwarp();
-    const int i = k0 + kb + blockIdx.x * kCholNb + t;
-    if (i >= n) return;
-    double *row = L + (long long)i * n + k0;
-    double x[kCholNb];
-#pragma unroll
-    for (int c = 0; c < kCholNb; c++) {
-        if (c < kb) {
-            double s0 = row[c], s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll
-            for (int m = 0; m < c; m++) {
-                const double p = x[m] * lkk[c][m];
-                if ((m & 3) == 0) s0 -= p;
-                else if ((m & 3) == 1) s1 -= p;
-                else if ((m & 3) == 2) s2 -= p;
-                else s3 -= p;
-            }
-            x[c] = ((s0 + s1) + (s2 + s3)) * inv[c];
-            row[c] = x[c];
-        } else {
-            x[c] = 0.0;
-        }
+    __shared__ CholFlags flags;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r0 = k0 + kb;
+    if (blockIdx.x == 0) {
+        chol_flags_init(flags);
+        if (tid == 0) s_fail = 0;
     }
-}
-
-// Trailing update: tile (bi, bj), bj <= bi, of the blocks after k0 + kb:
-// L_ij -= L_ik L_jk^T (lower triangle only on diagonal tiles).
-__global__ void __launch_bounds__(256) chol_update_kernel(double *__restrict__ L, int n, int k0, int kb,
-                                                          const int *__restrict__ info)
-{
+    pdl_enter();
     if (*info != 0) return;
-    __shared__ double P[kCholNb][kCholNb + 1], Q[kCholNb][kCholNb + 1];
-    // blockIdx.x -> (bi, bj) over the lower triangle of tiles, row by row
-    const int t = blockIdx.x;
-    int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f); // then corrected exactly
-    while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
-    while (bi * (bi + 1) / 2 > t) bi--;
-    const int bj = t - bi * (bi + 1) / 2;
-    const int r0 = k0 + kb + bi * kCholNb, c0 = k0 + kb + bj * kCholNb;
-    for (int e = threadIdx.x; e < kCholNb * kCholNb; e += blockDim.x) {
+
+    if (blockIdx.x > 0) {
+        // one 16 x 16 tile (bi, bj), bj <= bi, of the trailing triangle, row
+        // by row; tiles 0..2 are the diagonal block's
+        const int t = (int)blockIdx.x + 2;
+        int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f); // then corrected exactly
+        while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
+        while (bi * (bi + 1) / 2 > t) bi--;
+        const int bj = t - bi * (bi + 1) / 2;
+        const int i0 = r0 + bi * kCholTile, c0 = r0 + bj * kCholTile;
+        // kb == 32 here: a shorter block is the last and has no trailing rows
+        for (int e = tid; e < kCholTile * kCholNb; e += blockDim.x) {
+            const int r = e / kCholNb, m = e % kCholNb;
+            P[r][m] = (i0 + r < n) ? L[(long long)(i0 + r) * n + k0 + m] : 0.0;
+            T[r][m] = (c0 + r < n) ? L[(long long)(c0 + r) * n + k0 + m] : 0.0;
+        }
+        const int r = tid >> 4, c = tid & 15, gi = i0 + r, gj = c0 + c;
+        const bool live = gi < n && gj <= gi;
+        const double old = live ? L[(long long)gi * n + gj] : 0.0;
+        __syncthreads();
+        double v = 0.0;
+#pragma unroll
+        for (int m = 0; m < kCholNb; m++) v = fma(P[r][m], T[c][m], v);
+        if (live) L[(long long)gi * n + gj] = old - v;
+        return;
+    }
+
+    const int nb = min(kCholNb, n - r0);
+    for (int e = tid; e < kCholNb * kCholNb; e += blockDim.x) {
         const int r = e / kCholNb, m = e % kCholNb;
-        P[r][m] = (r0 + r < n && m < kb) ? L[(long long)(r0 + r) * n + k0 + m] : 0.0;
-        Q[r][m] = (c0 + r < n && m < kb) ? L[(long long)(c0 + r) * n + k0 + m] : 0.0;
+        const bool in = r < nb;
+        P[r][m] = (in && m < kb) ? L[(long long)(r0 + r) * n + k0 + m] : 0.0;
+        col[m * kCholNb + r] = (in && m <= r) ? L[(long long)(r0 + r) * n + r0 + m] : 0.0;
     }
     __syncthreads();
-    const int r = threadIdx.x >> 3, cb = (threadIdx.x & 7) * 4;
-    const int gi = r0 + r;
-    if (gi >= n) return;
+    if (kb > 0) {
+        // lower triangle of P P^T in 17 full-width units: unit u holds column
+        // u (rows u..31) and, in the lanes left over, column 32 - u (rows
+        // 32-u..31): half the warp FMAs of the full square
+        int row[3], cc[3];
+        double v[3] = {0.0, 0.0, 0.0};
+        constexpr int kW = kCholCta / 32;
+        const int units = warp == 0 ? 3 : 2;
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int c = cb + u, gj = c0 + c;
-        if (gj >= n || gj > gi) continue;
-        double v = 0.0;
-        for (int m = 0; m < kb; m++) v = fma(P[r][m], Q[c][m], v);
-        L[(long long)gi * n + gj] -= v;
+        for (int q = 0; q < 3; q++) {
+            const int u = warp + kW * q;
+            row[q] = lane < 32 - u ? u + lane : lane;
+            cc[q] = lane < 32 - u ? u : 32 - u;
+            if (q == 2 && warp != 0) row[q] = cc[q] = 0;
+        }
+#pragma unroll 4
+        for (int m = 0; m < kCholNb; m++) {
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                if (q < units) v[q] = fma(P[row[q]][m], P[cc[q]][m], v[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            if (q < units && (q < 2 || lane < 16)) col[cc[q] * kCholNb + row[q]] -= v[q];
+        __syncthreads();
     }
+    if (chol_takes_part()) chol_factor_cta<kCholNb>(nb, col, inv, flags, &s_fail);
+    __syncthreads();
+    if (s_fail) {
+        if (tid == 0) *info = s_fail < 0 ? kCholTimeout : r0 + s_fail;
+        return;
+    }
+    for (int e = tid; e < kCholNb * kCholNb; e += blockDim.x) {
+        const int r = e / kCholNb, m = e % kCholNb;
+        if (r < nb && m <= r) L[(long long)(r0 + r) * n + r0 + m] = col[m * kCholNb + r];
+    }
+    if (tid < nb) dinv[tid] = inv[tid];
+}
+
+// Rows below the diagonal block at k0 (32 columns): x L_kk^T = a, one warp
+// per row, lane j holding column j.  With l'_jc = l_jc / l_jj and
+// s_j = a_j / l_jj the solve is s_j -= x_c l'_jc for c < j, x_j = s_j: one
+// shuffle and one FMA a step.
+static constexpr int kPanelWarps = 4;
+__global__ void __launch_bounds__(32 * kPanelWarps) chol_panel_kernel(double *__restrict__ L, int n, int k0,
+                                                                      const double *__restrict__ dinv,
+                                                                      const int *__restrict__ info)
+{
+    __shared__ double lp[kCholNb][kCholNb + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    pdl_enter();
+    if (*info != 0) return;
+    const double di = dinv[lane];
+    for (int j = warp; j < kCholNb; j += kPanelWarps) {
+        const double dj = __shfl_sync(0xffffffffu, di, j);
+        lp[j][lane] = lane < j ? L[(long long)(k0 + j) * n + k0 + lane] * dj : 0.0;
+    }
+    const int i = k0 + kCholNb + (int)blockIdx.x * kPanelWarps + warp;
+    double s = i < n ? L[(long long)i * n + k0 + lane] * di : 0.0;
+    __syncthreads();
+    if (i >= n) return;
+#pragma unroll
+    for (int c = 0; c < kCholNb - 1; c++) {
+        const double x = __shfl_sync(0xffffffffu, s, c);
+        const double t = fma(-x, lp[lane][c], s);
+        s = lane > c ? t : s;
+    }
+    L[(long long)i * n + k0 + lane] = s;
 }
 
 // Packed FP32 rows, and the moment sums in a fixed order (one CTA reduces).
@@ -305,6 +630,7 @@ __global__ void chol_finish_kernel(const double *__restrict__ L, int n, float *_
                                    double *__restrict__ aux, const int *__restrict__ info)
 {
     __shared__ double red[33];
+    pdl_enter();
     if (*info != 0) return;
     // one warp per row
     const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
@@ -327,31 +653,60 @@ __global__ void chol_finish_kernel(const double *__restrict__ L, int n, float *_
     }
 }
 
+// Launch behind the kernel before it in the stream, without waiting for that
+// one to drain (the kernels wait in pdl_enter).
+template <class... P, class... A>
+static cudaError_t launch_pdl(void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// aux: 2 moments, then 2 n per-row terms, then 32 reciprocal pivots.
 static cudaError_t launch_cholesky_blocked(const double *A, long long lda, int n, const double *w,
                                            const double *mu, double *L64, float *Lp, float *w32,
                                            double *aux, int *info, cudaStream_t s)
 {
     cudaError_t e = cudaMemsetAsync(info, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
+    double *dinv = aux + 2 + 2 * (size_t)n;
+    e = cudaFuncSetAttribute(chol_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCholAlone);
+    if (e != cudaSuccess) return e;
     chol_prep_kernel<<<(n + 7) / 8, 256, 0, s>>>(A, lda, n, w, mu, L64, w32, aux, info);
-    for (int k0 = 0; k0 < n; k0 += kCholNb) {
-        const int kb = (n - k0 < kCholNb) ? n - k0 : kCholNb;
-        chol_diag_kernel<<<1, kCholNb, 0, s>>>(L64, n, k0, kb, info);
+    e = cudaGetLastError();
+    for (int k0 = 0, kb = 0; e == cudaSuccess && k0 + kb < n;) {
+        const int r0 = k0 + kb, nt = (n - r0 + kCholTile - 1) / kCholTile;
+        const int tiles = (kb > 0 && nt > 2) ? nt * (nt + 1) / 2 - 3 : 0;
+        // While the factoring CTA is the longest, it keeps its SM's FP64 pipe
+        // to itself (shared memory for one CTA an SM); with more than about
+        // six tiles an SM the trailing update is, and packs the SMs.
+        const size_t alone = tiles <= 6 * 152 ? kCholAlone : 0;
+        e = launch_pdl(chol_step_kernel, 1 + tiles, kCholCta, alone, s, L64, n, k0, kb, dinv, info);
+        k0 = r0;
+        kb = n - r0 < kCholNb ? n - r0 : kCholNb;
         const int rest = n - k0 - kb;
-        if (rest > 0) {
-            const int mb = (rest + kCholNb - 1) / kCholNb;
-            chol_panel_kernel<<<mb, kCholNb, 0, s>>>(L64, n, k0, kb, info);
-            chol_update_kernel<<<mb * (mb + 1) / 2, 256, 0, s>>>(L64, n, k0, kb, info);
-        }
+        if (e == cudaSuccess && rest > 0)
+            e = launch_pdl(chol_panel_kernel, (rest + kPanelWarps - 1) / kPanelWarps, 32 * kPanelWarps, 0, s, L64, n, k0,
+                           (const double *)dinv, (const int *)info);
     }
-    chol_finish_kernel<<<(n + 7) / 8, 256, 0, s>>>(L64, n, Lp, aux, info);
-    return cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_pdl(chol_finish_kernel, (n + 7) / 8, 256, 0, s, (const double *)L64, n, Lp, aux, (const int *)info);
 }
 
 int cholesky_max_n() { return kCholMaxN; }
 
-// Scratch: aux holds 2 + 2 n doubles (the moments, then the blocked form's
-// per-row terms).
+// aux holds cholesky_aux_len(n) doubles: the two moments, then scratch.
+size_t cholesky_aux_len(int n) { return 2 + 2 * (size_t)n + kCholNb; }
+
 cudaError_t launch_cholesky(const double *A, long long lda, int n, const double *w,
                             const double *mu, double *L64, float *Lp, float *w32, double *aux,
                             int *info, cudaStream_t s)
@@ -359,10 +714,17 @@ cudaError_t launch_cholesky(const double *A, long long lda, int n, const double 
     if (n > kCholMaxN) return cudaErrorInvalidValue;
     // RG_CHOLESKY=single|blocked overrides the size rule (for tests)
     const char *sel = getenv("RG_CHOLESKY");
-    bool blocked = n > kCholSingleMaxN;
+    bool blocked = n > kCholSmallMaxN;
     if (sel && strstr(sel, "single")) blocked = false;
     if (sel && strstr(sel, "blocked")) blocked = true;
     if (blocked) return launch_cholesky_blocked(A, lda, n, w, mu, L64, Lp, w32, aux, info, s);
+    if (n <= kCholSmallMaxN) {
+        // NC in steps of 16: columns between n and NC cost their multiply-adds
+        auto kern = n <= 16 ? chol_small_kernel<16> : n <= 32 ? chol_small_kernel<32> : n <= 48 ? chol_small_kernel<48>
+                                                                                               : chol_small_kernel<64>;
+        kern<<<1, kCholCta, 0, s>>>(A, lda, n, w, mu, L64, Lp, w32, aux, info);
+        return cudaGetLastError();
+    }
     const size_t smem = sizeof(double) * (size_t)(n > 0 ? n : 1);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(cholesky_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

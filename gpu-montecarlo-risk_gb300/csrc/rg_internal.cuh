@@ -149,7 +149,7 @@ struct Portfolio {
     unsigned char *d_tc[2] = {nullptr, nullptr}; // tensor-core tiles (FP16, BF16), N <= tc_max_n()
     unsigned int *d_err = nullptr; // error word of the tensor-core kernel
     float *d_w32 = nullptr;    // n (zeros when no weights)
-    double *d_aux = nullptr;   // [2 + 2n]: w^T Sigma w, w.mu, then factorisation scratch
+    double *d_aux = nullptr;   // [cholesky_aux_len(n)]: w^T Sigma w, w.mu, then factorisation scratch
     int *d_info = nullptr;
     double wsw = 0.0, wmu = 0.0;
     float ms_chol = 0.f;
@@ -243,6 +243,7 @@ cudaError_t launch_cholesky(const double *A, long long lda, int n, const double 
                             const double *mu, double *L64, float *Lp, float *w32, double *aux,
                             int *info, cudaStream_t s);
 int cholesky_max_n();
+size_t cholesky_aux_len(int n);
 
 // Error helpers (rg_capi.cu).
 int set_error(int status, const char *fmt, ...);
