@@ -453,7 +453,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t otc0 = want_tc[0] ? bp.take(tc_tile_bytes(n)) : 0;
         const size_t otc1 = want_tc[1] ? bp.take(tc_tile_bytes(n)) : 0;
         const size_t ow32 = bp.take((size_t)n * sizeof(float));
-        const size_t oaux = bp.take(cholesky_aux_len(n) * sizeof(double)); // moments + factorisation scratch
+        const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
         RG_CUDA_TRY(cudaMalloc(&p->d_block, bp.total));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
@@ -511,8 +511,8 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     p->wsw = aux[0];
     p->wmu = aux[1];
     if (p->d_Lt) RG_CUDA_TRY(launch_build_lt(p->d_L64, n, p->d_Lt, s));
-    if (p->d_tc[0]) RG_CUDA_TRY(launch_build_tc_tiles(p->d_L64, p->d_w32, n, 0, p->d_tc[0], s));
-    if (p->d_tc[1]) RG_CUDA_TRY(launch_build_tc_tiles(p->d_L64, p->d_w32, n, 1, p->d_tc[1], s));
+    if (p->d_tc[0] || p->d_tc[1])
+        RG_CUDA_TRY(launch_build_tc_tiles(p->d_L64, p->d_w32, n, p->d_aux + cholesky_aux_len(n), p->d_tc[0], p->d_tc[1], s));
     RG_CUDA_TRY(cudaMemsetAsync(p->d_err, 0, sizeof(unsigned int), s));
     // host copies for the kernels that take the factor by value: the packed
     // rows from the device; mu and the FP32 weights from the caller's host

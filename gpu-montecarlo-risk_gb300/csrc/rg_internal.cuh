@@ -149,7 +149,7 @@ struct Portfolio {
     unsigned char *d_tc[2] = {nullptr, nullptr}; // tensor-core tiles (FP16, BF16), N <= tc_max_n()
     unsigned int *d_err = nullptr; // error word of the tensor-core kernel
     float *d_w32 = nullptr;    // n (zeros when no weights)
-    double *d_aux = nullptr;   // [cholesky_aux_len(n)]: w^T Sigma w, w.mu, then factorisation scratch
+    double *d_aux = nullptr;   // w^T Sigma w, w.mu, then scratch of the factorisation and the tile build
     int *d_info = nullptr;
     double wsw = 0.0, wmu = 0.0;
     float ms_chol = 0.f;
@@ -215,8 +215,10 @@ int tiled_kpad(int n);
 // rg_mc_tc.cu: tcgen05 precision form (Philox layout), N <= tc_max_n().
 cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, bool aggregated, double wmu,
                       unsigned int *err, bool inject_stall, int sm_count, cudaStream_t s);
-cudaError_t launch_build_tc_tiles(const double *L64, const float *w32, int n, int bf16, unsigned char *tiles,
-                                  cudaStream_t s);
+// the tensor tiles of either split (null: not wanted); scratch: tc_scratch_len(n) doubles
+cudaError_t launch_build_tc_tiles(const double *L64, const float *w32, int n, double *scratch, unsigned char *fp16,
+                                  unsigned char *bf16, cudaStream_t s);
+size_t tc_scratch_len(int n);
 int tc_max_n();
 size_t tc_tile_bytes(int n);
 // batches of (portfolio, query) items in one persistent launch

@@ -1180,10 +1180,34 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     if (VAR) cta_flush(a, 0, 0, n_tail, tail_fx, sacc, nullptr, true);
 }
 
+// Row segment blockIdx.y's part of w^T L for 32 columns (lane = column, rows
+// dealt to the CTA's 8 warps, their sums added in warp order):
+// part[segment][column].  w^T L summed by the one thread that wrote each of
+// its elements was a chain of N dependent FP64 multiply-adds (64 cycles
+// each): 152 us a tile build at N = 600, now 6 + 5 (both under ncu).
+static constexpr int kWtlSegs = 8;
+__global__ void __launch_bounds__(256) wtl_kernel(const double *__restrict__ L, const float *__restrict__ w, int n,
+                                                  double *__restrict__ part)
+{
+    __shared__ double red[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x * 32 + lane;
+    const int per = (n + kWtlSegs - 1) / kWtlSegs, i0 = blockIdx.y * per, i1 = min(n, i0 + per);
+    double v = 0.0;
+    for (int i = i0 + warp; i < i1; i += 8)
+        if (c <= i) v = fma((double)w[i], L[(long long)i * n + c], v);
+    red[warp][lane] = v;
+    __syncthreads();
+    if (warp == 0 && c < n) {
+        for (int q = 1; q < 8; q++) v += red[q][lane];
+        part[(size_t)blockIdx.y * n + c] = v;
+    }
+}
+
 // Pre-swizzled Lhat tiles: rows 0..N-1 = L (lower triangle), row N = w^T L,
 // scaled by 2^8, split into hi and lo (FP16 or BF16), each (row tile, K tile)
 // block laid out exactly as the kernel's shared memory expects.
-__global__ void build_tc_tiles_kernel(const double *L, const float *w, int n, int n_mt, int n_kt, int bf16,
+__global__ void build_tc_tiles_kernel(const double *L, const double *wtl, int n, int n_mt, int n_kt, int bf16,
                                       unsigned char *tiles)
 {
     const long long total = (long long)n_mt * kTcRows * n_kt * kTcKt;
@@ -1196,7 +1220,7 @@ __global__ void build_tc_tiles_kernel(const double *L, const float *w, int n, in
             if (row < n) {
                 if (col <= row) v = L[(long long)row * n + col];
             } else if (row == n) {
-                for (int i = col; i < n; i++) v += (double)w[i] * L[(long long)i * n + col];
+                for (int q = 0; q < kWtlSegs; q++) v += wtl[(size_t)q * n + col];
             }
         }
         const float f = (float)(v * kTcLScale);
@@ -1224,10 +1248,15 @@ static int tc_row_tiles(int n) { return (n + 1 + kTcRows - 1) / kTcRows; }
 static int tc_k_tiles(int n) { return (n + kTcKt - 1) / kTcKt; }
 size_t tc_tile_bytes(int n) { return (size_t)tc_row_tiles(n) * tc_k_tiles(n) * 2 * kTcTileBytes; }
 
-cudaError_t launch_build_tc_tiles(const double *L64, const float *w32, int n, int bf16, unsigned char *tiles,
-                                  cudaStream_t s)
+size_t tc_scratch_len(int n) { return (size_t)kWtlSegs * n; }
+
+cudaError_t launch_build_tc_tiles(const double *L64, const float *w32, int n, double *scratch, unsigned char *fp16,
+                                  unsigned char *bf16, cudaStream_t s)
 {
-    build_tc_tiles_kernel<<<256, 256, 0, s>>>(L64, w32, n, tc_row_tiles(n), tc_k_tiles(n), bf16, tiles);
+    wtl_kernel<<<dim3((n + 31) / 32, kWtlSegs), 256, 0, s>>>(L64, w32, n, scratch);
+    const int n_mt = tc_row_tiles(n), n_kt = tc_k_tiles(n);
+    if (fp16) build_tc_tiles_kernel<<<608, 256, 0, s>>>(L64, scratch, n, n_mt, n_kt, 0, fp16);
+    if (bf16) build_tc_tiles_kernel<<<608, 256, 0, s>>>(L64, scratch, n, n_mt, n_kt, 1, bf16);
     return cudaGetLastError();
 }
 
