@@ -1,4 +1,4 @@
-"""FP64 factorisation at the edges of its forms: the one-CTA form's column
+"""FP64 factorisation and sample moments at the edges of their forms: the one-CTA form's column
 counts (16, 32, 48, 64 and their neighbours), the blocked form's 32-column
 blocks and 16 x 16 update tiles, and a failing pivot in each place.
 
@@ -58,3 +58,42 @@ def test_extreme_scales(gpu, n, scale):
     L = gpu.Portfolio(np.zeros(n), unit * scale).factor()
     ref = np.linalg.cholesky(unit) * np.sqrt(scale)
     assert np.max(np.abs(L - ref)) <= np.linalg.cond(unit) * n * 2.0 ** -52 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("T,n", [(2, 31), (2, 32), (31, 33), (32, 1), (33, 32), (63, 5), (64, 64), (127, 65), (128, 2),
+                                 (129, 97), (2049, 31), (4100, 3)])
+def test_moments_edges(gpu, T, n):
+    """Row segments and 32 x 32 tiles at their edges, against exactly rounded
+    sums (math.fsum).  mu: 2 eps of the mean absolute value; Sigma: two
+    roundings of the deviations and at most T of the sum, (T + 4) eps of the
+    sum of absolute products."""
+    import math
+    X = np.random.default_rng(T * 131 + n).normal(3e-4, 0.01, size=(T, n))
+    mu, sigma = gpu.moments(X)
+    eps = 2.0 ** -52
+    for j in range(n):
+        assert abs(mu[j] - math.fsum(X[:, j]) / T) <= 2 * eps * np.mean(np.abs(X[:, j]))
+    D = X - mu
+    S_abs = np.abs(D).T @ np.abs(D) / (T - 1) + eps * np.abs(X).max() ** 2
+    for i in range(0, n, max(1, n // 4)):
+        for j in range(0, n, max(1, n // 5)):
+            ref = math.fsum(D[:, i] * D[:, j]) / (T - 1)
+            assert abs(sigma[i, j] - ref) <= (T + 4) * eps * S_abs[i, j]
+    assert np.array_equal(sigma, sigma.T)
+
+
+@pytest.mark.parametrize("T,n,at", [(2, 1, 1), (40, 33, 40 * 33 - 1), (70, 40, 0), (70, 40, 1234), (300, 65, 7777)])
+def test_first_entry_not_finite(gpu, T, n, at):
+    """The first entry (row by row) that is not finite is named, whichever
+    kernel meets it first; the outputs are not written."""
+    X = np.zeros((T, n))
+    X.flat[at] = np.inf
+    if at + 1 < T * n:
+        X.flat[-1] = np.nan
+    where = rf"returns\[{at // n}\]\[{at % n}\] is not finite"
+    with pytest.raises(gpu.RiskGpuError, match=where) as e:
+        gpu.moments(X)
+    assert e.value.status == gpu.RG_ERR_INVALID
+    with pytest.raises(gpu.RiskGpuError, match=where) as e:
+        gpu.crash_frequency(X, 0.01, 1)
+    assert e.value.status == gpu.RG_ERR_INVALID
