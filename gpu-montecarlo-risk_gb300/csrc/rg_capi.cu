@@ -38,11 +38,33 @@ int set_error(int status, const char *fmt, ...)
     return status;
 }
 
+// What one rg_simulate call needs besides device memory: its timing events
+// and a pinned buffer for the counters and the first VaR candidates, so that
+// they come back in one wait without a pageable copy's staging.
+struct QueryRes {
+    static constexpr size_t kCand = 16384; // candidates copied with the counters
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    unsigned char *h = nullptr;
+};
+
+// Process-global state of one device.  `pool` holds what the engine's calls
+// allocate and free on their way (query scratch, portfolios, preprocessing
+// buffers): stream-ordered, thread-safe, and at each synchronisation the
+// driver gets back whatever it keeps beyond kPoolKeep bytes (pool_trim gives
+// back the rest).  From the device's default pool, which keeps nothing, every
+// call after a device synchronisation mapped its scratch anew (a 9-asset call
+// alone: 228 us, of which about 190).  `idle` keeps the resources of a few
+// calls for the next ones.
 struct DevCtx {
     bool ready = false;
     int sm_count = 0;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;
+    std::vector<QueryRes> idle;
 };
+
+static constexpr unsigned long long kPoolKeep = 64ull << 20;
+static constexpr size_t kIdleQueries = 8;
 
 static std::mutex g_mu;
 static DevCtx g_ctx[64];
@@ -74,7 +96,19 @@ static int get_ctx(DevCtx **out, int *dev_out)
     DevCtx &c = g_ctx[dev];
     if (!c.ready) {
         cudaError_t e = cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess && !c.stream) e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess && !c.pool) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            e = cudaMemPoolCreate(&c.pool, &props);
+        }
+        if (e == cudaSuccess) {
+            unsigned long long keep = kPoolKeep;
+            e = cudaMemPoolSetAttribute(c.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
         if (e != cudaSuccess)
             return set_error(RG_ERR_CUDA, "device init failed: %s", cudaGetErrorString(e));
         c.ready = true;
@@ -82,6 +116,57 @@ static int get_ctx(DevCtx **out, int *dev_out)
     *out = &c;
     if (dev_out) *dev_out = dev;
     return RG_OK;
+}
+
+int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
+{
+    DevCtx *c = nullptr;
+    *err = cudaSuccess;
+    const int st = get_ctx(&c, nullptr);
+    if (st) return st;
+    *err = cudaMallocFromPoolAsync(p, bytes, c->pool, s);
+    return RG_OK;
+}
+
+// Everything the pool of the current device keeps but does not use goes back
+// to the driver.
+void pool_trim()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (g_ctx[dev].pool) cudaMemPoolTrimTo(g_ctx[dev].pool, 0);
+}
+
+static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (!c->idle.empty()) {
+            *r = c->idle.back();
+            c->idle.pop_back();
+            return cudaSuccess;
+        }
+    }
+    cudaError_t e = cudaEventCreate(&r->e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&r->e1);
+    if (e == cudaSuccess) e = cudaMallocHost(&r->h, 64 + QueryRes::kCand * sizeof(float));
+    return e;
+}
+
+// Back to the list (the call's work is complete), or freed when it is full.
+static void query_res_give(DevCtx *c, QueryRes &r)
+{
+    if (r.e0 && r.e1 && r.h) {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (c->idle.size() < kIdleQueries) {
+            c->idle.push_back(r);
+            return;
+        }
+    }
+    if (r.e0) cudaEventDestroy(r.e0);
+    if (r.e1) cudaEventDestroy(r.e1);
+    if (r.h) cudaFreeHost(r.h);
 }
 
 #define RG_CUDA_TRY(call)                                                                          \
@@ -112,8 +197,12 @@ static int admit(size_t need)
     if (h && h[0]) {
         size_t headroom = (size_t)strtoull(h, nullptr, 10);
         size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess)
-            return set_error(RG_ERR_CUDA, "cudaMemGetInfo failed");
+        for (int tries = 0; tries < 2; tries++) {
+            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess)
+                return set_error(RG_ERR_CUDA, "cudaMemGetInfo failed");
+            if (fr >= need && fr - need >= headroom) break;
+            if (tries == 0) pool_trim(); // what the engine keeps for later calls does not refuse this one
+        }
         if (fr < need || fr - need < headroom)
             return set_error(RG_ERR_ADMISSION,
                              "admission refused: %zu bytes requested, %zu free, headroom %zu", need,
@@ -122,10 +211,21 @@ static int admit(size_t need)
     return RG_OK;
 }
 
-static void portfolio_free(Portfolio *p)
+// `quiet`: no work that uses the portfolio is in flight on any stream.
+// Otherwise the device is waited for first, as cudaFree would: a caller may
+// have launched on a stream of its own.
+static void portfolio_free(Portfolio *p, bool quiet)
 {
     if (!p) return;
-    cudaFree(p->d_block);
+    if (p->d_block) {
+        int dev = p->device;
+        cudaGetDevice(&dev);
+        if (dev != p->device) cudaSetDevice(p->device);
+        if (!quiet) cudaDeviceSynchronize();
+        DevCtx *c = nullptr;
+        if (get_ctx(&c, nullptr) == RG_OK) cudaFreeAsync(p->d_block, c->stream);
+        if (dev != p->device) cudaSetDevice(dev);
+    }
     delete p;
 }
 
@@ -184,6 +284,7 @@ static double inv_norm_cdf(double prob)
     double lo = -40.0, hi = 40.0;
     for (int it = 0; it < 200; it++) {
         const double mid = 0.5 * (lo + hi);
+        if (mid <= lo || mid >= hi) break; // no double between them
         if (0.5 * std::erfc(-mid / std::sqrt(2.0)) < prob) lo = mid; else hi = mid;
     }
     return 0.5 * (lo + hi);
@@ -200,8 +301,10 @@ static cudaError_t launch_counting(const Portfolio *p, const rg_query *q, const 
     if (q->precision == RG_PREC_BF16X3 || q->precision == RG_PREC_FP16X3) {
         const int bf16 = q->precision == RG_PREC_BF16X3 ? 1 : 0;
         if (!p->d_tc[bf16] || !a.err) return cudaErrorInvalidValue; // prepared at creation
-        const cudaError_t e = cudaMemsetAsync(a.err, 0, sizeof(unsigned int), s);
-        if (e != cudaSuccess) return e;
+        if (a.err == p->d_err) { // else the caller's, cleared by it
+            const cudaError_t e = cudaMemsetAsync(a.err, 0, sizeof(unsigned int), s);
+            if (e != cudaSuccess) return e;
+        }
         // RG_FAULT_INJECT=tcstall: one pipeline stage is never filled, so the
         // kernel's bounded wait runs out (host-side injection; no fault)
         return launch_tc(a, p->d_tc[bf16], bf16, q->draw_mode == RG_DRAWS_AGGREGATED, p->wmu, a.err,
@@ -219,32 +322,41 @@ static cudaError_t launch_counting(const Portfolio *p, const rg_query *q, const 
 }
 
 // Device scratch of one query: counters, VaR tail sums, candidate count,
-// histogram and candidate list, carved from one stream-ordered allocation.
+// error word, candidate list and histogram, carved from one stream-ordered
+// allocation.  The head and the candidates after it come back in one copy.
 struct QueryScratch {
     unsigned long long *counts = nullptr;  // [2]
     unsigned long long *counts2 = nullptr; // [2] counters of the extra VaR passes (discarded)
     unsigned long long *tail = nullptr;    // [2]
     unsigned int *cand_count = nullptr;    // [1]
-    unsigned long long *hist = nullptr;    // [kVarHistBins + 2]
+    unsigned int *err = nullptr;           // [1] error word of the tensor-core kernel
     float *cand = nullptr;                 // [cap]
+    unsigned long long *hist = nullptr;    // [kVarHistBins + 2]
     unsigned int cap = 0;
     void *base = nullptr;
 };
+// The same fields in the pinned buffer.
+struct QueryHead {
+    unsigned long long counts[2], counts2[2], tail[2];
+    unsigned int cand_count, err;
+};
+static_assert(sizeof(QueryHead) == 56, "device and host layout");
 
-static cudaError_t scratch_alloc(QueryScratch &sc, unsigned int cap, bool with_var, cudaStream_t s)
+static cudaError_t scratch_alloc(DevCtx *ctx, QueryScratch &sc, unsigned int cap, bool with_var, cudaStream_t s)
 {
-    const size_t head = 8 * 2 + 8 * 2 + 8 * 2 + 8;
+    const size_t head = sizeof(QueryHead);
+    const size_t cand = with_var ? ((4 * (size_t)cap + 7) & ~(size_t)7) : 0;
     const size_t hist = with_var ? 8 * (size_t)(kVarHistBins + 2) : 0;
-    const size_t total = head + hist + 4 * (size_t)(with_var ? cap : 0) + 16;
-    cudaError_t e = cudaMallocAsync(&sc.base, total, s);
+    cudaError_t e = cudaMallocFromPoolAsync(&sc.base, head + cand + hist + 16, ctx->pool, s);
     if (e != cudaSuccess) return e;
     char *b = (char *)sc.base;
     sc.counts = (unsigned long long *)b;
     sc.counts2 = sc.counts + 2;
     sc.tail = sc.counts + 4;
     sc.cand_count = (unsigned int *)(sc.counts + 6);
-    sc.hist = with_var ? (unsigned long long *)(b + head) : nullptr;
-    sc.cand = with_var ? (float *)(b + head + hist) : nullptr;
+    sc.err = sc.cand_count + 1;
+    sc.cand = with_var ? (float *)(b + head) : nullptr;
+    sc.hist = with_var ? (unsigned long long *)(b + head + cand) : nullptr;
     sc.cap = with_var ? cap : 0;
     return cudaMemsetAsync(sc.base, 0, head, s);
 }
@@ -290,6 +402,12 @@ static int check_device(const Portfolio *p)
     return RG_OK;
 }
 
+static int tc_status(unsigned int err)
+{
+    if (err) return set_error(RG_ERR_TIMEOUT, "tensor-core kernel gave up a bounded wait (error word 0x%x)", err);
+    return RG_OK;
+}
+
 // Status of a completed tensor-core pass: the kernel sets its error word
 // when one of its bounded waits ran out, and its counts are then
 // incomplete.  Reads the word on stream s (which it synchronises); RG_OK
@@ -302,8 +420,7 @@ static int tc_pass_status(const Portfolio *p, const rg_query *q, cudaStream_t s)
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)
         return set_error(RG_ERR_CUDA, "read of the tensor-core error word failed: %s", cudaGetErrorString(e));
-    if (err) return set_error(RG_ERR_TIMEOUT, "tensor-core kernel gave up a bounded wait (error word 0x%x)", err);
-    return RG_OK;
+    return tc_status(err);
 }
 
 // Shared with rg_noalloc.cu (same checks, same launch selection).
@@ -455,7 +572,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t ow32 = bp.take((size_t)n * sizeof(float));
         const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
-        RG_CUDA_TRY(cudaMalloc(&p->d_block, bp.total));
+        RG_CUDA_TRY(cudaMallocFromPoolAsync(&p->d_block, bp.total, ctx->pool, s));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
         p->d_L64 = reinterpret_cast<double *>(blk + oL64);
         p->d_mu64 = reinterpret_cast<double *>(blk + omu);
@@ -471,9 +588,12 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     if (!dev_in) {
         // Sigma and the weights share one upload buffer
         const size_t a_bytes = (nn * sizeof(double) + 255) & ~(size_t)255;
-        RG_CUDA_TRY(cudaMalloc(&dA, a_bytes + (weights ? (size_t)n * sizeof(double) : 0)));
-        RG_CUDA_TRY(cudaMemcpy2DAsync(dA, (size_t)n * sizeof(double), sigma, (size_t)ld * sizeof(double),
-                                      (size_t)n * sizeof(double), (size_t)n, cudaMemcpyHostToDevice, s));
+        RG_CUDA_TRY(cudaMallocFromPoolAsync((void **)&dA, a_bytes + (weights ? (size_t)n * sizeof(double) : 0), ctx->pool, s));
+        if (ld == n)
+            RG_CUDA_TRY(cudaMemcpyAsync(dA, sigma, nn * sizeof(double), cudaMemcpyHostToDevice, s));
+        else
+            RG_CUDA_TRY(cudaMemcpy2DAsync(dA, (size_t)n * sizeof(double), sigma, (size_t)ld * sizeof(double),
+                                          (size_t)n * sizeof(double), (size_t)n, cudaMemcpyHostToDevice, s));
         RG_CUDA_TRY(cudaMemcpyAsync(p->d_mu64, mu, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s));
         if (weights) {
             dW = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(dA) + a_bytes);
@@ -530,25 +650,26 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
             p->h_w[(size_t)i] = weights ? (float)weights[i] : 0.f; // as the factorisation writes d_w32
         }
     }
+    if (dA) RG_CUDA_TRY(cudaFreeAsync(dA, s));
+    dA = nullptr;
     RG_CUDA_TRY(cudaStreamSynchronize(s));
-    cudaFree(dA);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     *out = reinterpret_cast<rg_portfolio *>(p);
     return RG_OK;
 fail:
     cudaStreamSynchronize(s);
-    cudaFree(dA);
+    if (dA) cudaFreeAsync(dA, s);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    portfolio_free(p);
+    portfolio_free(p, true);
     return st;
 }
 
 int rg_portfolio_destroy(rg_portfolio *h)
 {
     if (!h) return RG_OK;
-    portfolio_free(reinterpret_cast<Portfolio *>(h));
+    portfolio_free(reinterpret_cast<Portfolio *>(h), false);
     return RG_OK;
 }
 
@@ -627,21 +748,23 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         cap = (unsigned int)std::min(4.0 * expect + 4096.0, 64.0 * 1024 * 1024);
     }
     QueryScratch sc;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    QueryRes res;
+    QueryHead head;
     float ms = 0.f, ms_pass = 0.f;
-    unsigned long long counts[2] = {0, 0}, tail[2] = {0, 0};
     unsigned int ncand = 0;
-    std::vector<float> cand;
+    size_t pre = 0;   // candidates copied with the counters
+    float *cand = nullptr;
+    std::vector<float> cand_v;
     std::vector<unsigned long long> hist;
     int passes = 0;
     int64_t n_tail = 0;
     PlainArgs a;
     st = admit(64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2));
     if (st) return st;
-    RG_CUDA_TRY(scratch_alloc(sc, cap, want_var, s));
-    RG_CUDA_TRY(cudaEventCreate(&e0));
-    RG_CUDA_TRY(cudaEventCreate(&e1));
+    RG_CUDA_TRY(query_res_take(ctx, &res));
+    RG_CUDA_TRY(scratch_alloc(ctx, sc, cap, want_var, s));
     a = make_args(p, q, sc.counts);
+    a.err = sc.err;
     if (want_var) {
         a.var_mode = 1;
         a.sel_bins = 1;
@@ -654,20 +777,19 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         a.tail = sc.tail;
         a.hist = sc.hist;
     }
-    RG_CUDA_TRY(cudaEventRecord(e0, s));
+    RG_CUDA_TRY(cudaEventRecord(res.e0, s));
     RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-    RG_CUDA_TRY(cudaEventRecord(e1, s));
-    RG_CUDA_TRY(cudaMemcpyAsync(counts, sc.counts, sizeof(counts), cudaMemcpyDeviceToHost, s));
-    if (want_var) {
-        RG_CUDA_TRY(cudaMemcpyAsync(tail, sc.tail, sizeof(tail), cudaMemcpyDeviceToHost, s));
-        RG_CUDA_TRY(cudaMemcpyAsync(&ncand, sc.cand_count, sizeof(ncand), cudaMemcpyDeviceToHost, s));
-    }
+    RG_CUDA_TRY(cudaEventRecord(res.e1, s));
+    pre = want_var ? std::min((size_t)sc.cap, QueryRes::kCand) : 0;
+    RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head) + 4 * pre, cudaMemcpyDeviceToHost, s));
     RG_CUDA_TRY(cudaStreamSynchronize(s));
-    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventElapsedTime(&ms, res.e0, res.e1);
+    memcpy(&head, res.h, sizeof(head));
+    ncand = head.cand_count;
     passes = 1;
-    st = tc_pass_status(p, q, s);
+    st = tc_status(head.err);
     if (st) goto fail;
-    n_tail = (int64_t)tail[0];
+    n_tail = (int64_t)head.tail[0];
     if (want_var && !(n_tail < T && T <= n_tail + (int64_t)ncand && ncand <= sc.cap)) {
         // The band missed the order statistic: histogram pass over
         // mean -+ 12 sd, then a select pass on the bin that holds it.
@@ -678,14 +800,15 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         a.sel_lo = (float)(mean - 12.0 * sd);
         a.sel_inv_w = (float)(kVarHistBins / (24.0 * sd));
         RG_CUDA_TRY(cudaMemsetAsync(sc.hist, 0, hist.size() * 8, s));
-        RG_CUDA_TRY(cudaEventRecord(e0, s));
+        RG_CUDA_TRY(cudaEventRecord(res.e0, s));
         RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-        RG_CUDA_TRY(cudaEventRecord(e1, s));
+        RG_CUDA_TRY(cudaEventRecord(res.e1, s));
         RG_CUDA_TRY(cudaMemcpyAsync(hist.data(), sc.hist, hist.size() * 8, cudaMemcpyDeviceToHost, s));
+        RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head), cudaMemcpyDeviceToHost, s));
         RG_CUDA_TRY(cudaStreamSynchronize(s));
-        st = tc_pass_status(p, q, s);
+        st = tc_status(reinterpret_cast<const QueryHead *>(res.h)->err);
         if (st) goto fail;
-        cudaEventElapsedTime(&ms_pass, e0, e1);
+        cudaEventElapsedTime(&ms_pass, res.e0, res.e1);
         ms += ms_pass;
         int64_t cum = 0;
         int j = 0;
@@ -701,8 +824,9 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         if (need > sc.cap) {
             RG_CUDA_TRY(cudaFreeAsync(sc.base, s));
             sc.base = nullptr;
-            RG_CUDA_TRY(scratch_alloc(sc, need, true, s));
+            RG_CUDA_TRY(scratch_alloc(ctx, sc, need, true, s));
             a.counts = sc.counts2;
+            a.err = sc.err;
             a.cand = sc.cand;
             a.cand_count = sc.cand_count;
             a.tail = sc.tail;
@@ -711,37 +835,45 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         a.var_mode = 1;
         a.sel_target = j - 1;
         a.cand_cap = sc.cap;
-        RG_CUDA_TRY(cudaMemsetAsync(sc.tail, 0, 2 * 8, s));
-        RG_CUDA_TRY(cudaMemsetAsync(sc.cand_count, 0, 4, s));
-        RG_CUDA_TRY(cudaEventRecord(e0, s));
+        RG_CUDA_TRY(cudaMemsetAsync(sc.tail, 0, 2 * 8 + 4, s)); // and the candidate count behind it
+        RG_CUDA_TRY(cudaEventRecord(res.e0, s));
         RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-        RG_CUDA_TRY(cudaEventRecord(e1, s));
-        RG_CUDA_TRY(cudaMemcpyAsync(tail, sc.tail, sizeof(tail), cudaMemcpyDeviceToHost, s));
-        RG_CUDA_TRY(cudaMemcpyAsync(&ncand, sc.cand_count, sizeof(ncand), cudaMemcpyDeviceToHost, s));
+        RG_CUDA_TRY(cudaEventRecord(res.e1, s));
+        pre = std::min((size_t)sc.cap, QueryRes::kCand);
+        RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head) + 4 * pre, cudaMemcpyDeviceToHost, s));
         RG_CUDA_TRY(cudaStreamSynchronize(s));
-        st = tc_pass_status(p, q, s);
+        {
+            QueryHead again;
+            memcpy(&again, res.h, sizeof(again));
+            st = tc_status(again.err);
+            head.tail[0] = again.tail[0]; // the counters are the first pass's
+            head.tail[1] = again.tail[1];
+            ncand = again.cand_count;
+        }
         if (st) goto fail;
-        cudaEventElapsedTime(&ms_pass, e0, e1);
+        cudaEventElapsedTime(&ms_pass, res.e0, res.e1);
         ms += ms_pass;
         passes = 3;
-        n_tail = (int64_t)tail[0];
+        n_tail = (int64_t)head.tail[0];
         if (n_tail != cum || ncand != need || ncand > sc.cap) {
             st = set_error(RG_ERR_CUDA, "VaR select pass disagrees with its histogram");
             goto fail;
         }
     }
-    if (want_var) {
-        cand.resize(ncand);
-        if (ncand)
-            RG_CUDA_TRY(cudaMemcpyAsync(cand.data(), sc.cand, (size_t)ncand * 4, cudaMemcpyDeviceToHost, s));
+    if (want_var && ncand > pre) {
+        cand_v.resize(ncand);
+        cand = cand_v.data();
+        RG_CUDA_TRY(cudaMemcpyAsync(cand, sc.cand, (size_t)ncand * 4, cudaMemcpyDeviceToHost, s));
         RG_CUDA_TRY(cudaStreamSynchronize(s));
+    } else if (want_var) {
+        cand = reinterpret_cast<float *>(res.h + sizeof(head));
     }
     RG_CUDA_TRY(cudaFreeAsync(sc.base, s));
     sc.base = nullptr;
     memset(out, 0, sizeof(*out));
     out->n_paths = M;
-    out->crash_count = (int64_t)counts[0];
-    out->breach_count = (int64_t)counts[1];
+    out->crash_count = (int64_t)head.counts[0];
+    out->breach_count = (int64_t)head.counts[1];
     rg_estimator_stats(out->crash_count, M, &out->p_crash, &out->se_crash, &out->ci_lower, &out->ci_upper);
     rg_estimator_stats(out->breach_count, M, &out->p_breach, &out->se_breach, nullptr, nullptr);
     out->var = NAN;
@@ -749,9 +881,9 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
     if (want_var) {
         // the T-th smallest w.R overall is the (T - n_tail)-th smallest candidate
         const size_t kth = (size_t)(T - n_tail - 1);
-        std::nth_element(cand.begin(), cand.begin() + (long)kth, cand.end());
+        std::nth_element(cand, cand + kth, cand + ncand);
         const float vport = cand[kth];
-        double tail_sum = (double)(long long)tail[1] * 0x1p-32;
+        double tail_sum = (double)(long long)head.tail[1] * 0x1p-32;
         for (size_t i = 0; i < kth; i++) tail_sum += -(double)cand[i];
         tail_sum += -(double)vport;
         out->var = -(double)vport;
@@ -760,14 +892,12 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         out->var_passes = passes;
     }
     out->ms_device = ms;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    query_res_give(ctx, res);
     return RG_OK;
 fail:
     cudaStreamSynchronize(s);
-    if (sc.base) cudaFree(sc.base);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
+    if (sc.base) cudaFreeAsync(sc.base, s);
+    query_res_give(ctx, res);
     return st;
 }
 
@@ -780,7 +910,7 @@ int rg_run(int32_t n, const double *mu, const double *sigma, int64_t ld, const d
     st = create_portfolio(n, mu, sigma, ld, weights, 0, parts_for_query(q, n), &h);
     if (st) return st;
     st = rg_simulate(h, q, out, nullptr);
-    rg_portfolio_destroy(h);
+    portfolio_free(reinterpret_cast<Portfolio *>(h), true); // rg_simulate has waited for its work
     return st;
 }
 
@@ -845,7 +975,8 @@ static int plugin_portfolio(int n, const double *mu, const double *sigma, long l
     rg_portfolio *h = nullptr;
     const int st = create_portfolio(n, mu, sigma, tda, nullptr, 0, parts, &h);
     if (st != RG_OK) return st;
-    PortfolioRef ref(h, [](rg_portfolio *x) { rg_portfolio_destroy(x); });
+    // every call that held it has waited for its own work
+    PortfolioRef ref(h, [](rg_portfolio *x) { portfolio_free(reinterpret_cast<Portfolio *>(x), true); });
     *out = ref;
     if (!use_cache) return RG_OK;
     std::lock_guard<std::mutex> lk(g_plugin_mu);

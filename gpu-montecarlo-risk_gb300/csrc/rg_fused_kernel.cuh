@@ -25,6 +25,7 @@
 //  * Counts: per-thread integers -> warp reduction -> one 64-bit atomic per
 //    CTA per counter.
 #pragma once
+#include <atomic>
 #include <cstring>
 #include "rg_internal.cuh"
 
@@ -242,10 +243,19 @@ static cudaError_t launch_fused_nq(const PlainArgs &a, const float *Lp_host, con
     const bool one_day = (a.horizon == 1 || a.aggregated);
     auto kern = (a.var_mode != 0) ? (one_day ? mc_rows_kernel<NQ, true, true> : mc_rows_kernel<NQ, false, true>)
                 : one_day ? mc_rows_kernel<NQ, true, false> : mc_rows_kernel<NQ, false, false>;
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFusedThreads, 0);
+    // CTAs an SM of each form, asked of the runtime once per device
+    static std::atomic<int> occupancy[64][2][2];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
+    std::atomic<int> &occ = occupancy[dev & 63][a.var_mode != 0][one_day];
+    int per_sm = occ.load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFusedThreads, 0);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) per_sm = 1;
+        occ.store(per_sm, std::memory_order_relaxed);
+    }
     long long want = (a.n_paths + kFusedThreads - 1) / kFusedThreads;
     long long grid = (long long)sm_count * per_sm;
     if (want < grid) grid = want;

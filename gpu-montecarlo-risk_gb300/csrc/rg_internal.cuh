@@ -250,4 +250,10 @@ size_t cholesky_aux_len(int n);
 // Error helpers (rg_capi.cu).
 int set_error(int status, const char *fmt, ...);
 
+// Stream-ordered device memory from the engine's pool of the current device
+// (rg_capi.cu; freed with cudaFreeAsync).  Returns RG_OK with *err the
+// allocation's result, or the status of a device that could not be set up.
+int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err);
+void pool_trim();
+
 } // namespace rg

@@ -243,7 +243,8 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
                  ocov = ocol + 2 * (size_t)kMomSegs * n, obad = ocov + (size_t)segs * tiles * kMomTile * kMomTile;
     double *d = nullptr;
     unsigned long long bad = kAllFinite;
-    cudaError_t e = cudaMalloc(&d, (obad + 1) * sizeof(double));
+    cudaError_t e = cudaSuccess;
+    if ((st = pool_alloc((void **)&d, (obad + 1) * sizeof(double), s, &e)) != RG_OK) return st;
     if (e == cudaSuccess) {
         unsigned long long *dbad = reinterpret_cast<unsigned long long *>(d + obad);
         e = cudaMemsetAsync(dbad, 0xff, sizeof(*dbad), s);
@@ -266,7 +267,7 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }
     }
-    cudaFree(d);
+    if (d) cudaFreeAsync(d, s);
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_moments: %s",
                          cudaGetErrorString(e));
@@ -286,7 +287,8 @@ extern "C" int rg_crash_frequency(const double *returns, int64_t T, int32_t n, i
     const size_t xbytes = (size_t)T * (size_t)n * sizeof(double);
     unsigned char *d = nullptr;
     unsigned long long got[2] = {0, kAllFinite}; // crash days, first entry that is not finite
-    cudaError_t e = cudaMalloc(&d, xbytes + sizeof(got));
+    cudaError_t e = cudaSuccess;
+    if ((st = pool_alloc((void **)&d, xbytes + sizeof(got), s, &e)) != RG_OK) return st;
     if (e == cudaSuccess) {
         unsigned long long *dgot = reinterpret_cast<unsigned long long *>(d + xbytes);
         e = cudaMemsetAsync(dgot, 0, sizeof(got[0]), s);
@@ -300,7 +302,7 @@ extern "C" int rg_crash_frequency(const double *returns, int64_t T, int32_t n, i
         if (e == cudaSuccess) e = cudaMemcpyAsync(got, dgot, sizeof(got), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
-    cudaFree(d);
+    if (d) cudaFreeAsync(d, s);
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_crash_frequency: %s",
                          cudaGetErrorString(e));

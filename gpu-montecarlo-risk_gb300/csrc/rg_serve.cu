@@ -208,7 +208,11 @@ static bool schedule_once(Server *sv)
             }
         if (!free_slot) break;
         size_t fr = 0, tot = 0;
-        const bool mem_ok = cudaMemGetInfo(&fr, &tot) == cudaSuccess && (long long)fr > sv->cfg.headroom_bytes;
+        bool mem_ok = cudaMemGetInfo(&fr, &tot) == cudaSuccess && (long long)fr > sv->cfg.headroom_bytes;
+        if (!mem_ok) { // not for what the engine keeps for later calls
+            pool_trim();
+            mem_ok = cudaMemGetInfo(&fr, &tot) == cudaSuccess && (long long)fr > sv->cfg.headroom_bytes;
+        }
         if (!mem_ok) {
             // refuse requests that have waited too long for headroom
             while (!sv->pending.empty()) {
