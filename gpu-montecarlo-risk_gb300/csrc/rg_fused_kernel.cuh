@@ -4,8 +4,8 @@
 // (src/05-GPU/monte_carlos_cuda.cu:23-72), organised for issue throughput on
 // sm_103a:
 //
-//  * One thread owns one path at a time (grid-stride over paths, grid =
-//    SMs x resident CTAs).  Nothing per path reaches HBM unless the caller
+//  * One thread owns one path at a time (grid-stride over paths, one CTA an
+//    SM: FusedShape).  Nothing per path reaches HBM unless the caller
 //    asks for S or w.R per path.
 //  * Row order with packed FP32 pairs.  Row group g (rows 4g..4g+3) needs
 //    the normals of quads 0..g; the normals of quad g+1 (one Philox4x32-10
@@ -25,13 +25,29 @@
 //  * Counts: per-thread integers -> warp reduction -> one 64-bit atomic per
 //    CTA per counter.
 #pragma once
-#include <atomic>
 #include <cstring>
 #include "rg_internal.cuh"
 
 namespace rg {
 
-static constexpr int kFusedThreads = 256;
+// CTA shape: the threads an SM holds in one CTA (two for the smallest
+// kernels), so that the SM's registers are divided once.  In CTAs of 256 at
+// the same registers a thread, 23 warps were active on average instead of 28
+// to 32 (4 CTAs of 64 registers a thread fill the register file to the last
+// word, and the fourth often started late).  Fewer threads than 1024 where
+// the rows need the registers; more days a path, more registers.
+// Measured, before (4 x 256, several days 3 x 256) -> now, ms:
+//   one day:  NQ = 3, 4e7 paths 0.510 -> 0.464; NQ = 5, 4e7 0.887 -> 0.829;
+//             NQ = 8, 4e7 1.581 -> 1.501; NQ = 13, 1e7 0.869 -> 0.763
+//   ten days: NQ = 3, 4e6 0.378 -> 0.357; NQ = 5, 4e6 0.623 -> 0.573;
+//             NQ = 8, 4e6 1.066 -> 0.946; NQ = 13, 1e6 0.482 -> 0.436
+// and the shapes on either side of each line: NQ = 3 1 x 1024 0.487; NQ = 5
+// 2 x 768 0.836; NQ = 8 1 x 896 1.505; NQ = 13 1 x 1024 0.789, 1 x 768 0.768;
+// ten days NQ = 3 2 x 768 0.366, NQ = 5 2 x 640 0.622.
+template <int NQ, bool ONE_DAY> struct FusedShape {
+    static constexpr int kCtas = (ONE_DAY && NQ <= 3) ? 2 : 1;
+    static constexpr int kThreads = ONE_DAY ? (NQ <= 3 ? 768 : NQ <= 8 ? 1024 : 896) : (NQ <= 5 ? 1024 : 768);
+};
 
 template <int NQ>
 struct ConstBlock {
@@ -137,12 +153,12 @@ __device__ __forceinline__ void cta_flush(const PlainArgs &a, int crash, int bre
 
 // NQ = ceil(N/4) exactly (the launcher dispatches on it), so every row
 // group exists; rows >= N occur only in the last group, hold zeros and are
-// masked out of S.  ONE_DAY drops the horizon loop for H = 1.  Four CTAs of
-// 256 threads per SM (64 registers a thread); with the horizon loop three
-// (85 registers: fewer spills, 5 % faster at N = 50, H = 10).  VAR adds the VaR/CVaR
-// bookkeeping of var_path (the counting-only form carries none of it).
+// masked out of S.  ONE_DAY drops the horizon loop for H = 1.  VAR adds the
+// VaR/CVaR bookkeeping of var_path (the counting-only form carries none of
+// it).
 template <int NQ, bool ONE_DAY, bool VAR>
-__global__ void __launch_bounds__(kFusedThreads, ONE_DAY ? 4 : 3) mc_rows_kernel(const PlainArgs a, const ConstBlock<NQ> cb)
+__global__ void __launch_bounds__(FusedShape<NQ, ONE_DAY>::kThreads, FusedShape<NQ, ONE_DAY>::kCtas)
+    mc_rows_kernel(const PlainArgs a, const ConstBlock<NQ> cb)
 {
     __shared__ unsigned long long sacc[4];
     __shared__ unsigned int shist[VAR ? kVarHistBins + 2 : 1];
@@ -243,24 +259,17 @@ static cudaError_t launch_fused_nq(const PlainArgs &a, const float *Lp_host, con
     const bool one_day = (a.horizon == 1 || a.aggregated);
     auto kern = (a.var_mode != 0) ? (one_day ? mc_rows_kernel<NQ, true, true> : mc_rows_kernel<NQ, false, true>)
                 : one_day ? mc_rows_kernel<NQ, true, false> : mc_rows_kernel<NQ, false, false>;
-    // CTAs an SM of each form, asked of the runtime once per device
-    static std::atomic<int> occupancy[64][2][2];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::atomic<int> &occ = occupancy[dev & 63][a.var_mode != 0][one_day];
-    int per_sm = occ.load(std::memory_order_relaxed);
-    if (per_sm == 0) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFusedThreads, 0);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
-        occ.store(per_sm, std::memory_order_relaxed);
-    }
-    long long want = (a.n_paths + kFusedThreads - 1) / kFusedThreads;
-    long long grid = (long long)sm_count * per_sm;
-    if (want < grid) grid = want;
-    if (grid < 1) grid = 1;
-    kern<<<(unsigned)grid, kFusedThreads, 0, s>>>(a, cb);
+    // Every thread gets the same number of paths, or one more: with `rounds`
+    // paths a thread at the full shape, the CTAs shrink until they are all
+    // busy in the last round (also with fewer paths than threads).
+    const long long ctas = (long long)sm_count * (one_day ? FusedShape<NQ, true>::kCtas : FusedShape<NQ, false>::kCtas);
+    const int most = one_day ? FusedShape<NQ, true>::kThreads : FusedShape<NQ, false>::kThreads;
+    const long long rounds = (a.n_paths - 1) / (ctas * most) + 1;
+    long long threads = (a.n_paths - 1) / (ctas * rounds) + 1;
+    threads = (threads + 31) / 32 * 32;
+    if (threads > most) threads = most;
+    const long long want = (a.n_paths - 1) / threads + 1;
+    kern<<<(unsigned)(want < ctas ? want : ctas), (unsigned)threads, 0, s>>>(a, cb);
     return cudaGetLastError();
 }
 
