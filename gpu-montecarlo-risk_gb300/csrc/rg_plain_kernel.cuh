@@ -3,7 +3,7 @@
 // Replaces the reference kernel monte_carlo_kernel
 // (src/05-GPU/monte_carlos_cuda.cu:23-72).  One thread owns one path at a
 // time (grid sized to fill every SM; grid-stride over paths in the Philox
-// layout, a contiguous run of paths per thread in the XORWOW layout):
+// layout, a contiguous run of paths per CTA in the XORWOW layout):
 //   1. normals in registers: Philox4x32-10 + Box-Muller (engine layout) or
 //      the reference's own cuRAND XORWOW stream (curand_init(seed, path, 0)
 //      + curand_normal_double, rounded to FP32), summed over H days;
@@ -51,24 +51,39 @@ __global__ void __launch_bounds__(kPlainThreads, 2) mc_plain_small_kernel(const 
 
     const int nq = (n + 3) >> 2;
     int crash = 0, breach = 0;
-    // Philox: grid-stride over paths.  XORWOW: each thread walks a
-    // contiguous run of paths, so the cuRAND state of path p + 1 (the
-    // seeded state advanced by p + 1 subsequences) comes from the saved
-    // state of path p by one cuRAND skipahead_sequence(1) instead of a full
-    // curand_init(seed, p + 1, 0), whose skip-ahead costs about one matrix
-    // product per base-4 digit of the path index.
+    // Philox: grid-stride over paths.  XORWOW: the CTA takes a contiguous run
+    // of paths, its threads side by side, and the cuRAND state of path
+    // p + blockDim comes from that of path p by one skipahead_sequence
+    // (blockDim is a power of 4: one matrix product).
     const long long nthreads = (long long)gridDim.x * blockDim.x;
-    const long long gtid = (long long)blockIdx.x * blockDim.x + tid;
-    long long p_begin = gtid, p_end = a.n_paths, p_step = nthreads;
-    if (RNG != RG_RNG_PHILOX) {
-        const long long chunk = (a.n_paths + nthreads - 1) / nthreads;
-        p_begin = gtid * chunk;
-        p_end = p_begin + chunk < a.n_paths ? p_begin + chunk : a.n_paths;
-        p_step = 1;
-    }
+    long long p_begin = (long long)blockIdx.x * blockDim.x + tid, p_end = a.n_paths, p_step = nthreads;
     curandStateXORWOW_t next_state;
-    if (RNG != RG_RNG_PHILOX && p_begin < p_end)
-        curand_init(a.seed, a.path0 + (unsigned long long)p_begin, 0ull, &next_state);
+    if (RNG != RG_RNG_PHILOX) {
+        // The states of the CTA's first blockDim paths: thread 0 skips to the
+        // CTA's first subsequence, then in each step the threads [w, 2w) take
+        // the state of the thread w below and skip w.  A full curand_init in
+        // every thread, whose skip costs up to three matrix products per
+        // base-4 digit of the path index (lanes differ in their digits), was
+        // most of the time of a call with a few paths a thread: 1e5 paths at
+        // N = 9 took 231 us, now 174; 1e6 paths 866, now 784.
+        __shared__ curandStateXORWOW_t sstate[RNG == RG_RNG_PHILOX ? 1 : kPlainThreads];
+        const long long run = ((a.n_paths - 1) / nthreads + 1) * blockDim.x;
+        p_begin = blockIdx.x * run + tid;
+        p_end = min((blockIdx.x + 1) * run, a.n_paths);
+        p_step = blockDim.x;
+        if (tid == 0) {
+            curand_init(a.seed, a.path0 + (unsigned long long)(blockIdx.x * run), 0ull, &next_state);
+            sstate[0] = next_state;
+        }
+        for (int w = 1; w < (int)blockDim.x; w <<= 1) {
+            __syncthreads();
+            if (tid >= w && tid < 2 * w) {
+                next_state = sstate[tid - w];
+                skipahead_sequence((unsigned long long)w, &next_state);
+                sstate[tid] = next_state;
+            }
+        }
+    }
     for (long long p = p_begin; p < p_end; p += p_step) {
         const unsigned long long path = a.path0 + (unsigned long long)p;
         float z[NP];
@@ -96,7 +111,7 @@ __global__ void __launch_bounds__(kPlainThreads, 2) mc_plain_small_kernel(const 
         } else {
             // this path's state as curand_init(seed, path, 0) leaves it
             curandStateXORWOW_t st = next_state;
-            if (p + 1 < p_end) skipahead_sequence(1ull, &next_state);
+            if (p + p_step < p_end) skipahead_sequence((unsigned long long)p_step, &next_state);
             for (int d = 0; d < a.horizon; d++) {
 #pragma unroll
                 for (int j = 0; j < NP; j++)
@@ -154,6 +169,21 @@ template <int NP, int RNG>
 static cudaError_t launch_np(const PlainArgs &a, int sm_count, cudaStream_t s)
 {
     auto kern = mc_plain_small_kernel<NP, RNG>;
+    if (RNG != RG_RNG_PHILOX) {
+        // Two CTAs of 256 an SM once each has at least four rounds of paths,
+        // else eight of 64, which spread few paths better and start sooner.
+        // cuRAND's FP64 normals bound both (about 74 FP64 instructions a
+        // pair: 0.72 of the 0.78 ms of 1e6 paths at N = 9).  Device time in
+        // us, 2 x 256 and 8 x 64: 1e5 paths N = 9 198 and 174, N = 50 620 and
+        // 580; 1e6 paths N = 9 784 and 811, N = 50 3529 and 4338.
+        const bool wide = a.n_paths > 4ll * 2 * 256 * sm_count;
+        const long long ctas = (wide ? 2ll : 8ll) * sm_count;
+        const int threads = wide ? kPlainThreads : 64;
+        const long long run = ((a.n_paths - 1) / (ctas * threads) + 1) * threads;
+        const long long grid = (a.n_paths - 1) / run + 1;
+        kern<<<(unsigned)grid, threads, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPlainThreads, 0);
     if (e != cudaSuccess) return e;
