@@ -44,6 +44,7 @@ struct Batch {
     bool use_graph = true;
     bool tuned = false;
     unsigned char *d_items = nullptr;
+    PhiloxBlock *d_blocks = nullptr;        // the items' Philox block tables, one after the other
     unsigned long long *d_counts = nullptr; // [count][2]
     unsigned int *d_work = nullptr;         // [0] unit counter, [1] error word
     unsigned long long *h_counts = nullptr; // pinned [count][2]
@@ -179,6 +180,7 @@ static void destroy_batch(Batch *b)
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     cudaFree(b->d_items);
+    cudaFree(b->d_blocks);
     cudaFree(b->d_counts);
     cudaFree(b->d_work);
     cudaFreeHost(b->h_counts);
@@ -237,12 +239,28 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
         if (mt > b->n_mt_max) b->n_mt_max = mt;
     }
     const int paths = tc_batch_paths(b->n_mt_max);
+    auto table_len = [](const Portfolio *p, const rg_query &q) {
+        return philox_table_len(p->n, q.draw_mode == RG_DRAWS_AGGREGATED ? 1 : q.horizon, q.path_offset, q.n_paths);
+    };
+    size_t blocks = 0;
+    for (int i = 0; i < count; i++)
+        blocks += table_len(reinterpret_cast<const Portfolio *>(items[i].portfolio), items[i].query);
+    if (blocks) e = cudaMalloc(&b->d_blocks, blocks * sizeof(PhiloxBlock));
+    if (e != cudaSuccess) {
+        destroy_batch(b);
+        return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "batch setup failed: %s",
+                         cudaGetErrorString(e));
+    }
+    PhiloxBlock *next = b->d_blocks;
     long long tile = 0;
     for (int i = 0; i < count; i++) {
         const Portfolio *p = reinterpret_cast<const Portfolio *>(items[i].portfolio);
         const rg_query &q = items[i].query;
         const int bf16 = q.precision == RG_PREC_BF16X3 ? 1 : 0;
         PlainArgs a = query_args(p, &q, b->d_counts + 2 * (size_t)i);
+        const size_t len = table_len(p, q);
+        a.blocks = len ? next : nullptr;
+        next += len;
         tc_fill_batch_item(host.data() + (size_t)i * tc_item_bytes(), a, p->d_tc[bf16], bf16,
                            q.draw_mode == RG_DRAWS_AGGREGATED, p->wmu, tile);
         tile += tc_tiles_of(q.n_paths, paths);
@@ -250,6 +268,8 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     }
     b->total_tiles = tile;
     e = cudaMemcpy(b->d_items, host.data(), host.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && blocks) e = launch_batch_tables(b->d_items, count, b->cap_stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->cap_stream);
     if (e != cudaSuccess) {
         destroy_batch(b);
         return set_error(RG_ERR_CUDA, "batch upload failed: %s", cudaGetErrorString(e));

@@ -332,6 +332,7 @@ struct QueryScratch {
     unsigned int *err = nullptr;           // [1] error word of the tensor-core kernel
     float *cand = nullptr;                 // [cap]
     unsigned long long *hist = nullptr;    // [kVarHistBins + 2]
+    PhiloxBlock *blocks = nullptr;         // room for the Philox block table, or null
     unsigned int cap = 0;
     void *base = nullptr;
 };
@@ -342,14 +343,28 @@ struct QueryHead {
 };
 static_assert(sizeof(QueryHead) == 56, "device and host layout");
 
-static cudaError_t scratch_alloc(DevCtx *ctx, QueryScratch &sc, unsigned int cap, bool with_var, cudaStream_t s)
+// Bytes for the block table of a tensor-core query with enough normals that
+// the table's own launch (about 3 us) pays: 6 % of a generator that draws
+// 1.2e12 normals a second.
+static size_t table_bytes(const Portfolio *p, const rg_query *q)
+{
+    const bool tensor = q->precision == RG_PREC_BF16X3 || q->precision == RG_PREC_FP16X3;
+    const int days = q->draw_mode == RG_DRAWS_AGGREGATED ? 1 : q->horizon;
+    if (!tensor || (double)q->n_paths * p->n * days < 1e8) return 0;
+    return sizeof(PhiloxBlock) * philox_table_len(p->n, days, q->path_offset, q->n_paths);
+}
+
+static cudaError_t scratch_alloc(DevCtx *ctx, QueryScratch &sc, unsigned int cap, bool with_var, size_t table,
+                                 cudaStream_t s)
 {
     const size_t head = sizeof(QueryHead);
     const size_t cand = with_var ? ((4 * (size_t)cap + 7) & ~(size_t)7) : 0;
     const size_t hist = with_var ? 8 * (size_t)(kVarHistBins + 2) : 0;
-    cudaError_t e = cudaMallocFromPoolAsync(&sc.base, head + cand + hist + 16, ctx->pool, s);
+    const size_t table_at = (head + cand + hist + 15) & ~(size_t)15;
+    cudaError_t e = cudaMallocFromPoolAsync(&sc.base, table_at + table + 16, ctx->pool, s);
     if (e != cudaSuccess) return e;
     char *b = (char *)sc.base;
+    sc.blocks = table ? (PhiloxBlock *)(b + table_at) : nullptr;
     sc.counts = (unsigned long long *)b;
     sc.counts2 = sc.counts + 2;
     sc.tail = sc.counts + 4;
@@ -707,7 +722,21 @@ int rg_launch_counts(const rg_portfolio *h, const rg_query *q, unsigned long lon
     if (st) return st;
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     cudaError_t e = cudaMemsetAsync(d_counts, 0, 2 * sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = launch_counting(p, q, make_args(p, q, d_counts), ctx->sm_count, s);
+    PlainArgs a = make_args(p, q, d_counts);
+    // the block table lives for this launch, in stream order; a captured
+    // launch allocates nothing and goes without
+    const size_t table = table_bytes(p, q);
+    if (e == cudaSuccess && table) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        else if (cap == cudaStreamCaptureStatusNone)
+            e = cudaMallocFromPoolAsync((void **)&a.blocks, table, ctx->pool, s);
+    }
+    if (e == cudaSuccess) e = launch_counting(p, q, a, ctx->sm_count, s);
+    if (a.blocks) {
+        const cudaError_t f = cudaFreeAsync(a.blocks, s);
+        if (e == cudaSuccess) e = f;
+    }
     if (e != cudaSuccess) return set_error(RG_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
     return RG_OK;
 }
@@ -762,9 +791,10 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
     st = admit(64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2));
     if (st) return st;
     RG_CUDA_TRY(query_res_take(ctx, &res));
-    RG_CUDA_TRY(scratch_alloc(ctx, sc, cap, want_var, s));
+    RG_CUDA_TRY(scratch_alloc(ctx, sc, cap, want_var, table_bytes(p, q), s));
     a = make_args(p, q, sc.counts);
     a.err = sc.err;
+    a.blocks = sc.blocks;
     if (want_var) {
         a.var_mode = 1;
         a.sel_bins = 1;
@@ -824,9 +854,10 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         if (need > sc.cap) {
             RG_CUDA_TRY(cudaFreeAsync(sc.base, s));
             sc.base = nullptr;
-            RG_CUDA_TRY(scratch_alloc(ctx, sc, need, true, s));
+            RG_CUDA_TRY(scratch_alloc(ctx, sc, need, true, table_bytes(p, q), s));
             a.counts = sc.counts2;
             a.err = sc.err;
+            a.blocks = sc.blocks;
             a.cand = sc.cand;
             a.cand_count = sc.cand_count;
             a.tail = sc.tail;

@@ -71,6 +71,72 @@ __device__ __forceinline__ void rg_philox2(uint4 &a, uint4 &b, const PhiloxKeys 
     }
 }
 
+// The first two rounds of Philox4x32-10 for counter (block, 0, lo, hi), split
+// by what they depend on.  With hi1(.), lo1(.) the halves of 0xCD9E8D57 x and
+// hi0, lo0 those of 0xD2511F53 x, the state after round 2 is
+//   x = hi1(hi0(block) ^ hi ^ k1[0]) ^ k0[1]  ^  lo1(lo)
+//   y = lo1(hi0(block) ^ hi ^ k1[0])
+//   z = hi0(hi1(lo) ^ k0[0])  ^  lo0(block) ^ k1[1]
+//   w = lo0(hi1(lo) ^ k0[0])
+// so for path indexes with the same high word, the left term of x, y and the
+// right term of z belong to the block alone (PhiloxBlock, with round 3's k0
+// folded into y; a table over a query's blocks is laid out once per launch)
+// and the rest to the path (PhiloxPath, with round 3's k1 folded into w).
+// A block of four words then costs 16 wide multiplies instead of 18; each
+// takes 4.2 cycles of one multiplier pipe per SM sub-partition (measured),
+// the busiest pipe of Philox.
+struct __align__(16) PhiloxBlock {
+    uint32_t x, y, z, pad;
+};
+struct PhiloxPath {
+    uint32_t x, z, w;
+};
+__host__ __device__ __forceinline__ PhiloxBlock philox_block(uint32_t block, uint32_t hi, const PhiloxKeys &k)
+{
+    const uint64_t p = (uint64_t)0xD2511F53u * block;
+    const uint64_t q = (uint64_t)0xCD9E8D57u * ((uint32_t)(p >> 32) ^ hi ^ k.k1[0]);
+    PhiloxBlock b;
+    b.x = (uint32_t)(q >> 32) ^ k.k0[1];
+    b.y = (uint32_t)q ^ k.k0[2];
+    b.z = (uint32_t)p ^ k.k1[1];
+    b.pad = 0u;
+    return b;
+}
+__device__ __forceinline__ PhiloxPath philox_path(uint32_t lo, const PhiloxKeys &k)
+{
+    const uint64_t q = (uint64_t)0xCD9E8D57u * lo;
+    const uint64_t p = (uint64_t)0xD2511F53u * ((uint32_t)(q >> 32) ^ k.k0[0]);
+    PhiloxPath c;
+    c.x = (uint32_t)q;
+    c.z = (uint32_t)(p >> 32);
+    c.w = (uint32_t)p ^ k.k1[2];
+    return c;
+}
+// State after round 3 (of 10).
+__device__ __forceinline__ uint4 philox_join(const uint4 &b, const PhiloxPath &c)
+{
+    const uint64_t p0 = (uint64_t)0xD2511F53u * (b.x ^ c.x);
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * (b.z ^ c.z);
+    return make_uint4((uint32_t)(p1 >> 32) ^ b.y, (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w, (uint32_t)p0);
+}
+// The words of two blocks of one path, rounds interleaved: the same as
+// rg_philox2 on their counters.
+__device__ __forceinline__ void rg_philox2_from(const uint4 &ta, const uint4 &tb, const PhiloxPath &path,
+                                                const PhiloxKeys &k, uint4 &a, uint4 &b)
+{
+    a = philox_join(ta, path);
+    b = philox_join(tb, path);
+#pragma unroll
+    for (int r = 3; r < 10; r++) {
+        const uint64_t p0 = (uint64_t)0xD2511F53u * a.x, p1 = (uint64_t)0xCD9E8D57u * a.z;
+        const uint64_t q0 = (uint64_t)0xD2511F53u * b.x, q1 = (uint64_t)0xCD9E8D57u * b.z;
+        a = make_uint4((uint32_t)(p1 >> 32) ^ a.y ^ k.k0[r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ a.w ^ k.k1[r],
+                       (uint32_t)p0);
+        b = make_uint4((uint32_t)(q1 >> 32) ^ b.y ^ k.k0[r], (uint32_t)q1, (uint32_t)(q0 >> 32) ^ b.w ^ k.k1[r],
+                       (uint32_t)q0);
+    }
+}
+
 __device__ __forceinline__ float rg_lg2_approx(float x)
 {
     float y;
@@ -195,7 +261,19 @@ struct PlainArgs {
     unsigned long long *tail;   // [0] tail paths, [1] sum of -w.R * 2^32 (int64 bits)
     unsigned long long *hist;   // [sel_bins + 2]
     unsigned int *err;          // device error word of the tensor-core kernel (bounded waits)
+    // room for the query's PhiloxBlock table (philox_table_len entries), or null
+    PhiloxBlock *blocks;
 };
+
+// Entries of a query's block table (block = day * ceil(N/4) + quad), or 0
+// where it is not used: the paths' high words differ or the table is longer
+// than 1 MiB.
+inline size_t philox_table_len(int n, int days, unsigned long long path0, long long n_paths)
+{
+    const unsigned long long last = path0 + (unsigned long long)(n_paths - 1);
+    const size_t len = (size_t)((n + 3) / 4) * (size_t)days;
+    return (path0 >> 32) == (last >> 32) && len <= 65536 ? len : 0;
+}
 
 // Shared-memory histogram size of the VaR pass: bins plus under/overflow.
 static constexpr int kVarHistBins = 4096;
@@ -221,7 +299,9 @@ cudaError_t launch_build_tc_tiles(const double *L64, const float *w32, int n, do
 size_t tc_scratch_len(int n);
 int tc_max_n();
 size_t tc_tile_bytes(int n);
-// batches of (portfolio, query) items in one persistent launch
+// batches of (portfolio, query) items in one persistent launch (a.blocks: room
+// for the item's block table, filled by launch_batch_tables, or null)
+cudaError_t launch_batch_tables(const void *d_items, int count, cudaStream_t s);
 void tc_fill_batch_item(void *item_out, const PlainArgs &a, const unsigned char *tiles, int bf16,
                         bool aggregated, double wmu, long long tile_begin);
 size_t tc_item_bytes();
