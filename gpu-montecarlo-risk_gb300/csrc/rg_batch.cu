@@ -17,6 +17,7 @@
 // shared and tensor memory allow) with CUDA events and keeps the fastest in
 // a JSON file (RG_TUNE_CACHE, default ./riskgpu_tune.json), which later
 // batches of the same class read.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -251,9 +252,26 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "batch setup failed: %s",
                          cudaGetErrorString(e));
     }
+    // Items go into the table by falling time of one tile: CTAs claim units in
+    // table order, so the last units are short and no CTA is left with a long
+    // one (24 portfolios, 10..600 assets, 1..20 days: 2.5 % of the launch).
+    // Results stay in the caller's order (d_counts is indexed by item).
+    std::vector<int> order((size_t)count);
+    for (int i = 0; i < count; i++) order[(size_t)i] = i;
+    auto tile_cost = [&](int i) {
+        const Portfolio *p = reinterpret_cast<const Portfolio *>(items[i].portfolio);
+        const rg_query &q = items[i].query;
+        // SM cycles: about 4 normals a cycle, or 141 cycles an MMA of 12 a (row tile, K tile) pair
+        const double days = q.draw_mode == RG_DRAWS_AGGREGATED ? 1.0 : (double)q.horizon;
+        const double gen = (double)p->n * days * paths / 4.0;
+        const double mma = 12.0 * 141.0 * tc_row_tiles_of(p->n) * tc_k_tiles_of(p->n);
+        return gen > mma ? gen : mma;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tile_cost(x) > tile_cost(y); });
     PhiloxBlock *next = b->d_blocks;
     long long tile = 0;
-    for (int i = 0; i < count; i++) {
+    for (int at = 0; at < count; at++) {
+        const int i = order[(size_t)at];
         const Portfolio *p = reinterpret_cast<const Portfolio *>(items[i].portfolio);
         const rg_query &q = items[i].query;
         const int bf16 = q.precision == RG_PREC_BF16X3 ? 1 : 0;
@@ -261,11 +279,11 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
         const size_t len = table_len(p, q);
         a.blocks = len ? next : nullptr;
         next += len;
-        tc_fill_batch_item(host.data() + (size_t)i * tc_item_bytes(), a, p->d_tc[bf16], bf16,
+        tc_fill_batch_item(host.data() + (size_t)at * tc_item_bytes(), a, p->d_tc[bf16], bf16,
                            q.draw_mode == RG_DRAWS_AGGREGATED, p->wmu, tile);
         tile += tc_tiles_of(q.n_paths, paths);
-        b->queries.push_back(q);
     }
+    for (int i = 0; i < count; i++) b->queries.push_back(items[i].query);
     b->total_tiles = tile;
     e = cudaMemcpy(b->d_items, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && blocks) e = launch_batch_tables(b->d_items, count, b->cap_stream);

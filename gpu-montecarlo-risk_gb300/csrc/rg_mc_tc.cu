@@ -691,21 +691,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) mc_tc_kernel(const __grid_const
 // overwrite its accumulator once the epilogue has read it (acc_free): only
 // the last row tile's epilogue is on the critical path.
 // Barriers (all waits bounded):
-//   tile_pub[s]  generator -> other roles: tile index and item of slot s
+//   tile_pub[s]  first generator warp -> all roles: tile index and item of slot s
 //   zfull[z]     generator -> MMA: the K tile in slot z written (one arrival
 //                per generator thread)
 //   zempty[z]    MMA -> generator: the MMAs that read slot z are complete
 //   full/empty   Lhat ring (copy completion, MMA completion)
 //   acc_full[m]  MMA -> epilogue: row tile m of the tile accumulated
 //   acc_free[m]  epilogue -> MMA: row tile m read (one arrival per warp)
-//   slot_free[s] epilogue -> generator: the tile in slot s is finished
-// The K-tile number g, use counts per row tile and per item slot (the same
+//   slot_free[s] epilogue -> first generator warp: the tile in slot s is finished
+// The K-tile number g, use counts per row tile and per tile slot (the same
 // on both sides of each barrier) give the phase parities, since items of a
 // batch differ in size.  The tile index is read after tile_pub, never after
 // zfull[0]: slot s is republished only after the epilogue finished the tile
 // that used it, so no waiter can fall a whole phase behind.
 static constexpr int kWsThreads = 1024;
 static constexpr int kWsEpiWarps = 4;
+static constexpr unsigned kWsTileSlots = 3; // path tiles published: generated, multiplied or read back, next
 static constexpr int kWsMmaWarp = 4;
 static constexpr int kTcMaxMt = (kTcMaxKt * kTcKt + 1 + kTcRows - 1) / kTcRows;
 // Paths per tile P (the MMA's N): the widest of 128, 96, 64 at which the
@@ -771,17 +772,16 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
     __shared__ __align__(8) uint64_t zfull[kWsZSlots], zempty[kWsZSlots];
     __shared__ __align__(8) uint64_t acc_full[kTcMaxMt], acc_free[kTcMaxMt];
-    __shared__ __align__(8) uint64_t tile_pub[2], slot_free[2], drain_bar;
+    __shared__ __align__(8) uint64_t tile_pub[kWsTileSlots], slot_free[kWsTileSlots], drain_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ int sS[P];
     __shared__ float sPort[P];
     // set by a role whose bounded wait ran out; the others then make no
     // further waits and finish
     __shared__ int tm_abort;
-    __shared__ long long s_tile[2];
-    __shared__ long long s_unit;
+    __shared__ long long s_tile[kWsTileSlots];
     __shared__ unsigned long long sacc[4];
-    __shared__ __align__(16) TcItem s_item[BATCH ? 2 : 1];
+    __shared__ __align__(16) TcItem s_item[BATCH ? kWsTileSlots : 1];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ncols = b.tmem_cols;
@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             mbar_init(&acc_full[m], 1);
             mbar_init(&acc_free[m], kWsEpiWarps);
         }
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < kWsTileSlots; s++) {
             mbar_init(&tile_pub[s], 1);
             mbar_init(&slot_free[s], 1);
         }
@@ -827,84 +827,109 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
 
     if (warp >= kWsGenWarp0) {
         // ======================= generator =======================
-        // gab: this thread's abort flag.  Generator threads do not meet at
-        // K-tile boundaries, so a timeout is first local; the reduction
-        // barrier at the start of each tile makes it uniform before any
-        // decision that changes barrier participation.
+        // Threads of the role never meet: each walks its items of every K
+        // tile, in order across the path tiles, and arrives on the K tile's
+        // zfull.  Items are dealt round robin over all K tiles of the CTA, so
+        // every thread draws the same number in the end; with a barrier and a
+        // fresh deal at each path tile, tiles of few items (N = 300: 4.4 a
+        // thread) left threads idle for up to a fifth of it (24 portfolios of
+        // 10..600 assets in one launch: 5 % of its time).  A thread whose
+        // bounded wait runs out raises tm_abort and leaves; the others and
+        // the other roles follow at their next wait.
         const int gtid = tid - 32 * kWsGenWarp0;
         unsigned g0 = 0; // K tiles of the previous path tiles
-        int gab = 0;
         long long unit = -1, unit_end = 0, next_static = blockIdx.x;
-        for (unsigned j = 0;; j++) {
-            const int slot = j & 1;
-            // the slot must be free (epilogue of tile j-2 done); after an
-            // abort on either side no wait is made
-            if (!gab && !tm_abort && !mbar_wait(&slot_free[slot], ((j >> 1) & 1u) ^ 1u)) {
-                atomicOr(b.err, 8u);
-                gab = 1;
-            }
-            gab = named_sync_or(2, kWsGenThreads, gab);
-            if (gtid == 0) {
-                long long tile = -1;
-                if (!gab && !tm_abort) {
-                    if (b.work) {
-                        if (unit < 0 || unit_end <= 0) {
-                            unit = (long long)atomicAdd(b.work, 1u);
-                            unit_end = b.unit_tiles;
-                        }
-                        tile = unit * b.unit_tiles + (b.unit_tiles - unit_end);
-                        unit_end--;
-                        if (tile >= total || unit * b.unit_tiles >= total) tile = -1;
-                    } else {
-                        tile = next_static;
-                        next_static += gridDim.x;
-                        if (tile >= total) tile = -1;
+        bool more = true; // the last published tile was not the end
+        // The first generator warp claims tiles and publishes each (or the
+        // end, -1) to every role, a path tile ahead of its generation, so
+        // nobody waits for a claim.
+        auto publish = [&](unsigned j) -> bool {
+            const int slot = (int)(j % kWsTileSlots);
+            long long tile = -1;
+            int item = 0, ok = 1;
+            if (lane == 0) {
+                // the slot is free once the epilogue of tile j - 3 is done
+                if (tm_abort || !mbar_wait(&slot_free[slot], ((j / kWsTileSlots) & 1u) ^ 1u)) {
+                    if (!tm_abort) atomicOr(b.err, 8u);
+                    ok = 0;
+                } else if (b.work) {
+                    if (unit < 0 || unit_end <= 0) {
+                        unit = (long long)atomicAdd(b.work, 1u);
+                        unit_end = b.unit_tiles;
                     }
+                    tile = unit * b.unit_tiles + (b.unit_tiles - unit_end);
+                    unit_end--;
+                } else {
+                    tile = next_static;
+                    next_static += gridDim.x;
                 }
-                s_tile[slot] = tile;
+                if (tile >= total) tile = -1;
                 if (BATCH && tile >= 0) {
-                    int lo = 0, hi = n_items - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (b.items[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+                    int hi = n_items - 1;
+                    while (item < hi) {
+                        const int mid = (item + hi + 1) >> 1;
+                        if (b.items[mid].tile_begin <= tile) item = mid; else hi = mid - 1;
                     }
-                    s_unit = lo;
                 }
             }
-            named_sync(2, kWsGenThreads);
-            const long long tile = s_tile[slot];
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) return false;
+            tile = __shfl_sync(0xffffffffu, tile, 0);
             if (BATCH && tile >= 0) { // stage the item in its slot
-                const int *src = reinterpret_cast<const int *>(&b.items[s_unit]);
+                item = __shfl_sync(0xffffffffu, item, 0);
+                const int *src = reinterpret_cast<const int *>(&b.items[item]);
                 int *dst = reinterpret_cast<int *>(&s_item[slot]);
-                for (int w = gtid; w < (int)(sizeof(TcItem) / 4); w += kWsGenThreads) dst[w] = src[w];
-                named_sync(2, kWsGenThreads);
+                for (int w = lane; w < (int)(sizeof(TcItem) / 4); w += 32) dst[w] = src[w];
             }
-            // publish the tile (or the end, -1) to the other roles
-            if (gtid == 0) mbar_arrive(&tile_pub[slot]);
-            if (tile < 0) break; // uniform: every thread read the same s_tile
+            __syncwarp();
+            if (lane == 0) {
+                s_tile[slot] = tile;
+                mbar_arrive(&tile_pub[slot]);
+            }
+            more = tile >= 0;
+            return true;
+        };
+        constexpr int kPerKt = P * (kTcKt / 8); // items of a K tile
+        int first = gtid;                       // this thread's first item of the next K tile
+        bool dead = false;
+        for (unsigned j = 0; !dead; j++) {
+            if (warp == kWsGenWarp0) {
+                if ((j == 0 && !publish(0)) || (more && !publish(j + 1))) {
+                    tm_abort = 1;
+                    break;
+                }
+            }
+            const int slot = (int)(j % kWsTileSlots);
+            if (tm_abort || !mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
+                if (!tm_abort) atomicOr(b.err, 8u);
+                dead = true;
+            }
+            // (the publishing warp stays whole: its lanes leave together)
+            if (warp == kWsGenWarp0) dead = __any_sync(0xffffffffu, dead);
+            if (dead) {
+                tm_abort = 1;
+                break;
+            }
+            const long long tile = s_tile[slot];
+            if (tile < 0) break;
             const TcItem &it = BATCH ? s_item[slot] : b.one;
             const int n = it.n, nq = (n + 3) >> 2, n_kt = it.n_kt;
             const long long p0 = (tile - it.tile_begin) * P;
-            // each thread walks its items of the tile in K-tile order and
-            // arrives on zfull[kt] once it has written its share of kt (no
-            // group barrier, so no thread idles at K-tile boundaries)
+            const int days = it.aggregated ? 1 : it.horizon;
             for (int kt = 0; kt < n_kt; kt++) {
                 const unsigned g = g0 + (unsigned)kt;
                 const int zs = (int)(g % kWsZSlots);
                 // the MMAs on the slot's previous K tile (g - kWsZSlots) are done
-                if (!gab && !tm_abort && !mbar_wait(&zempty[zs], ((g / kWsZSlots) & 1u) ^ 1u)) {
-                    atomicOr(b.err, 16u);
-                    gab = 1;
+                if (tm_abort || !mbar_wait(&zempty[zs], ((g / kWsZSlots) & 1u) ^ 1u)) {
+                    if (!tm_abort) atomicOr(b.err, 16u);
+                    tm_abort = 1;
+                    dead = true;
+                    break;
                 }
                 // an item is one path's pair of adjacent quads (8 K columns,
-                // one 16-byte chunk of the swizzled Z row); items of kt are
-                // i = kt*per_kt + local, assigned round robin over the whole
-                // tile (i % kWsGenThreads == gtid)
-                const int per_kt = P * (kTcKt / 8);
-                int first = gtid - (kt * per_kt) % kWsGenThreads;
-                if (first < 0) first += kWsGenThreads;
-                const int days = it.aggregated ? 1 : it.horizon;
-                for (int item = first; item < per_kt; item += kWsGenThreads) {
+                // one 16-byte chunk of the swizzled Z row)
+                int item = first;
+                for (; item < kPerKt; item += kWsGenThreads) {
                     const int qp = item / P, p = item - qp * P, q = kt * (kTcKt / 4) + 2 * qp;
                     const unsigned long long path = it.path0 + (unsigned long long)(p0 + p);
                     const uint32_t plo = (uint32_t)path, phi = (uint32_t)(path >> 32);
@@ -936,9 +961,11 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                     *reinterpret_cast<uint4 *>(zhi + off) = make_uint4(hz.x, hz.y, hy.x, hy.y);
                     *reinterpret_cast<uint4 *>(zlo + off) = make_uint4(lz.x, lz.y, ly.x, ly.y);
                 }
+                first = item - kPerKt;
                 fence_async_shared(); // this thread's writes -> async proxy (tensor cores)
                 mbar_arrive(&zfull[zs]);
             }
+            if (warp == kWsGenWarp0) dead = __any_sync(0xffffffffu, dead);
             g0 += (unsigned)n_kt;
         }
     } else if (SPLIT && warp == kWsMmaWarp + 1) {
@@ -947,8 +974,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             unsigned prod_iter = 0;
             int skipped = -1; // the stage left unfilled by the fault injection
             for (unsigned j = 0; !tm_abort; j++) {
-                const int slot = j & 1;
-                if (!mbar_wait(&tile_pub[slot], (j >> 1) & 1u)) {
+                const int slot = (int)(j % kWsTileSlots);
+                if (!mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
                     atomicOr(b.err, 32u);
                     tm_abort = 1;
                     break;
@@ -1001,8 +1028,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                 while (!p_end && pi < ci + kStages) {
                     const bool must = need && pi == ci;
                     if (!p_live) {
-                        const int ps = (int)(pj & 1u);
-                        const unsigned par = (pj >> 1) & 1u;
+                        const int ps = (int)(pj % kWsTileSlots);
+                        const unsigned par = (pj / kWsTileSlots) & 1u;
                         if (!mbar_test(&tile_pub[ps], par)) {
                             if (!must) return true;
                             if (!mbar_wait(&tile_pub[ps], par)) return false;
@@ -1054,8 +1081,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             unsigned rs = 0, rph = 0;  // Lhat ring: stage and phase parity of pair ci
             const uint32_t lst_lo = sw128_desc_lo(smem_u32(lst));
             for (unsigned j = 0; !tm_abort; j++) {
-                const int slot = j & 1;
-                if (!mbar_wait(&tile_pub[slot], (j >> 1) & 1u)) {
+                const int slot = (int)(j % kWsTileSlots);
+                if (!mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
                     atomicOr(b.err, 32u);
                     tm_abort = 1;
                     break;
@@ -1125,9 +1152,9 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
         // ======================= epilogue (warps 0-3) =======================
         unsigned apar = 0; // bit m: parity of the uses of row tile m
         for (unsigned j = 0;; j++) {
-            const int slot = j & 1;
+            const int slot = (int)(j % kWsTileSlots);
             int ab = 0;
-            if (!tm_abort && !mbar_wait(&tile_pub[slot], (j >> 1) & 1u)) {
+            if (!tm_abort && !mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
                 atomicOr(b.err, 32u);
                 ab = 1;
             }
