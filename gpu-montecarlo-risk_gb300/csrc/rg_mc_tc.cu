@@ -749,6 +749,34 @@ __device__ __forceinline__ int tc_kts(int mt, int n_mt, int n_kt)
     return (mt == n_mt - 1) ? n_kt : min(n_kt, (kTcRows * (mt + 1) + kTcKt - 1) / kTcKt);
 }
 
+// 32 accumulator columns of this warp's TMEM lanes (one row a lane).
+__device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&v)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Bit (31 - c) of lane l's word -> bit l of lane c's word, c = 0..31: the
+// transpose of the 32 x 32 bit matrix whose row l is lane l's word reversed.
+__device__ __forceinline__ uint32_t warp_bit_transpose(uint32_t x, int lane)
+{
+    x = __brev(x);
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const uint32_t low = 0xffffffffu / ((1u << j) + 1u); // the low j bits of every 2 j
+        const uint32_t keep = (lane & j) ? ~low : low;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (x & keep) | (__funnelshift_l(y, y, (lane & j) ? 32 - j : j) & ~keep);
+    }
+    return x;
+}
+
 template <bool VAR, bool BATCH, int P, bool SPLIT>
 __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_constant__ TcBatch b)
 {
@@ -1167,6 +1195,18 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             const TcItem &it = BATCH ? s_item[slot] : b.one;
             const int n = it.n, n_mt = it.n_mt;
             bool dead = false;
+            // This lane's crash count of column 32 g + c, over the row tiles, is
+            // bit 31 - c of three bit planes (at most kTcMaxMt = 6 rows): two
+            // instructions an accumulator (subtract the threshold, shift the
+            // sign in) and one addition of planes a 32-column group.  A ballot,
+            // a population count and a select for every column of every row
+            // tile took about five, and with one draw an asset the epilogue's
+            // four warps held up the next tile's MMAs.
+            constexpr int kG = P / 32;
+            static_assert(kTcMaxMt < 8, "three bit planes");
+            uint32_t c0[kG], c1[kG], c2[kG];
+#pragma unroll
+            for (int g = 0; g < kG; g++) c0[g] = c1[g] = c2[g] = 0u;
             for (int mt = 0; mt < n_mt; mt++) {
                 int wab = 0;
                 if (!tm_abort && !mbar_wait(&acc_full[mt], (apar >> mt) & 1u)) {
@@ -1179,30 +1219,26 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                 }
                 tc_fence_after();
                 const int row = mt * kTcRows + warp * 32 + lane;
-                const bool asset = row < n;
-                const float thr = asset ? tc_threshold(it, row) : 0.f;
+                // d < thr is the sign of d - thr: exactly, with -0 for a zero
+                // threshold (-0 - +0 is -0) and -inf for rows that are no asset
+                float thr = row < n ? tc_threshold(it, row) : -__int_as_float(0x7f800000);
+                if (thr == 0.f) thr = -0.f;
 #pragma unroll
-                for (int cb = 0; cb < P / 16; cb++) {
-                    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * P + cb * 16);
-                    uint32_t v[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                                   "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                                   "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                                 : "r"(taddr));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    int cnt = 0;
+                for (int g = 0; g < kG; g++) {
+                    uint32_t v[32];
+                    tc_load32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * P + g * 32), v);
+                    uint32_t m = 0u;
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        const unsigned m = __ballot_sync(0xffffffffu, asset && __uint_as_float(v[c]) < thr);
-                        if (lane == c) cnt = __popc(m);
-                    }
-                    if (lane < 16 && cnt) atomicAdd(&sS[cb * 16 + lane], cnt);
+                    for (int c = 0; c < 32; c++)
+                        m = __funnelshift_l(__float_as_uint(__uint_as_float(v[c]) - thr), m, 1);
+                    const uint32_t t0 = c0[g] & m, t1 = c1[g] & t0;
+                    c0[g] ^= m;
+                    c1[g] ^= t0;
+                    c2[g] ^= t1;
                     if (row == n) {
 #pragma unroll
-                        for (int c = 0; c < 16; c++)
-                            sPort[cb * 16 + c] = it.hwmu_f + __uint_as_float(v[c]) * (1.0f / kTcLScale);
+                        for (int c = 0; c < 32; c++)
+                            sPort[g * 32 + c] = it.hwmu_f + __uint_as_float(v[c]) * (1.0f / kTcLScale);
                     }
                 }
                 // this warp's reads of row tile mt are complete: the next tile may overwrite it
@@ -1213,6 +1249,14 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             if (dead) {
                 tm_abort = 1;
                 break;
+            }
+#pragma unroll
+            for (int g = 0; g < kG; g++) {
+                // lane c: rows of this warp that crash in column 32 g + c
+                int cnt = __popc(warp_bit_transpose(c0[g], lane));
+                if (n_mt > 1) cnt += 2 * __popc(warp_bit_transpose(c1[g], lane));
+                if (n_mt > 3) cnt += 4 * __popc(warp_bit_transpose(c2[g], lane));
+                if (cnt) atomicAdd(&sS[g * 32 + lane], cnt);
             }
             apar ^= (1u << n_mt) - 1u;
             named_sync(1, 32 * kWsEpiWarps); // every count of the tile is in sS / sPort
