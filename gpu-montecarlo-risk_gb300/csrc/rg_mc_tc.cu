@@ -219,39 +219,49 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                  "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate));
 }
-// The 12 MMAs of one (row tile, K tile) pair in one block: for each of the
-// four 16-element K steps, Lhi.Zhi (accumulating unless acc_first == 0 on the
-// first step), Lhi.Zlo and Llo.Zhi.  Descriptors are passed as their low
-// words (sw128_desc_lo); a K step is 32 bytes (+2), the lo part of an Lhat
-// tile 16 KB (+1024) further.
+// One lane of a whole warp (the same one at every call).  Code under
+// `if (elect_one())` is known to run in one lane, so the operands that
+// tcgen05.mma and the bulk copies take from uniform registers are formed there;
+// under `if (lane == 0)` each operand is moved lane by lane: 157 cycles an MMA
+// of 64 beside 27 busy warps, 72 with elect.sync.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ void tc_mma_acc(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.eq.b32 p, 0, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                 "l"(a_desc), "l"(b_desc), "r"(idesc));
+}
+// The 12 MMAs of one (row tile, K tile) pair: for each of the four 16-element
+// K steps, Lhi.Zhi (accumulating unless acc_first == 0 on the first step),
+// Lhi.Zlo and Llo.Zhi.  Descriptors are passed as their low words
+// (sw128_desc_lo); a K step is 32 bytes (+2), the lo part of an Lhat tile
+// 16 KB (+1024) further.
 __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t zh_lo, uint32_t zl_lo,
                                             uint32_t idesc, uint32_t acc_first)
 {
-    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b32 ta, tl, th, tz;\n\t.reg .b64 da, dl, dh, dz;\n\t"
-                 "setp.ne.b32 p, %5, 0;\n\t"
-                 "setp.eq.b32 q, %5, %5;\n\t"
-                 "add.u32 ta, %1, 0;\n\tadd.u32 tl, %1, 1024;\n\tadd.u32 th, %2, 0;\n\tadd.u32 tz, %3, 0;\n\t"
-                 "mov.b64 da, {ta, %6};\n\tmov.b64 dl, {tl, %6};\n\tmov.b64 dh, {th, %6};\n\tmov.b64 dz, {tz, %6};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dh, %4, p;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dz, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], dl, dh, %4, q;\n\t"
-                 "add.u32 ta, %1, 2;\n\tadd.u32 tl, %1, 1026;\n\tadd.u32 th, %2, 2;\n\tadd.u32 tz, %3, 2;\n\t"
-                 "mov.b64 da, {ta, %6};\n\tmov.b64 dl, {tl, %6};\n\tmov.b64 dh, {th, %6};\n\tmov.b64 dz, {tz, %6};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dh, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dz, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], dl, dh, %4, q;\n\t"
-                 "add.u32 ta, %1, 4;\n\tadd.u32 tl, %1, 1028;\n\tadd.u32 th, %2, 4;\n\tadd.u32 tz, %3, 4;\n\t"
-                 "mov.b64 da, {ta, %6};\n\tmov.b64 dl, {tl, %6};\n\tmov.b64 dh, {th, %6};\n\tmov.b64 dz, {tz, %6};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dh, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dz, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], dl, dh, %4, q;\n\t"
-                 "add.u32 ta, %1, 6;\n\tadd.u32 tl, %1, 1030;\n\tadd.u32 th, %2, 6;\n\tadd.u32 tz, %3, 6;\n\t"
-                 "mov.b64 da, {ta, %6};\n\tmov.b64 dl, {tl, %6};\n\tmov.b64 dh, {th, %6};\n\tmov.b64 dz, {tz, %6};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dh, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dz, %4, q;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], dl, dh, %4, q;\n\t"
-                 "}"
-                 ::"r"(d_tmem), "r"(a_lo), "r"(zh_lo), "r"(zl_lo), "r"(idesc), "r"(acc_first), "r"(kSw128DescHi));
+    constexpr uint64_t hi = (uint64_t)kSw128DescHi << 32;
+    uint64_t da[4], dl[4], dh[4], dz[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        da[k] = hi | (a_lo + 2 * k);
+        dl[k] = hi | (a_lo + 1024 + 2 * k);
+        dh[k] = hi | (zh_lo + 2 * k);
+        dz[k] = hi | (zl_lo + 2 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (k == 0) tc_mma(d_tmem, da[k], dh[k], idesc, acc_first);
+        else tc_mma_acc(d_tmem, da[k], dh[k], idesc);
+        tc_mma_acc(d_tmem, da[k], dz[k], idesc);
+        tc_mma_acc(d_tmem, dl[k], dh[k], idesc);
+    }
 }
 __device__ __forceinline__ void tc_commit(uint64_t *bar)
 {
@@ -672,12 +682,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) mc_tc_kernel(const __grid_const
 // Warp-specialised form of the same computation.  1024 threads:
 //   warps 0-3    epilogue: warp w reads TMEM lanes 32 w .. +31 of a row tile
 //                as soon as that row tile is fully accumulated;
-//   warp 4       lane 0 issues the MMAs and, unless SPLIT, streams the Lhat
-//                tiles into the ring (bulk copies issued between MMA pairs
-//                whenever a stage is free);
-//   warp 5       SPLIT: lane 0 streams the Lhat tiles (used when the MMAs
-//                bound the kernel, so refills never wait for the MMA thread)
-//   warps 5|6-31 (864 | 832 threads) generator: draws the normals one
+//   warp 4       issues the MMAs and, unless SPLIT, streams the Lhat tiles
+//                into the ring (bulk copies issued between MMA pairs whenever
+//                a stage is free);
+//   warps 5, 6   SPLIT (used when the MMAs bound the kernel): warp 5 streams
+//                the Lhat tiles, warp 6 issues the odd row tiles' MMAs
+//   warps 5|7-31 (864 | 800 threads) generator: draws the normals one
 //                64-column K tile at a time into a ring of K-tile slots, a
 //                thread drawing one path's two adjacent quads at a time.
 // The MMAs run K-tile-outer (for each K tile, every row tile that needs it),
@@ -694,7 +704,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) mc_tc_kernel(const __grid_const
 //   tile_pub[s]  first generator warp -> all roles: tile index and item of slot s
 //   zfull[z]     generator -> MMA: the K tile in slot z written (one arrival
 //                per generator thread)
-//   zempty[z]    MMA -> generator: the MMAs that read slot z are complete
+//   zempty[z]    MMA -> generator: the MMAs that read slot z are complete (one
+//                arrival per issuer)
 //   full/empty   Lhat ring (copy completion, MMA completion)
 //   acc_full[m]  MMA -> epilogue: row tile m of the tile accumulated
 //   acc_free[m]  epilogue -> MMA: row tile m read (one arrival per warp)
@@ -783,9 +794,13 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     using Sh = WsShape<P>;
     constexpr int kStages = Sh::kStages, kZB = Sh::kZBytes, kWsZSlots = Sh::kZSlots;
     // SPLIT: warp 5 streams the Lhat tiles (when the MMAs bound the kernel,
-    // refills never wait for the MMA thread); otherwise the MMA thread
-    // issues the copies too and warp 5 draws normals
-    constexpr int kWsGenWarp0 = SPLIT ? 6 : 5;
+    // refills never wait for the MMA warp) and warps 4 and 6 issue the MMAs of
+    // the even and the odd row tiles (an issuer's waits and commits between
+    // two pairs cost about as much as half a pair's MMAs, beside 27 other
+    // warps); otherwise warp 4 issues MMAs and copies and warps 5 and 6 draw
+    // normals
+    constexpr int kWsGenWarp0 = SPLIT ? 7 : 5;
+    constexpr int kIssuers = SPLIT ? 2 : 1;
     constexpr int kWsGenThreads = kWsThreads - 32 * kWsGenWarp0;
     // days drawn side by side in the daily form: N = 600, H = 10, 4e6 paths
     // 19.4 -> 18.7 ms (3 days 18.8, 5 days 18.8); the aggregated form draws one
@@ -800,7 +815,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
     __shared__ __align__(8) uint64_t zfull[kWsZSlots], zempty[kWsZSlots];
     __shared__ __align__(8) uint64_t acc_full[kTcMaxMt], acc_free[kTcMaxMt];
-    __shared__ __align__(8) uint64_t tile_pub[kWsTileSlots], slot_free[kWsTileSlots], drain_bar;
+    __shared__ __align__(8) uint64_t tile_pub[kWsTileSlots], slot_free[kWsTileSlots], drain_bar[kIssuers];
     __shared__ uint32_t tmem_base_sh;
     __shared__ int sS[P];
     __shared__ float sPort[P];
@@ -825,7 +840,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
         }
         for (int z = 0; z < kWsZSlots; z++) {
             mbar_init(&zfull[z], kWsGenThreads);
-            mbar_init(&zempty[z], 1);
+            mbar_init(&zempty[z], kIssuers);
         }
         for (int m = 0; m < kTcMaxMt; m++) {
             mbar_init(&acc_full[m], 1);
@@ -835,7 +850,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             mbar_init(&tile_pub[s], 1);
             mbar_init(&slot_free[s], 1);
         }
-        mbar_init(&drain_bar, 1);
+        for (int i = 0; i < kIssuers; i++) mbar_init(&drain_bar[i], 1);
         tm_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -998,183 +1013,202 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
         }
     } else if (SPLIT && warp == kWsMmaWarp + 1) {
         // ======================= Lhat producer =======================
-        if (lane == 0) {
-            unsigned prod_iter = 0;
-            int skipped = -1; // the stage left unfilled by the fault injection
-            for (unsigned j = 0; !tm_abort; j++) {
-                const int slot = (int)(j % kWsTileSlots);
-                if (!mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
-                    atomicOr(b.err, 32u);
-                    tm_abort = 1;
-                    break;
-                }
-                if (s_tile[slot] < 0) break;
-                const TcItem &it = BATCH ? s_item[slot] : b.one;
-                const int n_kt = it.n_kt, n_mt = it.n_mt;
-                for (int kt = 0; kt < n_kt && !tm_abort; kt++) {
-                    for (int mt = 0; mt < n_mt; mt++) {
-                        if (kt >= tc_kts(mt, n_mt, n_kt)) continue;
-                        const int s = prod_iter % kStages;
-                        if (tm_abort || !mbar_wait(&empty_bar[s], ((prod_iter / kStages) & 1u) ^ 1u)) {
-                            atomicOr(b.err, 1u);
-                            tm_abort = 1;
-                            break;
-                        }
-                        if (b.inject_stall && prod_iter == 1) { // never filled: the consumer's wait runs out
-                            skipped = (int)prod_iter++;
-                            continue;
-                        }
+        // (the whole warp in step, one elected lane issuing, as the MMA warp)
+        unsigned prod_iter = 0;
+        int skipped = -1; // the stage left unfilled by the fault injection
+        auto same = [](int v) -> int { return __shfl_sync(0xffffffffu, v, 0); };
+        auto wait = [&](uint64_t *bar, unsigned par) -> bool { return same(mbar_wait(bar, par) ? 1 : 0) != 0; };
+        bool dead = false;
+        for (unsigned j = 0; !dead && !same(tm_abort); j++) {
+            const int slot = (int)(j % kWsTileSlots);
+            if (!wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
+                if (lane == 0) atomicOr(b.err, 32u);
+                tm_abort = 1;
+                break;
+            }
+            if (same(s_tile[slot] < 0)) break;
+            const TcItem &it = BATCH ? s_item[slot] : b.one;
+            const int n_kt = same(it.n_kt), n_mt = same(it.n_mt);
+            for (int kt = 0; kt < n_kt && !dead; kt++) {
+                for (int mt = 0; mt < n_mt; mt++) {
+                    if (kt >= tc_kts(mt, n_mt, n_kt)) continue;
+                    const int s = (int)(prod_iter % kStages);
+                    if (same(tm_abort) || !wait(&empty_bar[s], ((prod_iter / kStages) & 1u) ^ 1u)) {
+                        if (lane == 0) atomicOr(b.err, 1u);
+                        tm_abort = 1;
+                        dead = true;
+                        break;
+                    }
+                    if (b.inject_stall && prod_iter == 1) { // never filled: the consumer's wait runs out
+                        skipped = (int)prod_iter++;
+                        continue;
+                    }
+                    if (elect_one()) {
                         mbar_expect_tx(&full_bar[s], 2 * kTcTileBytes);
                         const unsigned char *src = it.tiles + ((size_t)(mt * n_kt + kt) * 2) * kTcTileBytes;
                         unsigned char *dst = lst + (size_t)s * 2 * kTcTileBytes;
                         bulk_copy(dst, src, kTcTileBytes, &full_bar[s]);
                         bulk_copy(dst + kTcTileBytes, src + kTcTileBytes, kTcTileBytes, &full_bar[s]);
-                        prod_iter++;
                     }
+                    prod_iter++;
                 }
             }
-            // the copies still in flight land before the kernel ends
-            for (unsigned i = prod_iter > kStages ? prod_iter - kStages : 0; i < prod_iter; i++)
-                if ((int)i != skipped) mbar_wait(&full_bar[i % kStages], (i / kStages) & 1u);
         }
+        // the copies still in flight land before the kernel ends
+        for (unsigned i = prod_iter > kStages ? prod_iter - kStages : 0; i < prod_iter; i++)
+            if ((int)i != skipped) mbar_wait(&full_bar[i % kStages], (i / kStages) & 1u);
         __syncwarp();
-    } else if (warp == kWsMmaWarp) {
+    } else if (warp == kWsMmaWarp || (SPLIT && warp == kWsMmaWarp + 2)) {
         // ============ MMA issue (and, unless SPLIT, the Lhat copies) ============
         // Pairs (row tile, K tile) are numbered in consumption order across
         // tiles: pi copies issued, ci pairs multiplied.  pump() issues copies
         // while the ring has room, probing its barriers without blocking; it
         // blocks only when the next pair to multiply has no copy yet (need).
         // The copy cursor enters a tile only once that tile is published.
-        if (lane == 0) {
-            unsigned pi = 0, ci = 0;
-            int skipped = -1;             // the pair left unfilled by the fault injection
-            unsigned pj = 0;              // tile (sequence number) of the copy cursor
-            bool p_live = false, p_end = false;
-            int pkt = 0, pmt = 0, p_nkt = 0, p_nmt = 0;
-            const unsigned char *p_tiles = nullptr;
-            auto pump = [&](bool need) -> bool {
-                while (!p_end && pi < ci + kStages) {
-                    const bool must = need && pi == ci;
-                    if (!p_live) {
-                        const int ps = (int)(pj % kWsTileSlots);
-                        const unsigned par = (pj / kWsTileSlots) & 1u;
-                        if (!mbar_test(&tile_pub[ps], par)) {
-                            if (!must) return true;
-                            if (!mbar_wait(&tile_pub[ps], par)) return false;
-                        }
-                        if (s_tile[ps] < 0) {
-                            p_end = true;
-                            return true;
-                        }
-                        const TcItem &pit = BATCH ? s_item[ps] : b.one;
-                        p_nkt = pit.n_kt;
-                        p_nmt = pit.n_mt;
-                        p_tiles = pit.tiles;
-                        pkt = 0;
-                        pmt = 0; // (K tile 0, row tile 0) is always a pair
-                        p_live = true;
-                    }
-                    const int st = (int)(pi % kStages);
-                    const unsigned eph = ((pi / kStages) & 1u) ^ 1u;
-                    if (!mbar_test(&empty_bar[st], eph)) {
+        //
+        // The whole warp runs this role in step, every value the same in all
+        // lanes (what is read from shared memory is taken from lane 0), and
+        // one elected lane issues the copies, MMAs and commits (elect_one).
+        const int me = __shfl_sync(0xffffffffu, warp == kWsMmaWarp ? 0 : 1, 0);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        auto same = [](int v) -> int { return __shfl_sync(0xffffffffu, v, 0); };
+        auto wait = [&](uint64_t *bar, unsigned par) -> bool { return same(mbar_wait(bar, par) ? 1 : 0) != 0; };
+        auto test = [&](uint64_t *bar, unsigned par) -> bool { return same(mbar_test(bar, par) ? 1 : 0) != 0; };
+        auto give_up = [&](unsigned bit) {
+            if (lane == 0) atomicOr(b.err, bit);
+            tm_abort = 1;
+        };
+        unsigned pi = 0, ci = 0;
+        int skipped = -1;             // the pair left unfilled by the fault injection
+        unsigned pj = 0;              // tile (sequence number) of the copy cursor
+        bool p_live = false, p_end = false;
+        int pkt = 0, pmt = 0, p_nkt = 0, p_nmt = 0;
+        const unsigned char *p_tiles = nullptr;
+        auto pump = [&](bool need) -> bool {
+            while (!p_end && pi < ci + kStages) {
+                const bool must = need && pi == ci;
+                if (!p_live) {
+                    const int ps = (int)(pj % kWsTileSlots);
+                    const unsigned par = (pj / kWsTileSlots) & 1u;
+                    if (!test(&tile_pub[ps], par)) {
                         if (!must) return true;
-                        if (!mbar_wait(&empty_bar[st], eph)) return false;
+                        if (!wait(&tile_pub[ps], par)) return false;
                     }
-                    if (b.inject_stall && pi == 1) { // never filled: the MMA side's wait runs out
-                        skipped = (int)pi;
-                    } else {
-                        mbar_expect_tx(&full_bar[st], 2 * kTcTileBytes);
-                        const unsigned char *src = p_tiles + ((size_t)(pmt * p_nkt + pkt) * 2) * kTcTileBytes;
-                        unsigned char *dst = lst + (size_t)st * 2 * kTcTileBytes;
-                        bulk_copy(dst, src, kTcTileBytes, &full_bar[st]);
-                        bulk_copy(dst + kTcTileBytes, src + kTcTileBytes, kTcTileBytes, &full_bar[st]);
+                    if (same(s_tile[ps] < 0)) {
+                        p_end = true;
+                        return true;
                     }
-                    pi++;
-                    // next pair: row tiles that need K tile pkt form a suffix of 0..n_mt-1
-                    do {
-                        if (++pmt == p_nmt) {
-                            pmt = 0;
-                            ++pkt;
-                        }
-                    } while (pkt < p_nkt && pkt >= tc_kts(pmt, p_nmt, p_nkt));
-                    if (pkt == p_nkt) {
-                        p_live = false;
-                        pj++;
-                    }
+                    const TcItem &pit = BATCH ? s_item[ps] : b.one;
+                    p_nkt = same(pit.n_kt);
+                    p_nmt = same(pit.n_mt);
+                    p_tiles = pit.tiles;
+                    pkt = 0;
+                    pmt = 0; // (K tile 0, row tile 0) is always a pair
+                    p_live = true;
                 }
-                return true;
-            };
+                const int st = (int)(pi % kStages);
+                const unsigned eph = ((pi / kStages) & 1u) ^ 1u;
+                if (!test(&empty_bar[st], eph)) {
+                    if (!must) return true;
+                    if (!wait(&empty_bar[st], eph)) return false;
+                }
+                if (b.inject_stall && pi == 1) { // never filled: the MMA side's wait runs out
+                    skipped = (int)pi;
+                } else if (elect_one()) {
+                    mbar_expect_tx(&full_bar[st], 2 * kTcTileBytes);
+                    const unsigned char *src = p_tiles + ((size_t)(pmt * p_nkt + pkt) * 2) * kTcTileBytes;
+                    unsigned char *dst = lst + (size_t)st * 2 * kTcTileBytes;
+                    bulk_copy(dst, src, kTcTileBytes, &full_bar[st]);
+                    bulk_copy(dst + kTcTileBytes, src + kTcTileBytes, kTcTileBytes, &full_bar[st]);
+                }
+                pi++;
+                // next pair: row tiles that need K tile pkt form a suffix of 0..n_mt-1
+                do {
+                    if (++pmt == p_nmt) {
+                        pmt = 0;
+                        ++pkt;
+                    }
+                } while (pkt < p_nkt && pkt >= tc_kts(pmt, p_nmt, p_nkt));
+                if (pkt == p_nkt) {
+                    p_live = false;
+                    pj++;
+                }
+            }
+            return true;
+        };
 
-            unsigned g0 = 0, fpar = 0; // fpar bit m: parity of the uses of row tile m
-            unsigned rs = 0, rph = 0;  // Lhat ring: stage and phase parity of pair ci
-            const uint32_t lst_lo = sw128_desc_lo(smem_u32(lst));
-            for (unsigned j = 0; !tm_abort; j++) {
-                const int slot = (int)(j % kWsTileSlots);
-                if (!mbar_wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
-                    atomicOr(b.err, 32u);
-                    tm_abort = 1;
+        unsigned g0 = 0, fpar = 0; // fpar bit m: parity of the uses of row tile m
+        unsigned rs = 0, rph = 0;  // Lhat ring: stage and phase parity of pair ci
+        const uint32_t lst_lo = sw128_desc_lo(smem_u32(lst));
+        bool dead = false;
+        for (unsigned j = 0; !dead && !same(tm_abort); j++) {
+            const int slot = (int)(j % kWsTileSlots);
+            if (!wait(&tile_pub[slot], (j / kWsTileSlots) & 1u)) {
+                give_up(32u);
+                break;
+            }
+            if (same(s_tile[slot] < 0)) break;
+            const TcItem &it = BATCH ? s_item[slot] : b.one;
+            const int n_kt = same(it.n_kt), n_mt = same(it.n_mt);
+            const uint32_t idesc = tc_idesc(same(it.bf16), kTcRows, P);
+            for (int kt = 0; kt < n_kt && !dead; kt++) {
+                const unsigned g = g0 + (unsigned)kt;
+                const int zs = (int)(g % kWsZSlots);
+                if ((!SPLIT && !pump(false)) || !wait(&zfull[zs], (g / kWsZSlots) & 1u)) {
+                    give_up(64u);
+                    dead = true;
                     break;
                 }
-                if (s_tile[slot] < 0) break;
-                const TcItem &it = BATCH ? s_item[slot] : b.one;
-                const int n_kt = it.n_kt, n_mt = it.n_mt;
-                const uint32_t idesc = tc_idesc(it.bf16, kTcRows, P);
-                for (int kt = 0; kt < n_kt && !tm_abort; kt++) {
-                    const unsigned g = g0 + (unsigned)kt;
-                    const int zs = (int)(g % kWsZSlots);
-                    if ((!SPLIT && !pump(false)) || !mbar_wait(&zfull[zs], (g / kWsZSlots) & 1u)) {
-                        atomicOr(b.err, 64u);
-                        tm_abort = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t zh_lo = sw128_desc_lo(smem_u32(zhi + (size_t)zs * kZB));
-                    const uint32_t zl_lo = sw128_desc_lo(smem_u32(zlo + (size_t)zs * kZB));
-                    for (int mt = 0; mt < n_mt; mt++) {
-                        const int kts = tc_kts(mt, n_mt, n_kt);
-                        if (kt >= kts) continue;
-                        // the first write to row tile mt: the epilogue has read the previous tile's
-                        if (kt == 0 && !mbar_wait(&acc_free[mt], ((fpar >> mt) & 1u) ^ 1u)) {
-                            atomicOr(b.err, 128u);
-                            tm_abort = 1;
-                            break;
-                        }
-                        if (!SPLIT && !pump(true)) {
-                            atomicOr(b.err, 1u);
-                            tm_abort = 1;
-                            break;
-                        }
-                        if (!mbar_wait(&full_bar[rs], rph)) {
-                            atomicOr(b.err, 2u);
-                            tm_abort = 1;
-                            break;
-                        }
-                        tc_fence_after();
-                        tc_mma_pair(tmem + (uint32_t)(mt * P), lst_lo + (uint32_t)rs * (2 * kTcTileBytes >> 4),
-                                    zh_lo, zl_lo, idesc, kt > 0 ? 1u : 0u);
-                        tc_commit(&empty_bar[rs]);
-                        ci++;
+                tc_fence_after();
+                const uint32_t zh_lo = sw128_desc_lo(smem_u32(zhi + (size_t)zs * kZB));
+                const uint32_t zl_lo = sw128_desc_lo(smem_u32(zlo + (size_t)zs * kZB));
+                for (int mt = 0; mt < n_mt; mt++) {
+                    const int kts = tc_kts(mt, n_mt, n_kt);
+                    if (kt >= kts) continue;
+                    if (SPLIT && (mt & 1) != me) { // the other issuer's pair
                         if (++rs == kStages) {
                             rs = 0;
                             rph ^= 1u;
                         }
+                        continue;
+                    }
+                    // the first write to row tile mt: the epilogue has read the previous tile's
+                    unsigned bad = 0u;
+                    if (kt == 0 && !wait(&acc_free[mt], ((fpar >> mt) & 1u) ^ 1u)) bad = 128u;
+                    else if (!SPLIT && !pump(true)) bad = 1u;
+                    else if (!wait(&full_bar[rs], rph)) bad = 2u;
+                    if (bad) {
+                        give_up(bad);
+                        dead = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (elect_one()) {
+                        tc_mma_pair(tm + (uint32_t)(mt * P), lst_lo + rs * (2 * kTcTileBytes >> 4), zh_lo, zl_lo, idesc,
+                                    kt > 0 ? 1u : 0u);
+                        tc_commit(&empty_bar[rs]);
                         if (kt == kts - 1) tc_commit(&acc_full[mt]); // row tile mt complete
                     }
-                    tc_commit(&zempty[zs]); // the slot may be overwritten once these MMAs complete
+                    ci++;
+                    if (++rs == kStages) {
+                        rs = 0;
+                        rph ^= 1u;
+                    }
                 }
-                g0 += (unsigned)n_kt;
-                fpar ^= (1u << n_mt) - 1u;
+                if (elect_one()) tc_commit(&zempty[zs]); // the slot may be overwritten once these MMAs complete
             }
-            // copies issued but not multiplied (only after an abort) land
-            // before the kernel ends; every MMA issued (and every commit's
-            // arrival) completes before the tensor memory and the barriers
-            // are released
-            if (!SPLIT)
-                for (unsigned i = ci; i < pi; i++)
-                    if ((int)i != skipped) mbar_wait(&full_bar[i % kStages], (i / kStages) & 1u);
-            tc_commit(&drain_bar);
-            mbar_wait(&drain_bar, 0u);
+            g0 += (unsigned)n_kt;
+            fpar ^= (1u << n_mt) - 1u;
         }
+        // copies issued but not multiplied (only after an abort) land
+        // before the kernel ends; every MMA issued (and every commit's
+        // arrival) completes before the tensor memory and the barriers
+        // are released
+        if (!SPLIT)
+            for (unsigned i = ci; i < pi; i++)
+                if ((int)i != skipped) mbar_wait(&full_bar[i % kStages], (i / kStages) & 1u);
+        if (elect_one()) tc_commit(&drain_bar[me]);
+        mbar_wait(&drain_bar[me], 0u);
         __syncwarp();
     } else {
         // ======================= epilogue (warps 0-3) =======================
