@@ -40,6 +40,7 @@ struct Batch {
     int sm_count = 0;
     long long total_tiles = 0;
     int n_kt_max = 0, n_mt_max = 0;
+    bool split = false;                     // form of the kernel (tc_split_wins over the whole batch)
     int unit_tiles = 2;
     int ctas_per_sm = 1;
     bool use_graph = true;
@@ -134,7 +135,7 @@ static cudaError_t enqueue(Batch *b, cudaStream_t s)
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_work, 0, 2 * sizeof(unsigned int), s);
     if (e == cudaSuccess)
         e = launch_tc_batch(b->d_items, b->count, b->total_tiles, b->unit_tiles, b->d_work, b->d_work + 1,
-                            b->n_kt_max, b->n_mt_max, b->sm_count * b->ctas_per_sm, s);
+                            b->n_kt_max, b->n_mt_max, b->split, b->sm_count * b->ctas_per_sm, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->h_counts, b->d_counts, sizeof(unsigned long long) * 2 * (size_t)b->count,
                             cudaMemcpyDeviceToHost, s);
@@ -258,16 +259,19 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     // Results stay in the caller's order (d_counts is indexed by item).
     std::vector<int> order((size_t)count);
     for (int i = 0; i < count; i++) order[(size_t)i] = i;
-    auto tile_cost = [&](int i) {
+    double gen = 0.0, mma = 0.0; // of the whole batch
+    std::vector<double> tile_cost((size_t)count);
+    for (int i = 0; i < count; i++) {
         const Portfolio *p = reinterpret_cast<const Portfolio *>(items[i].portfolio);
         const rg_query &q = items[i].query;
-        // SM cycles: about 4 normals a cycle, or 141 cycles an MMA of 12 a (row tile, K tile) pair
-        const double days = q.draw_mode == RG_DRAWS_AGGREGATED ? 1.0 : (double)q.horizon;
-        const double gen = (double)p->n * days * paths / 4.0;
-        const double mma = 12.0 * 141.0 * tc_row_tiles_of(p->n) * tc_k_tiles_of(p->n);
-        return gen > mma ? gen : mma;
-    };
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tile_cost(x) > tile_cost(y); });
+        const double g = tc_tile_gen(p->n, q.draw_mode == RG_DRAWS_AGGREGATED ? 1 : q.horizon, paths);
+        const double m = tc_tile_mma(p->n), tiles = (double)tc_tiles_of(q.n_paths, paths);
+        gen += g * tiles;
+        mma += m * tiles;
+        tile_cost[(size_t)i] = g > m ? g : m;
+    }
+    b->split = tc_split_wins(gen, mma);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tile_cost[(size_t)x] > tile_cost[(size_t)y]; });
     PhiloxBlock *next = b->d_blocks;
     long long tile = 0;
     for (int at = 0; at < count; at++) {

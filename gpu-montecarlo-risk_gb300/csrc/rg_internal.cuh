@@ -310,9 +310,12 @@ int tc_batch_paths(int n_mt_max);
 int tc_row_tiles_of(int n);
 int tc_k_tiles_of(int n);
 cudaError_t launch_tc_batch(const void *d_items, int n_items, long long total_tiles, int unit_tiles,
-                            unsigned int *work, unsigned int *err, int n_kt_max, int n_mt_max, int grid,
+                            unsigned int *work, unsigned int *err, int n_kt_max, int n_mt_max, bool split, int grid,
                             cudaStream_t s, const long long *dyn = nullptr);
 int tc_max_k_tiles();
+double tc_tile_gen(int n, int days, int paths);
+double tc_tile_mma(int n);
+bool tc_split_wins(double gen, double mma);
 cudaError_t tc_batch_prepare();
 int tc_batch_occupancy(int n_mt_max);
 // rg_mc_fused.cu: N <= 64 kernel, L in parameter space; Philox only.

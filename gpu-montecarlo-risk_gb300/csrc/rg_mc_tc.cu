@@ -33,6 +33,7 @@
 // Every wait is bounded: on expiry the kernel sets an error word, drains its
 // own copies and MMAs (again bounded), frees its tensor memory and returns;
 // the host reports RG_ERR_TIMEOUT.
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -1494,6 +1495,27 @@ static cudaError_t launch_one(K kern, const TcBatch &b, int threads, size_t smem
     return cudaGetLastError();
 }
 
+// (row tile, K tile) pairs of a path tile.
+static int tc_pairs(int n)
+{
+    const int n_mt = tc_row_tiles(n), n_kt = tc_k_tiles(n);
+    int pairs = 0;
+    for (int m = 0; m < n_mt; m++) pairs += m == n_mt - 1 ? n_kt : std::min(n_kt, (kTcRows * (m + 1) + kTcKt - 1) / kTcKt);
+    return pairs;
+}
+
+// SM cycles of one path tile on the normals (about four a cycle) and on the
+// MMAs (12 a pair, 80 cycles each with two issuers).
+double tc_tile_gen(int n, int days, int paths) { return (double)n * days * paths / 4.0; }
+double tc_tile_mma(int n) { return 12.0 * 80.0 * tc_pairs(n); }
+
+// Whether the split form (a copy warp, two MMA warps, 25 generator warps) is
+// the faster one: below about three times as many cycles of normals as of
+// MMAs.  1e6 paths, merged and split, us: N = 600 H = 1 2499 and 1559, H = 5
+// 3093 and 2701, H = 10 4682 and 4933; N = 333 H = 3 1108 and 1029, H = 4 1237
+// and 1278; N = 130 H = 3 489 and 469, H = 4 552 and 561.
+bool tc_split_wins(double gen, double mma) { return gen < 3.0 * mma; }
+
 cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, bool aggregated, double wmu,
                       unsigned int *err, bool inject_stall, int sm_count, cudaStream_t s)
 {
@@ -1517,9 +1539,9 @@ cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, 
     b.var = a;
     // The warp-specialised kernel (the widest path tile tensor memory
     // allows): generation, MMAs and the per-row-tile epilogue overlap.  With
-    // daily draws the normals bound it, and the MMA thread also issues the
-    // Lhat copies (one more generator warp); with aggregated draws the MMAs
-    // bound it, and a separate warp streams the copies (SPLIT).
+    // many days the normals bound it, and the MMA warp also issues the Lhat
+    // copies (two more generator warps); with few the MMAs count, and a
+    // separate warp streams the copies (SPLIT; tc_split_wins).
     // RG_TC_KERNEL overrides: "simple" the phase-serial kernel (64-path
     // tiles, kept as a second implementation that the tests compare),
     // "ws64" / "ws96" cap the tile, "split" / "merged" force the copy issuer.
@@ -1528,7 +1550,7 @@ cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, 
     int paths = simple ? 64 : tc_batch_paths(b.one.n_mt);
     if (sel && strstr(sel, "ws64")) paths = 64;
     if (sel && strstr(sel, "ws96") && paths > 96) paths = 96;
-    bool split = aggregated;
+    bool split = tc_split_wins(tc_tile_gen(a.n, aggregated ? 1 : a.horizon, paths), tc_tile_mma(a.n));
     if (sel && strstr(sel, "split")) split = true;
     if (sel && strstr(sel, "merged")) split = false;
     b.total_tiles = (a.n_paths + paths - 1) / paths;
@@ -1574,7 +1596,7 @@ int tc_k_tiles_of(int n) { return tc_k_tiles(n); }
 // must have run (it is not a stream operation, so it stays out of graph
 // captures).
 cudaError_t launch_tc_batch(const void *d_items, int n_items, long long total_tiles, int unit_tiles,
-                            unsigned int *work, unsigned int *err, int n_kt_max, int n_mt_max, int grid,
+                            unsigned int *work, unsigned int *err, int n_kt_max, int n_mt_max, bool split, int grid,
                             cudaStream_t s, const long long *dyn)
 {
     TcBatch b;
@@ -1590,12 +1612,17 @@ cudaError_t launch_tc_batch(const void *d_items, int n_items, long long total_ti
     const int paths = tc_batch_paths(n_mt_max);
     b.tmem_cols = tmem_cols_for(n_mt_max, paths);
     if (n_mt_max * paths > 512 || n_kt_max > kTcMaxKt) return cudaErrorInvalidValue;
-    if (paths == 128)
-        mc_tcws_kernel<false, true, 128, false><<<(unsigned)grid, kWsThreads, WsShape<128>::kSmem, s>>>(b);
-    else if (paths == 96)
-        mc_tcws_kernel<false, true, 96, false><<<(unsigned)grid, kWsThreads, WsShape<96>::kSmem, s>>>(b);
-    else
-        mc_tcws_kernel<false, true, 64, false><<<(unsigned)grid, kWsThreads, WsShape<64>::kSmem, s>>>(b);
+#define RG_WS_BATCH(PP)                                                                                                  \
+    if (split) mc_tcws_kernel<false, true, PP, true><<<(unsigned)grid, kWsThreads, WsShape<PP>::kSmem, s>>>(b);         \
+    else mc_tcws_kernel<false, true, PP, false><<<(unsigned)grid, kWsThreads, WsShape<PP>::kSmem, s>>>(b)
+    if (paths == 128) {
+        RG_WS_BATCH(128);
+    } else if (paths == 96) {
+        RG_WS_BATCH(96);
+    } else {
+        RG_WS_BATCH(64);
+    }
+#undef RG_WS_BATCH
     return cudaGetLastError();
 }
 
@@ -1619,16 +1646,19 @@ int tc_batch_occupancy(int n_mt_max)
 
 // Raise the batched kernels' dynamic shared-memory limit; called once
 // before any launch or capture.
+template <int P> static cudaError_t batch_prepare()
+{
+    const cudaError_t e = cudaFuncSetAttribute(mc_tcws_kernel<false, true, P, false>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WsShape<P>::kSmem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(mc_tcws_kernel<false, true, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)WsShape<P>::kSmem);
+}
 cudaError_t tc_batch_prepare()
 {
-    cudaError_t e = cudaFuncSetAttribute(mc_tcws_kernel<false, true, 128, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WsShape<128>::kSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mc_tcws_kernel<false, true, 96, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)WsShape<96>::kSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mc_tcws_kernel<false, true, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)WsShape<64>::kSmem);
+    cudaError_t e = batch_prepare<128>();
+    if (e == cudaSuccess) e = batch_prepare<96>();
+    if (e == cudaSuccess) e = batch_prepare<64>();
     return e;
 }
 

@@ -117,7 +117,7 @@ static int slot_init(Server *sv, Slot &sl)
         if (e2 == cudaSuccess) e2 = cudaMemsetAsync(sl.d_work, 0, 2 * sizeof(unsigned int), sl.stream);
         if (e2 == cudaSuccess)
             e2 = launch_tc_batch(sl.d_items, cap, 0, 1, sl.d_work, sl.d_work + 1, tc_max_k_tiles(),
-                                 kServedMaxRowTiles, sv->sm_count, sl.stream, sl.d_dyn);
+                                 kServedMaxRowTiles, false, sv->sm_count, sl.stream, sl.d_dyn);
         if (e2 == cudaSuccess)
             e2 = cudaMemcpyAsync(sl.h_counts, sl.d_counts, 16 * (size_t)cap, cudaMemcpyDeviceToHost, sl.stream);
         if (e2 == cudaSuccess)
