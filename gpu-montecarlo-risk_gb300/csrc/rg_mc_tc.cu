@@ -86,6 +86,7 @@ struct TcBatch {
     unsigned int *err;        // device error word
     int inject_stall;         // host-side fault injection: one stage is never filled
     int n_kt_max;             // K tiles of the largest item (shared-memory size)
+    int paths;                // paths per tile of the warp-specialised kernel: a multiple of 16, at most P
     int tmem_cols;            // tensor-memory columns allocated (power of 2 >= 64 n_mt_max)
     const long long *dyn;     // if set: [0] items, [1] total tiles, read from device memory
                               // (a graph captured once serves batches of any size)
@@ -829,6 +830,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ncols = b.tmem_cols;
+    const int paths = b.paths; // per tile, <= P: accumulators and Z slots are laid out for P
     if (tid < 4) sacc[tid] = 0ull;
     if (tid < P) {
         sS[tid] = 0;
@@ -933,7 +935,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             more = tile >= 0;
             return true;
         };
-        constexpr int kPerKt = P * (kTcKt / 8); // items of a K tile
+        const int per_kt = paths * (kTcKt / 8); // items of a K tile (at most 1024)
+        const uint32_t inv_paths = 0xffffffffu / (uint32_t)paths + 1u; // item / paths = umulhi(item, .)
         int first = gtid;                       // this thread's first item of the next K tile
         bool dead = false;
         for (unsigned j = 0; !dead; j++) {
@@ -958,7 +961,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             if (tile < 0) break;
             const TcItem &it = BATCH ? s_item[slot] : b.one;
             const int n = it.n, nq = (n + 3) >> 2, n_kt = it.n_kt;
-            const long long p0 = (tile - it.tile_begin) * P;
+            const long long p0 = (tile - it.tile_begin) * paths;
             const int days = it.aggregated ? 1 : it.horizon;
             for (int kt = 0; kt < n_kt; kt++) {
                 const unsigned g = g0 + (unsigned)kt;
@@ -973,8 +976,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                 // an item is one path's pair of adjacent quads (8 K columns,
                 // one 16-byte chunk of the swizzled Z row)
                 int item = first;
-                for (; item < kPerKt; item += kWsGenThreads) {
-                    const int qp = item / P, p = item - qp * P, q = kt * (kTcKt / 4) + 2 * qp;
+                for (; item < per_kt; item += kWsGenThreads) {
+                    const int qp = (int)__umulhi((uint32_t)item, inv_paths), p = item - qp * paths, q = kt * (kTcKt / 4) + 2 * qp;
                     const unsigned long long path = it.path0 + (unsigned long long)(p0 + p);
                     const uint32_t plo = (uint32_t)path, phi = (uint32_t)(path >> 32);
                     // the two quads' Philox rounds interleaved when both are real,
@@ -1005,7 +1008,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                     *reinterpret_cast<uint4 *>(zhi + off) = make_uint4(hz.x, hz.y, hy.x, hy.y);
                     *reinterpret_cast<uint4 *>(zlo + off) = make_uint4(lz.x, lz.y, ly.x, ly.y);
                 }
-                first = item - kPerKt;
+                first = item - per_kt;
                 fence_async_shared(); // this thread's writes -> async proxy (tensor cores)
                 mbar_arrive(&zfull[zs]);
             }
@@ -1151,7 +1154,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             if (same(s_tile[slot] < 0)) break;
             const TcItem &it = BATCH ? s_item[slot] : b.one;
             const int n_kt = same(it.n_kt), n_mt = same(it.n_mt);
-            const uint32_t idesc = tc_idesc(same(it.bf16), kTcRows, P);
+            const uint32_t idesc = tc_idesc(same(it.bf16), kTcRows, paths);
             for (int kt = 0; kt < n_kt && !dead; kt++) {
                 const unsigned g = g0 + (unsigned)kt;
                 const int zs = (int)(g % kWsZSlots);
@@ -1260,6 +1263,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                 if (thr == 0.f) thr = -0.f;
 #pragma unroll
                 for (int g = 0; g < kG; g++) {
+                    if (g * 32 >= paths) break; // (columns past the tile's paths are counted and not read)
                     uint32_t v[32];
                     tc_load32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * P + g * 32), v);
                     uint32_t m = 0u;
@@ -1288,6 +1292,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
 #pragma unroll
             for (int g = 0; g < kG; g++) {
                 // lane c: rows of this warp that crash in column 32 g + c
+                if (g * 32 >= paths) break;
                 int cnt = __popc(warp_bit_transpose(c0[g], lane));
                 if (n_mt > 1) cnt += 2 * __popc(warp_bit_transpose(c1[g], lane));
                 if (n_mt > 3) cnt += 4 * __popc(warp_bit_transpose(c2[g], lane));
@@ -1296,9 +1301,9 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             apar ^= (1u << n_mt) - 1u;
             named_sync(1, 32 * kWsEpiWarps); // every count of the tile is in sS / sPort
             if (tid < P) {
-                const long long p = (tile - it.tile_begin) * P + tid;
+                const long long p = (tile - it.tile_begin) * paths + tid;
                 int crash = 0, breach = 0;
-                if (p < it.n_paths) {
+                if (tid < paths && p < it.n_paths) {
                     const int S = sS[tid];
                     const float port = sPort[tid];
                     crash = (S >= it.k) ? 1 : 0;
@@ -1516,6 +1521,28 @@ double tc_tile_mma(int n) { return 12.0 * 80.0 * tc_pairs(n); }
 // and 1278; N = 130 H = 3 489 and 469, H = 4 552 and 561.
 bool tc_split_wins(double gen, double mma) { return gen < 3.0 * mma; }
 
+// Paths per tile of a query on sm_count SMs, at most `most`: the multiple of
+// 16 with the least rounds x time of a tile.  A tile's time is its normals
+// (four a cycle) or its MMAs (32 + paths / 4 cycles each, measured alone: 48,
+// 56 and 64 at 64, 96 and 128 paths), whichever is longer, and about 3000
+// cycles to fill and drain the pipeline.  5000 paths at N = 333, H = 5: 48
+// paths a tile on 105 SMs, 26 us; 128 on 40, 37 us.
+static int tc_query_paths(int n, int days, long long n_paths, int most, int sm_count)
+{
+    int best = most;
+    double best_t = 0.0;
+    for (int p = most; p >= 16; p -= 16) {
+        const long long tiles = (n_paths - 1) / p + 1, rounds = (tiles - 1) / sm_count + 1;
+        const double gen = tc_tile_gen(n, days, p), mma = 12.0 * (32.0 + 0.25 * p) * 1.1 * tc_pairs(n);
+        const double t = (double)rounds * ((gen > mma ? gen : mma) + 3000.0);
+        if (p == most || t < best_t) {
+            best = p;
+            best_t = t;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, bool aggregated, double wmu,
                       unsigned int *err, bool inject_stall, int sm_count, cudaStream_t s)
 {
@@ -1553,7 +1580,8 @@ cudaError_t launch_tc(const PlainArgs &a, const unsigned char *tiles, int bf16, 
     bool split = tc_split_wins(tc_tile_gen(a.n, aggregated ? 1 : a.horizon, paths), tc_tile_mma(a.n));
     if (sel && strstr(sel, "split")) split = true;
     if (sel && strstr(sel, "merged")) split = false;
-    b.total_tiles = (a.n_paths + paths - 1) / paths;
+    b.paths = simple ? paths : tc_query_paths(a.n, aggregated ? 1 : a.horizon, a.n_paths, paths, sm_count);
+    b.total_tiles = (a.n_paths - 1) / b.paths + 1;
     b.tmem_cols = tmem_cols_for(b.one.n_mt, paths);
     if (b.one.n_mt * paths > 512) return cudaErrorInvalidValue;
     long long grid = sm_count;
@@ -1610,6 +1638,7 @@ cudaError_t launch_tc_batch(const void *d_items, int n_items, long long total_ti
     b.err = err;
     b.n_kt_max = n_kt_max;
     const int paths = tc_batch_paths(n_mt_max);
+    b.paths = paths;
     b.tmem_cols = tmem_cols_for(n_mt_max, paths);
     if (n_mt_max * paths > 512 || n_kt_max > kTcMaxKt) return cudaErrorInvalidValue;
 #define RG_WS_BATCH(PP)                                                                                                  \
