@@ -38,13 +38,17 @@ int set_error(int status, const char *fmt, ...)
     return status;
 }
 
-// What one rg_simulate call needs besides device memory: its timing events
-// and a pinned buffer for the counters and the first VaR candidates, so that
-// they come back in one wait without a pageable copy's staging.
+// What one rg_simulate call needs: its timing events, the device counters
+// (zero between calls: the last CTA of a kernel resets what it reports) and a
+// pinned buffer that the kernels write the counters and the VaR candidates
+// to.  A 9-asset call has nothing but its kernel between two events in the
+// stream; clearing scratch before and copying it back after took 8 of 34 us.
 struct QueryRes {
-    static constexpr size_t kCand = 16384; // candidates copied with the counters
+    static constexpr size_t kCand = 65536; // VaR candidates the pinned buffer holds
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    unsigned char *h = nullptr;
+    QueryHead *d = nullptr; // device
+    QueryHead *h = nullptr; // pinned, followed by kCand floats
+    float *cand() const { return reinterpret_cast<float *>(h + 1); }
 };
 
 // Process-global state of one device.  `pool` holds what the engine's calls
@@ -150,14 +154,18 @@ static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
     }
     cudaError_t e = cudaEventCreate(&r->e0);
     if (e == cudaSuccess) e = cudaEventCreate(&r->e1);
-    if (e == cudaSuccess) e = cudaMallocHost(&r->h, 64 + QueryRes::kCand * sizeof(float));
+    if (e == cudaSuccess) e = cudaMallocHost(&r->h, sizeof(QueryHead) + QueryRes::kCand * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&r->d, sizeof(QueryHead));
+    if (e == cudaSuccess) e = cudaMemsetAsync(r->d, 0, sizeof(QueryHead), c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return e;
 }
 
-// Back to the list (the call's work is complete), or freed when it is full.
-static void query_res_give(DevCtx *c, QueryRes &r)
+// Back to the list (the call's work is complete and its kernels have reset
+// the counters: `clean`), or freed when it is full or the call failed.
+static void query_res_give(DevCtx *c, QueryRes &r, bool clean)
 {
-    if (r.e0 && r.e1 && r.h) {
+    if (clean) {
         std::lock_guard<std::mutex> lk(g_mu);
         if (c->idle.size() < kIdleQueries) {
             c->idle.push_back(r);
@@ -167,6 +175,7 @@ static void query_res_give(DevCtx *c, QueryRes &r)
     if (r.e0) cudaEventDestroy(r.e0);
     if (r.e1) cudaEventDestroy(r.e1);
     if (r.h) cudaFreeHost(r.h);
+    if (r.d) cudaFree(r.d);
 }
 
 #define RG_CUDA_TRY(call)                                                                          \
@@ -321,28 +330,6 @@ static cudaError_t launch_counting(const Portfolio *p, const rg_query *q, const 
     return launch_plain_small(a, q->rng, sm_count, s);
 }
 
-// Device scratch of one query: counters, VaR tail sums, candidate count,
-// error word, candidate list and histogram, carved from one stream-ordered
-// allocation.  The head and the candidates after it come back in one copy.
-struct QueryScratch {
-    unsigned long long *counts = nullptr;  // [2]
-    unsigned long long *counts2 = nullptr; // [2] counters of the extra VaR passes (discarded)
-    unsigned long long *tail = nullptr;    // [2]
-    unsigned int *cand_count = nullptr;    // [1]
-    unsigned int *err = nullptr;           // [1] error word of the tensor-core kernel
-    float *cand = nullptr;                 // [cap]
-    unsigned long long *hist = nullptr;    // [kVarHistBins + 2]
-    PhiloxBlock *blocks = nullptr;         // room for the Philox block table, or null
-    unsigned int cap = 0;
-    void *base = nullptr;
-};
-// The same fields in the pinned buffer.
-struct QueryHead {
-    unsigned long long counts[2], counts2[2], tail[2];
-    unsigned int cand_count, err;
-};
-static_assert(sizeof(QueryHead) == 56, "device and host layout");
-
 // Bytes for the block table of a tensor-core query with enough normals that
 // the table's own launch (about 3 us) pays: 6 % of a generator that draws
 // 1.2e12 normals a second.
@@ -352,28 +339,6 @@ static size_t table_bytes(const Portfolio *p, const rg_query *q)
     const int days = q->draw_mode == RG_DRAWS_AGGREGATED ? 1 : q->horizon;
     if (!tensor || (double)q->n_paths * p->n * days < 1e8) return 0;
     return sizeof(PhiloxBlock) * philox_table_len(p->n, days, q->path_offset, q->n_paths);
-}
-
-static cudaError_t scratch_alloc(DevCtx *ctx, QueryScratch &sc, unsigned int cap, bool with_var, size_t table,
-                                 cudaStream_t s)
-{
-    const size_t head = sizeof(QueryHead);
-    const size_t cand = with_var ? ((4 * (size_t)cap + 7) & ~(size_t)7) : 0;
-    const size_t hist = with_var ? 8 * (size_t)(kVarHistBins + 2) : 0;
-    const size_t table_at = (head + cand + hist + 15) & ~(size_t)15;
-    cudaError_t e = cudaMallocFromPoolAsync(&sc.base, table_at + table + 16, ctx->pool, s);
-    if (e != cudaSuccess) return e;
-    char *b = (char *)sc.base;
-    sc.blocks = table ? (PhiloxBlock *)(b + table_at) : nullptr;
-    sc.counts = (unsigned long long *)b;
-    sc.counts2 = sc.counts + 2;
-    sc.tail = sc.counts + 4;
-    sc.cand_count = (unsigned int *)(sc.counts + 6);
-    sc.err = sc.cand_count + 1;
-    sc.cand = with_var ? (float *)(b + head) : nullptr;
-    sc.hist = with_var ? (unsigned long long *)(b + head + cand) : nullptr;
-    sc.cap = with_var ? cap : 0;
-    return cudaMemsetAsync(sc.base, 0, head, s);
 }
 
 static PlainArgs make_args(const Portfolio *p, const rg_query *q, unsigned long long *d_counts)
@@ -776,69 +741,76 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         const double expect = (double)M * dens * 2.0 * half;
         cap = (unsigned int)std::min(4.0 * expect + 4096.0, 64.0 * 1024 * 1024);
     }
-    QueryScratch sc;
     QueryRes res;
     QueryHead head;
     float ms = 0.f, ms_pass = 0.f;
     unsigned int ncand = 0;
-    size_t pre = 0;   // candidates copied with the counters
+    void *d_table = nullptr, *d_hist = nullptr, *d_cand = nullptr; // from the pool, when needed
     float *cand = nullptr;
     std::vector<float> cand_v;
     std::vector<unsigned long long> hist;
     int passes = 0;
     int64_t n_tail = 0;
+    size_t table = 0;
     PlainArgs a;
+    // one launch, waited for; its counters in `head`
+    auto pass = [&](float *pass_ms) -> cudaError_t {
+        cudaError_t e = cudaEventRecord(res.e0, s);
+        if (e == cudaSuccess) e = launch_counting(p, q, a, ctx->sm_count, s);
+        if (e == cudaSuccess) e = cudaEventRecord(res.e1, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(pass_ms, res.e0, res.e1);
+        if (e == cudaSuccess) memcpy(&head, res.h, sizeof(head));
+        return e;
+    };
+    unsigned long long counts[2] = {0, 0};
     st = admit(64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2));
     if (st) return st;
     RG_CUDA_TRY(query_res_take(ctx, &res));
-    RG_CUDA_TRY(scratch_alloc(ctx, sc, cap, want_var, table_bytes(p, q), s));
-    a = make_args(p, q, sc.counts);
-    a.err = sc.err;
-    a.blocks = sc.blocks;
+    table = table_bytes(p, q);
+    if (table) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s));
+    if (cap > QueryRes::kCand) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_cand, 4 * (size_t)cap, ctx->pool, s));
+    a = make_args(p, q, res.d->counts);
+    a.err = &res.d->err;
+    a.head = res.d;
+    a.host = res.h;
+    a.blocks = static_cast<PhiloxBlock *>(d_table);
     if (want_var) {
         a.var_mode = 1;
         a.sel_bins = 1;
         a.sel_target = 0;
         a.sel_lo = (float)band_lo;
         a.sel_inv_w = (float)(1.0 / (band_hi - band_lo));
-        a.cand = sc.cand;
-        a.cand_count = sc.cand_count;
-        a.cand_cap = sc.cap;
-        a.tail = sc.tail;
-        a.hist = sc.hist;
+        a.cand = d_cand ? static_cast<float *>(d_cand) : res.cand();
+        a.cand_count = &res.d->cand_count;
+        a.cand_cap = cap;
+        a.tail = res.d->tail;
     }
-    RG_CUDA_TRY(cudaEventRecord(res.e0, s));
-    RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-    RG_CUDA_TRY(cudaEventRecord(res.e1, s));
-    pre = want_var ? std::min((size_t)sc.cap, QueryRes::kCand) : 0;
-    RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head) + 4 * pre, cudaMemcpyDeviceToHost, s));
-    RG_CUDA_TRY(cudaStreamSynchronize(s));
-    cudaEventElapsedTime(&ms, res.e0, res.e1);
-    memcpy(&head, res.h, sizeof(head));
-    ncand = head.cand_count;
+    RG_CUDA_TRY(pass(&ms));
     passes = 1;
     st = tc_status(head.err);
     if (st) goto fail;
+    counts[0] = head.counts[0];
+    counts[1] = head.counts[1];
+    ncand = head.cand_count;
     n_tail = (int64_t)head.tail[0];
-    if (want_var && !(n_tail < T && T <= n_tail + (int64_t)ncand && ncand <= sc.cap)) {
+    if (want_var && !(n_tail < T && T <= n_tail + (int64_t)ncand && ncand <= cap)) {
         // The band missed the order statistic: histogram pass over
-        // mean -+ 12 sd, then a select pass on the bin that holds it.
+        // mean -+ 12 sd, then a select pass on the bin that holds it (their
+        // counts are discarded).
         hist.assign(kVarHistBins + 2, 0ull);
-        a.counts = sc.counts2;
+        RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_hist, hist.size() * 8, ctx->pool, s));
         a.var_mode = 2;
         a.sel_bins = kVarHistBins;
         a.sel_lo = (float)(mean - 12.0 * sd);
         a.sel_inv_w = (float)(kVarHistBins / (24.0 * sd));
-        RG_CUDA_TRY(cudaMemsetAsync(sc.hist, 0, hist.size() * 8, s));
-        RG_CUDA_TRY(cudaEventRecord(res.e0, s));
-        RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-        RG_CUDA_TRY(cudaEventRecord(res.e1, s));
-        RG_CUDA_TRY(cudaMemcpyAsync(hist.data(), sc.hist, hist.size() * 8, cudaMemcpyDeviceToHost, s));
-        RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head), cudaMemcpyDeviceToHost, s));
-        RG_CUDA_TRY(cudaStreamSynchronize(s));
-        st = tc_status(reinterpret_cast<const QueryHead *>(res.h)->err);
+        a.hist = static_cast<unsigned long long *>(d_hist);
+        RG_CUDA_TRY(cudaMemsetAsync(d_hist, 0, hist.size() * 8, s));
+        RG_CUDA_TRY(pass(&ms_pass));
+        st = tc_status(head.err);
         if (st) goto fail;
-        cudaEventElapsedTime(&ms_pass, res.e0, res.e1);
+        RG_CUDA_TRY(cudaMemcpyAsync(hist.data(), d_hist, hist.size() * 8, cudaMemcpyDeviceToHost, s));
+        RG_CUDA_TRY(cudaStreamSynchronize(s));
         ms += ms_pass;
         int64_t cum = 0;
         int j = 0;
@@ -851,60 +823,43 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
             goto fail;
         }
         const unsigned int need = (unsigned int)hist[(size_t)j];
-        if (need > sc.cap) {
-            RG_CUDA_TRY(cudaFreeAsync(sc.base, s));
-            sc.base = nullptr;
-            RG_CUDA_TRY(scratch_alloc(ctx, sc, need, true, table_bytes(p, q), s));
-            a.counts = sc.counts2;
-            a.err = sc.err;
-            a.blocks = sc.blocks;
-            a.cand = sc.cand;
-            a.cand_count = sc.cand_count;
-            a.tail = sc.tail;
-            a.hist = sc.hist;
+        if (need > cap) {
+            if (d_cand) RG_CUDA_TRY(cudaFreeAsync(d_cand, s));
+            d_cand = nullptr;
+            cap = need;
+            if (cap > QueryRes::kCand) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_cand, 4 * (size_t)cap, ctx->pool, s));
+            a.cand = d_cand ? static_cast<float *>(d_cand) : res.cand();
         }
         a.var_mode = 1;
         a.sel_target = j - 1;
-        a.cand_cap = sc.cap;
-        RG_CUDA_TRY(cudaMemsetAsync(sc.tail, 0, 2 * 8 + 4, s)); // and the candidate count behind it
-        RG_CUDA_TRY(cudaEventRecord(res.e0, s));
-        RG_CUDA_TRY(launch_counting(p, q, a, ctx->sm_count, s));
-        RG_CUDA_TRY(cudaEventRecord(res.e1, s));
-        pre = std::min((size_t)sc.cap, QueryRes::kCand);
-        RG_CUDA_TRY(cudaMemcpyAsync(res.h, sc.base, sizeof(head) + 4 * pre, cudaMemcpyDeviceToHost, s));
-        RG_CUDA_TRY(cudaStreamSynchronize(s));
-        {
-            QueryHead again;
-            memcpy(&again, res.h, sizeof(again));
-            st = tc_status(again.err);
-            head.tail[0] = again.tail[0]; // the counters are the first pass's
-            head.tail[1] = again.tail[1];
-            ncand = again.cand_count;
-        }
+        a.cand_cap = cap;
+        RG_CUDA_TRY(pass(&ms_pass));
+        st = tc_status(head.err);
         if (st) goto fail;
-        cudaEventElapsedTime(&ms_pass, res.e0, res.e1);
         ms += ms_pass;
         passes = 3;
+        ncand = head.cand_count;
         n_tail = (int64_t)head.tail[0];
-        if (n_tail != cum || ncand != need || ncand > sc.cap) {
+        if (n_tail != cum || ncand != need || ncand > cap) {
             st = set_error(RG_ERR_CUDA, "VaR select pass disagrees with its histogram");
             goto fail;
         }
     }
-    if (want_var && ncand > pre) {
+    if (want_var && d_cand) {
         cand_v.resize(ncand);
         cand = cand_v.data();
-        RG_CUDA_TRY(cudaMemcpyAsync(cand, sc.cand, (size_t)ncand * 4, cudaMemcpyDeviceToHost, s));
+        if (ncand) RG_CUDA_TRY(cudaMemcpyAsync(cand, d_cand, (size_t)ncand * 4, cudaMemcpyDeviceToHost, s));
         RG_CUDA_TRY(cudaStreamSynchronize(s));
     } else if (want_var) {
-        cand = reinterpret_cast<float *>(res.h + sizeof(head));
+        cand = res.cand();
     }
-    RG_CUDA_TRY(cudaFreeAsync(sc.base, s));
-    sc.base = nullptr;
+    if (d_table) cudaFreeAsync(d_table, s);
+    if (d_hist) cudaFreeAsync(d_hist, s);
+    if (d_cand) cudaFreeAsync(d_cand, s);
     memset(out, 0, sizeof(*out));
     out->n_paths = M;
-    out->crash_count = (int64_t)head.counts[0];
-    out->breach_count = (int64_t)head.counts[1];
+    out->crash_count = (int64_t)counts[0];
+    out->breach_count = (int64_t)counts[1];
     rg_estimator_stats(out->crash_count, M, &out->p_crash, &out->se_crash, &out->ci_lower, &out->ci_upper);
     rg_estimator_stats(out->breach_count, M, &out->p_breach, &out->se_breach, nullptr, nullptr);
     out->var = NAN;
@@ -923,12 +878,14 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         out->var_passes = passes;
     }
     out->ms_device = ms;
-    query_res_give(ctx, res);
+    query_res_give(ctx, res, true);
     return RG_OK;
 fail:
     cudaStreamSynchronize(s);
-    if (sc.base) cudaFreeAsync(sc.base, s);
-    query_res_give(ctx, res);
+    if (d_table) cudaFreeAsync(d_table, s);
+    if (d_hist) cudaFreeAsync(d_hist, s);
+    if (d_cand) cudaFreeAsync(d_cand, s);
+    query_res_give(ctx, res, false);
     return st;
 }
 

@@ -116,7 +116,8 @@ __device__ __forceinline__ void var_path(const PlainArgs &a, float port, unsigne
 }
 
 // Per-CTA reduction of the counters: warp sums, one 64-bit atomic per CTA
-// per counter, and the CTA's histogram merged into the global one.
+// per counter, and the CTA's histogram merged into the global one; the
+// launch's last CTA reports the counters.
 __device__ __forceinline__ void cta_flush(const PlainArgs &a, int crash, int breach, int n_tail,
                                           long long tail_fx, unsigned long long *sacc,
                                           unsigned int *shist, bool var)
@@ -145,6 +146,7 @@ __device__ __forceinline__ void cta_flush(const PlainArgs &a, int crash, int bre
             if (sacc[2]) atomicAdd(&a.tail[0], sacc[2]);
             if (sacc[3]) atomicAdd(&a.tail[1], sacc[3]);
         }
+        cta_report(a);
     }
     if (shist && a.var_mode == 2)
         for (int t = tid; t < a.sel_bins + 2; t += blockDim.x)

@@ -225,6 +225,18 @@ struct Portfolio {
     std::vector<float> h_w;    // weights, FP32 (zeros when none)
 };
 
+// Counters of one query.  Kernels add to the device copy; with PlainArgs::head
+// set, the last CTA of a launch writes them to `host` and resets them.
+struct QueryHead {
+    unsigned long long counts[2];  // crash, breach
+    unsigned long long tail[2];    // VaR tail: paths, sum of -w.R * 2^32 (int64 bits)
+    unsigned int cand_count;       // VaR candidates
+    unsigned int err;              // error word of the tensor-core kernel
+    unsigned int ctas;             // CTAs that are done (device)
+    unsigned int pad[5];
+};
+static_assert(sizeof(QueryHead) == 64, "read in 8-byte words");
+
 // Arguments of the fused counting kernels.
 struct PlainArgs {
     const float4 *Lp;
@@ -261,9 +273,33 @@ struct PlainArgs {
     unsigned long long *tail;   // [0] tail paths, [1] sum of -w.R * 2^32 (int64 bits)
     unsigned long long *hist;   // [sel_bins + 2]
     unsigned int *err;          // device error word of the tensor-core kernel (bounded waits)
+    QueryHead *head;            // device counters to report and reset, or null
+    QueryHead *host;            // pinned host memory they are reported to
     // room for the query's PhiloxBlock table (philox_table_len entries), or null
     PhiloxBlock *blocks;
 };
+
+// End of a launch for one thread of each CTA, after every count of its CTA has
+// been added (a CTA barrier before it).  The CTA that is last reports the
+// query's counters to pinned host memory and leaves zeros for the next launch.
+__device__ __forceinline__ void cta_report(const PlainArgs &a)
+{
+    if (!a.head) return;
+    __threadfence();
+    if (atomicAdd(&a.head->ctas, 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    unsigned long long *d = reinterpret_cast<unsigned long long *>(a.head);
+    volatile unsigned long long *h = reinterpret_cast<volatile unsigned long long *>(a.host);
+    unsigned long long v[sizeof(QueryHead) / 8];
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(QueryHead) / 8); i++) v[i] = __ldcg(d + i);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(QueryHead) / 8); i++) {
+        h[i] = v[i];
+        d[i] = 0ull;
+    }
+    __threadfence_system();
+}
 
 // Entries of a query's block table (block = day * ceil(N/4) + quad), or 0
 // where it is not used: the paths' high words differ or the table is longer

@@ -678,6 +678,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mc_tc_kernel(const __grid_const
     tc_fence_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
     if (VAR) cta_flush(a, 0, 0, n_tail, tail_fx, sacc, nullptr, true);
+    else if (tid == 0) cta_report(a);
 }
 
 // ----------------------------------------------------------------------
@@ -1330,6 +1331,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     tc_fence_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
     if (VAR) cta_flush(a, 0, 0, n_tail, tail_fx, sacc, nullptr, true);
+    else if (tid == 0) cta_report(a);
 }
 
 // Row segment blockIdx.y's part of w^T L for 32 columns (lane = column, rows

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(kPlainThreads, 2) mc_plain_small_kernel(const 
     if (tid == 0) {
         if (sacc[0]) atomicAdd(&a.counts[0], sacc[0]);
         if (sacc[1]) atomicAdd(&a.counts[1], sacc[1]);
+        cta_report(a);
     }
 }
 
