@@ -315,6 +315,9 @@ inline size_t philox_table_len(int n, int days, unsigned long long path0, long l
 static constexpr int kVarHistBins = 4096;
 
 // Launchers.  Return cudaSuccess or the launch error.
+// Fills a query's block table (rg_mc_tc.cu).
+cudaError_t launch_philox_table(PhiloxBlock *t, size_t len, unsigned long long path0, const PhiloxKeys &keys,
+                                cudaStream_t s);
 // rg_mc_plain.cu / rg_mc_xorwow.cu: row-order kernel, L staged in shared
 // memory; both normal layouts.
 cudaError_t launch_plain_small(const PlainArgs &a, int rng, int sm_count, cudaStream_t s);
