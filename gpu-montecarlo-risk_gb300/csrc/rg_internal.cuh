@@ -219,7 +219,7 @@ struct Portfolio {
     int *d_info = nullptr;
     double wsw = 0.0, wmu = 0.0;
     float ms_chol = 0.f;
-    // host copies for kernels that take the factor by value
+    // N <= 64: host copies for the kernel that takes the factor by value
     std::vector<float> h_Lp;   // packed rows, FP32
     std::vector<double> h_mu;  // daily means, FP64
     std::vector<float> h_w;    // weights, FP32 (zeros when none)
