@@ -247,11 +247,12 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     size_t blocks = 0;
     for (int i = 0; i < count; i++)
         blocks += table_len(reinterpret_cast<const Portfolio *>(items[i].portfolio), items[i].query);
-    if (blocks) e = cudaMalloc(&b->d_blocks, blocks * sizeof(PhiloxBlock));
-    if (e != cudaSuccess) {
-        destroy_batch(b);
-        return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "batch setup failed: %s",
-                         cudaGetErrorString(e));
+    // the tables are left out beyond 256 MiB, or where there is no room
+    if (blocks > (256ull << 20) / sizeof(PhiloxBlock)) blocks = 0;
+    if (blocks && cudaMalloc(&b->d_blocks, blocks * sizeof(PhiloxBlock)) != cudaSuccess) {
+        cudaGetLastError();
+        b->d_blocks = nullptr;
+        blocks = 0;
     }
     // Items go into the table by falling time of one tile: CTAs claim units in
     // table order, so the last units are short and no CTA is left with a long
@@ -280,7 +281,7 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
         const rg_query &q = items[i].query;
         const int bf16 = q.precision == RG_PREC_BF16X3 ? 1 : 0;
         PlainArgs a = query_args(p, &q, b->d_counts + 2 * (size_t)i);
-        const size_t len = table_len(p, q);
+        const size_t len = blocks ? table_len(p, q) : 0;
         a.blocks = len ? next : nullptr;
         next += len;
         tc_fill_batch_item(host.data() + (size_t)at * tc_item_bytes(), a, p->d_tc[bf16], bf16,

@@ -152,12 +152,16 @@ static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
             return cudaSuccess;
         }
     }
+    // (allowed beside a stream capture of another thread, as the rest of a call is)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     cudaError_t e = cudaEventCreate(&r->e0);
     if (e == cudaSuccess) e = cudaEventCreate(&r->e1);
     if (e == cudaSuccess) e = cudaMallocHost(&r->h, sizeof(QueryHead) + QueryRes::kCand * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&r->d, sizeof(QueryHead));
     if (e == cudaSuccess) e = cudaMemsetAsync(r->d, 0, sizeof(QueryHead), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     return e;
 }
 
@@ -530,7 +534,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     const size_t nn = (size_t)n * n;
     const bool want_lt = (parts & kPartLt) && n <= tiled_max_n();
     const bool want_tc[2] = {(parts & kPartTcFp16) && n <= tc_max_n(), (parts & kPartTcBf16) && n <= tc_max_n()};
-    const size_t need = nn * 8 * (dev_in ? 1 : 2) + (size_t)n * 40 + (size_t)packed_len(n) * 4 +
+    const size_t need = nn * 8 * (dev_in ? 1 : 2) + (size_t)n * 104 + (size_t)packed_len(n) * 4 +
                         (want_lt ? (size_t)tiled_kpad(n) * tiled_npad(n) * 4 : 0) +
                         (want_tc[0] ? tc_tile_bytes(n) : 0) + (want_tc[1] ? tc_tile_bytes(n) : 0) + 64;
     st = admit(need);
@@ -703,8 +707,11 @@ int rg_launch_counts(const rg_portfolio *h, const rg_query *q, unsigned long lon
     if (e == cudaSuccess && table) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-        else if (cap == cudaStreamCaptureStatusNone)
-            e = cudaMallocFromPoolAsync((void **)&a.blocks, table, ctx->pool, s);
+        else if (cap == cudaStreamCaptureStatusNone &&
+                 cudaMallocFromPoolAsync((void **)&a.blocks, table, ctx->pool, s) != cudaSuccess) {
+            cudaGetLastError();
+            a.blocks = nullptr;
+        }
     }
     if (e == cudaSuccess) e = launch_counting(p, q, a, ctx->sm_count, s);
     if (a.blocks) {
@@ -782,7 +789,10 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
     if (st) return st;
     RG_CUDA_TRY(query_res_take(ctx, &res));
     table = table_bytes(p, q);
-    if (table) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s));
+    if (table && cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s) != cudaSuccess) {
+        cudaGetLastError(); // the query runs without the table
+        d_table = nullptr;
+    }
     if (cap > QueryRes::kCand) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_cand, 4 * (size_t)cap, ctx->pool, s));
     a = make_args(p, q, res.d->counts);
     a.err = &res.d->err;

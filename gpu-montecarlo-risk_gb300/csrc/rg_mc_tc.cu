@@ -19,12 +19,12 @@
 //
 // Two kernels, one CTA per SM, persistent over path tiles:
 //   mc_tcws_kernel   (the engine's default) warp-specialised, 1024 threads:
-//                    26 generator warps draw the next tile's normals into a
-//                    ring of K-tile slots while one thread streams the
-//                    pre-swizzled Lhat tiles (cp.async.bulk, mbarrier ring),
-//                    one thread issues the MMAs K-tile-outer, and four warps
-//                    read each row tile's accumulators (tcgen05.ld) as soon
-//                    as it is complete.  P = 128 paths up to N = 511, 96
+//                    25 or 27 generator warps draw the next tile's normals
+//                    into a ring of K-tile slots while others stream the
+//                    pre-swizzled Lhat tiles (cp.async.bulk, mbarrier ring)
+//                    and issue the MMAs K-tile-outer, and four warps read each
+//                    row tile's accumulators (tcgen05.ld) as soon as it is
+//                    complete.  At most P = 128 paths a tile up to N = 511, 96
 //                    up to N = 639, else 64 (tensor-memory columns).
 //   mc_tc_kernel     phase-serial, 512 threads, P = 64: all threads draw the
 //                    tile's normals, one thread streams Lhat through a

@@ -4,7 +4,7 @@
 // at its definition: the pipelined mc_tiled_pipe_kernel (default), the
 // phase-serial mc_tiled_kernel it is built from (RG_PLAIN_KERNEL=serial) and
 // the warp-specialised mc_tiled_ws_kernel (RG_PLAIN_KERNEL=ws).  At N = 600,
-// H = 10, 1e7 paths: 116.8, 136.6 and 170 ms with daily draws; 86.5, 94.1
+// H = 10, 1e7 paths: 111.6, 136.6 and 170 ms with daily draws; 83.2, 94.1
 // and 149 ms with aggregated draws.
 //
 // Phase-serial form: a CTA owns a tile of 64 paths at a time (grid-stride
