@@ -15,13 +15,16 @@
 //   to theirs (chol_factor_cta).
 // Above (launch_cholesky_blocked): right-looking over 32-column blocks, two
 //   launches a block:
-//   chol_step   CTA 0 subtracts the previous panel from the next 32 x 32
-//               diagonal block and factors it (the same scheme); the other
-//               CTAs subtract the panel from the rest of the trailing lower
-//               triangle, a 16 x 16 tile each, at the same time;
+//   chol_step   CTA 0 factors the next 32 x 32 diagonal block (the same
+//               scheme); the other CTAs subtract the previous panel from the
+//               rest of the trailing lower triangle, a 16 x 16 tile each, at
+//               the same time;
 //   chol_panel  one warp per row below the block solves x L_kk^T = a with a
 //               lane per column: 32 steps of one shuffle and one FMA, on the
-//               rows of L_kk divided by their pivots.
+//               rows of L_kk divided by their pivots.  Its first cluster of
+//               eight CTAs then subtracts its 32 rows' products from the next
+//               diagonal block (in chol_step's CTA 0 they stood before the
+//               pivots: N = 600 673 us, now 552).
 //   A 32 x 32 x 32 update is 19.5k cycles of one SM's FP64 pipe, hence the
 //   16 x 16 tiles (N = 600: 663 in the first step), and a row per warp in the
 //   panel (a row per lane put all 32 rows of a CTA on one sub-partition: 28 us
@@ -35,9 +38,9 @@
 // lane in the panel, 32 x 32 update tiles) and now:
 //   N        9    20    50    64    65   200   333   600   1000   2000
 //   before  34    65   178   249   188   538   924  1578   2810   7246
-//   now     12    20    49    58    81   223   364   673   1237   3706
+//   now     11    18    49    57    68   189   310   552   1037   3440
 // Both forms cross at N = 64, the widest block whose columns stay in
-// registers (58 us against about 75 us blocked).
+// registers (57 us against about 66 us blocked).
 // RG_CHOLESKY=single forces cholesky_kernel, one CTA left-looking column by
 // column in place in the row-major output, above N = 64 too (a second
 // implementation that the tests compare).
@@ -178,7 +181,7 @@ static constexpr int kCholSmallMaxN = 64;   // the one-CTA form up to here
 static constexpr int kCholCta = 256;        // threads of the factoring CTA and of chol_step's others
 static constexpr int kCholTimeout = -2;     // info: a bounded wait ran out
 static constexpr int kCholTile = 16;        // trailing-update tile
-static constexpr size_t kCholAlone = 96 * 1024; // dynamic shared memory that, with the static, leaves one CTA an SM
+static constexpr size_t kCholAlone = 104 * 1024; // dynamic shared memory that, with the static, leaves one CTA an SM
 
 // A positive finite pivot, tested on the bits (no FP64-pipe instruction).
 __device__ __forceinline__ bool good_pivot(double d)
@@ -501,12 +504,13 @@ __global__ void chol_prep_kernel(const double *__restrict__ A, long long lda, in
 
 // The previous panel (columns k0 .. k0 + kb - 1, kb = 0 before the first
 // block) applied to the trailing lower triangle, whose first row is
-// r0 = k0 + kb; CTA 0 then factors the 32 x 32 diagonal block at r0 and
-// leaves its reciprocal pivots in dinv.
-__global__ void __launch_bounds__(kCholCta) chol_step_kernel(double *__restrict__ L, int n, int k0, int kb,
+// r0 = k0 + kb, beside CTA 0, which factors the 32 x 32 diagonal block at r0
+// (the panel's kernel has brought it up to date) and leaves its reciprocal
+// pivots in dinv.
+__global__ void __launch_bounds__(kCholCta, 1) chol_step_kernel(double *__restrict__ L, int n, int k0, int kb,
                                                                     double *__restrict__ dinv, int *__restrict__ info)
 {
-    __shared__ double P[kCholNb][kCholNb + 1];
+    __shared__ double P[kCholTile][kCholNb + 1];
     __shared__ double col[kCholNb * kCholNb];
     __shared__ double T[kCholTile][kCholNb + 1];
     __shared__ double inv[kCholNb];
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(kCholCta) chol_step_kernel(double *__restrict_
 
     if (blockIdx.x > 0) {
         // one 16 x 16 tile (bi, bj), bj <= bi, of the trailing triangle, row
-        // by row; tiles 0..2 are the diagonal block's
+        // by row; tiles 0..2 are the diagonal block's, not touched here
         const int t = (int)blockIdx.x + 2;
         int bi = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f); // then corrected exactly
         while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
@@ -550,37 +554,9 @@ __global__ void __launch_bounds__(kCholCta) chol_step_kernel(double *__restrict_
     const int nb = min(kCholNb, n - r0);
     for (int e = tid; e < kCholNb * kCholNb; e += blockDim.x) {
         const int r = e / kCholNb, m = e % kCholNb;
-        const bool in = r < nb;
-        P[r][m] = (in && m < kb) ? L[(long long)(r0 + r) * n + k0 + m] : 0.0;
-        col[m * kCholNb + r] = (in && m <= r) ? L[(long long)(r0 + r) * n + r0 + m] : 0.0;
+        col[m * kCholNb + r] = (r < nb && m <= r) ? L[(long long)(r0 + r) * n + r0 + m] : 0.0;
     }
     __syncthreads();
-    if (kb > 0) {
-        // lower triangle of P P^T in 17 full-width units: unit u holds column
-        // u (rows u..31) and, in the lanes left over, column 32 - u (rows
-        // 32-u..31): half the warp FMAs of the full square
-        int row[3], cc[3];
-        double v[3] = {0.0, 0.0, 0.0};
-        constexpr int kW = kCholCta / 32;
-        const int units = warp == 0 ? 3 : 2;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const int u = warp + kW * q;
-            row[q] = lane < 32 - u ? u + lane : lane;
-            cc[q] = lane < 32 - u ? u : 32 - u;
-            if (q == 2 && warp != 0) row[q] = cc[q] = 0;
-        }
-#pragma unroll 4
-        for (int m = 0; m < kCholNb; m++) {
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-                if (q < units) v[q] = fma(P[row[q]][m], P[cc[q]][m], v[q]);
-        }
-#pragma unroll
-        for (int q = 0; q < 3; q++)
-            if (q < units && (q < 2 || lane < 16)) col[cc[q] * kCholNb + row[q]] -= v[q];
-        __syncthreads();
-    }
     if (chol_takes_part()) chol_factor_cta<kCholNb>(nb, col, inv, flags, &s_fail);
     __syncthreads();
     if (s_fail) {
@@ -598,31 +574,71 @@ __global__ void __launch_bounds__(kCholCta) chol_step_kernel(double *__restrict_
 // per row, lane j holding column j.  With l'_jc = l_jc / l_jj and
 // s_j = a_j / l_jj the solve is s_j -= x_c l'_jc for c < j, x_j = s_j: one
 // shuffle and one FMA a step.
+//
+// The 32 rows of cluster 0 are those of the next diagonal block, and it goes
+// on to subtract their products from that block: each row is handed to all
+// eight CTAs, and 17 warps take a unit of the lower triangle each, two a CTA
+// (one SM's FP64 pipe needs 10k cycles for the block; in the factoring CTA
+// they stood before the chain of pivots).  The cluster's barriers stand where
+// every thread passes them.
 static constexpr int kPanelWarps = 4;
-__global__ void __launch_bounds__(32 * kPanelWarps) chol_panel_kernel(double *__restrict__ L, int n, int k0,
-                                                                      const double *__restrict__ dinv,
-                                                                      const int *__restrict__ info)
+static constexpr int kPanelCluster = kCholNb / kPanelWarps;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(32 * kPanelWarps)
+    chol_panel_kernel(double *__restrict__ L, int n, int k0, const double *__restrict__ dinv,
+                      const int *__restrict__ info)
 {
     __shared__ double lp[kCholNb][kCholNb + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double X[kCholNb][kCholNb + 1]; // cluster 0: the rows of the next diagonal block
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)blockIdx.x; // rank: in cluster 0
+    const bool next = blockIdx.x < kPanelCluster;
     pdl_enter();
-    if (*info != 0) return;
+    if (*info != 0) return; // the same in every CTA
+    if (next) cluster_arrive(); // this CTA runs: its X may be written
     const double di = dinv[lane];
     for (int j = warp; j < kCholNb; j += kPanelWarps) {
         const double dj = __shfl_sync(0xffffffffu, di, j);
         lp[j][lane] = lane < j ? L[(long long)(k0 + j) * n + k0 + lane] * dj : 0.0;
     }
-    const int i = k0 + kCholNb + (int)blockIdx.x * kPanelWarps + warp;
+    const int r1 = k0 + kCholNb, i = r1 + (int)blockIdx.x * kPanelWarps + warp;
     double s = i < n ? L[(long long)i * n + k0 + lane] * di : 0.0;
+    // Unit u of the block's lower triangle: column u (rows u..31) and, in the
+    // lanes left over, column 32 - u (rows 32 - u..31): 17 full-width units
+    // are half the warp FMAs of the square.
+    const int u = warp < 2 ? rank + kPanelCluster * warp : kCholNb / 2;
+    const bool unit = next && (warp < 2 || (warp == 2 && rank == 0)) && (u < kCholNb / 2 || lane < kCholNb / 2);
+    const int row = lane < kCholNb - u ? u + lane : lane, cc = lane < kCholNb - u ? u : kCholNb - u;
+    const bool live = unit && r1 + row < n;
+    double *out = L + (live ? (long long)(r1 + row) * n + r1 + cc : 0);
+    const double old = live ? *out : 0.0;
     __syncthreads();
-    if (i >= n) return;
+    if (i < n || next) {
 #pragma unroll
-    for (int c = 0; c < kCholNb - 1; c++) {
-        const double x = __shfl_sync(0xffffffffu, s, c);
-        const double t = fma(-x, lp[lane][c], s);
-        s = lane > c ? t : s;
+        for (int c = 0; c < kCholNb - 1; c++) {
+            const double x = __shfl_sync(0xffffffffu, s, c);
+            const double t = fma(-x, lp[lane][c], s);
+            s = lane > c ? t : s;
+        }
+        if (i < n) L[(long long)i * n + k0 + lane] = s;
     }
-    L[(long long)i * n + k0 + lane] = s;
+    if (!next) return;
+    cluster_wait();
+    const unsigned at = chol_smem(&X[rank * kPanelWarps + warp][lane]);
+#pragma unroll
+    for (int r = 0; r < kPanelCluster; r++) {
+        unsigned remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(r));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(s) : "memory");
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (!live) return;
+    double v = 0.0;
+#pragma unroll
+    for (int m = 0; m < kCholNb; m++) v = fma(X[row][m], X[cc][m], v);
+    *out = old - v;
 }
 
 // Packed FP32 rows, and the moment sums in a fixed order (one CTA reduces).
@@ -695,8 +711,8 @@ static cudaError_t launch_cholesky_blocked(const double *A, long long lda, int n
         kb = n - r0 < kCholNb ? n - r0 : kCholNb;
         const int rest = n - k0 - kb;
         if (e == cudaSuccess && rest > 0)
-            e = launch_pdl(chol_panel_kernel, (rest + kPanelWarps - 1) / kPanelWarps, 32 * kPanelWarps, 0, s, L64, n, k0,
-                           (const double *)dinv, (const int *)info);
+            e = launch_pdl(chol_panel_kernel, (rest + kCholNb - 1) / kCholNb * kPanelCluster, 32 * kPanelWarps, 0, s, L64,
+                           n, k0, (const double *)dinv, (const int *)info);
     }
     if (e != cudaSuccess) return e;
     return launch_pdl(chol_finish_kernel, (n + 7) / 8, 256, 0, s, (const double *)L64, n, Lp, aux, (const int *)info);
