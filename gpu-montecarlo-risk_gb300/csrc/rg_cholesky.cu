@@ -24,7 +24,7 @@
 //               rows of L_kk divided by their pivots.  Its first cluster of
 //               eight CTAs then subtracts its 32 rows' products from the next
 //               diagonal block (in chol_step's CTA 0 they stood before the
-//               pivots: N = 600 673 us, now 552).
+//               pivots: N = 600 673 us instead of 552).
 //   A 32 x 32 x 32 update is 19.5k cycles of one SM's FP64 pipe, hence the
 //   16 x 16 tiles (N = 600: 663 in the first step), and a row per warp in the
 //   panel (a row per lane put all 32 rows of a CTA on one sub-partition: 28 us
@@ -38,9 +38,9 @@
 // lane in the panel, 32 x 32 update tiles) and now:
 //   N        9    20    50    64    65   200   333   600   1000   2000
 //   before  34    65   178   249   188   538   924  1578   2810   7246
-//   now     11    18    49    57    68   189   310   552   1037   3440
+//   now     10    18    47    55    66   180   297   528    966   3352
 // Both forms cross at N = 64, the widest block whose columns stay in
-// registers (57 us against about 66 us blocked).
+// registers (55 us against about 64 us blocked).
 // RG_CHOLESKY=single forces cholesky_kernel, one CTA left-looking column by
 // column in place in the row-major output, above N = 64 too (a second
 // implementation that the tests compare).
@@ -194,18 +194,33 @@ __device__ __forceinline__ bool finite_bits(double v)
     return (__double_as_longlong(v) & 0x7ff0000000000000ll) != 0x7ff0000000000000ll;
 }
 
-// 1 / sqrt(d) of a positive finite d: the hardware's approximation y (about
-// 20 bits) and the binomial series of (1 - e)^(-1/2) to its second term with
-// e = 1 - d y^2; the rest, 5/16 e^3, is below FP64's rounding.  Five FP64
-// instructions, four deep, on the chain from pivot to pivot.
+// 1 / sqrt(d) of a positive finite d, in integers: an FP64 instruction takes
+// 64 cycles or more on the chain from pivot to pivot, where the Newton step in
+// FP64 (five instructions) was the longest piece: 470 cycles a column of a
+// 32-column block, now 340.  With d = x 2^(2k), 1 <= x < 4, y0 the hardware's
+// FP32 approximation to 22 bits after the point and e = 1 - x y0^2 (|e| <
+// 2^-20, exact to 2^-61), 1 / sqrt(x) = y0 (1 - e)^(-1/2) =
+// y0 (1 + e/2 + 3/8 e^2) to 5/16 e^3 < 2^-61.
+// Largest error over 2e7 arguments, on the CPU with the approximation off by
+// up to 3 ulp: 0.507 ulp (the FP64 form: 0.996).
 __device__ __forceinline__ double pivot_rsqrt(double d)
 {
-    const int ex = __double2hiint(d) >> 20; // biased exponent
-    if (ex < 64 || ex > 1983) return rsqrt(d); // out of the approximation's range
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-(d * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    const uint64_t b = (uint64_t)__double_as_longlong(d);
+    const int be = (int)(b >> 52); // biased exponent
+    if (be < 64 || be > 1983) return rsqrt(d);
+    const int ex = be - 1023, odd = ex & 1, k = ex >> 1;
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" // x cut to 24 bits
+        : "=f"(y0)
+        : "f"(__uint_as_float((uint32_t)(127 + odd) << 23 | ((uint32_t)(b >> 29) & 0x7fffffu))));
+    const uint32_t y = __float_as_uint(y0 + 2.0f) & 0x7fffffu;                        // y0 2^22
+    const uint64_t x = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << (10 + odd); // x 2^62
+    const int64_t e = (int64_t)((1ull << 61) - __umul64hi(x, (uint64_t)y * y << 19));  // e 2^61
+    const int es = (int)(e >> 12);                                                     // e 2^49
+    const int64_t c = e + ((3 * (int)(((int64_t)es * es) >> 32)) >> 7);                // (e/2 + 3/8 e^2) 2^62
+    const int64_t r = ((int64_t)y << 40) + (((int64_t)y * (c >> 2)) >> 20);            // 2^62 / sqrt(x)
+    // 53 bits, rounded; a carry out of them raises the exponent
+    return __longlong_as_double((long long)(((uint64_t)(1021 - k) << 52) + ((uint64_t)(r + 256) >> 9)));
 }
 
 // The warps that factor a block: the chain warp (0) and six bulk warps (1-3,
@@ -218,7 +233,7 @@ __device__ __forceinline__ bool chol_takes_part() { return (threadIdx.x >> 5) !=
 // a column and direction, each used once.
 struct CholFlags {
     unsigned long long fin[64]; // column final (chain -> bulk)
-    unsigned long long pre[64]; // column up to date but for the one before it (bulk -> chain)
+    unsigned long long pre[64]; // column up to date but for the two before it (bulk -> chain)
 };
 __device__ __forceinline__ unsigned chol_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void chol_flags_init(CholFlags &f)
@@ -260,11 +275,14 @@ __device__ __forceinline__ bool chol_wait(unsigned long long *bar)
 // first failing column, or -1 (a bounded wait ran out).
 //
 // Right-looking.  The chain warp, once column c - 1 is final and column c has
-// had every column before c - 1 applied, applies column c - 1, forms the pivot
-// and leaves column c final: one FMA, the reciprocal square root and one
-// multiply a column.  The bulk warps (column j in the registers of bulk warp
-// j mod 6, lane = row, two rows a lane for NC > 32) apply each final column c
-// to theirs; the one that owns column c + 2 does that one first, writes it
+// had every column before c - 2 applied, applies columns c - 2 and c - 1, forms
+// the pivot and leaves column c final: two FMAs, the reciprocal square root and
+// one multiply a column.  (With column c - 2 left to the bulk warps too, the
+// chain waited for them 280 of 1220 cycles a column of a 32-column block; now
+// 140 of 930, and the bulk warps are busy 0.8 of the time.)  The bulk warps
+// (column j in the registers of bulk warp j mod 6, lane = row, two rows a lane
+// for NC > 32) apply each final column c to theirs; the one that owns column
+// c + 3 does that one first, writes it
 // back for the chain warp and catches up with its other columns later
 // (`done`: columns applied so far).  Hand-over by column instead of a CTA
 // barrier a column lets a bulk warp fall behind while the chain goes on.
@@ -275,19 +293,23 @@ __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *failed = s_fail;
     if (warp == 0) {
-        double p[G]; // the previous column
+        double p[G], q[G]; // the previous column and the one before it
 #pragma unroll
-        for (int g = 0; g < G; g++) p[g] = 0.0;
+        for (int g = 0; g < G; g++) p[g] = q[g] = 0.0;
         int c = 0;
         for (; c < n; c++) {
-            if (c >= 2 && !chol_wait(&f.pre[c])) {
+            const double lp = -__shfl_sync(0xffffffffu, c >= 32 ? p[G - 1] : p[0], c & 31);
+            const double lq = -__shfl_sync(0xffffffffu, c >= 32 ? q[G - 1] : q[0], c & 31);
+            if (c >= 3 && !chol_wait(&f.pre[c])) {
                 if (lane == 0) *failed = -1;
                 break;
             }
             double v[G];
-            const double l = c > 0 ? -col[(c - 1) * NR + c] : 0.0;
 #pragma unroll
-            for (int g = 0; g < G; g++) v[g] = fma(p[g], l, col[c * NR + 32 * g + lane]);
+            for (int g = 0; g < G; g++) {
+                v[g] = fma(p[g], lp, fma(q[g], lq, col[c * NR + 32 * g + lane]));
+                q[g] = p[g];
+            }
             const double d = __shfl_sync(0xffffffffu, c >= 32 ? v[G - 1] : v[0], c & 31);
             if (!good_pivot(d)) { // the same value in every lane
                 if (lane == 0) *failed = c + 1;
@@ -321,13 +343,13 @@ __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv,
     // instruction whose predicate is false still takes its 64 cycles.
 #pragma unroll
     for (int s0 = 0; s0 < SL; s0++) {
-        for (int c = s0 * kCholBulk; c < (s0 + 1) * kCholBulk && c + 2 < n; c++) {
+        for (int c = s0 * kCholBulk; c < (s0 + 1) * kCholBulk && c + 3 < n; c++) {
             if (!chol_wait(&f.fin[c])) {
                 if (lane == 0) *failed = -1;
                 return;
             }
             if (*failed != 0) return;
-            if (b == (c + 2) % kCholBulk) {
+            if (b == (c + 3) % kCholBulk) {
                 // the owned column by masks: an index known only at run time
                 // would move the array to local memory
                 double v[G];
@@ -336,17 +358,17 @@ __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv,
                     long long bits = 0;
 #pragma unroll
                     for (int s = s0; s < SL; s++)
-                        bits |= __double_as_longlong(a[s][g]) & -(long long)(s == (c + 2) / kCholBulk);
+                        bits |= __double_as_longlong(a[s][g]) & -(long long)(s == (c + 3) / kCholBulk);
                     v[g] = __longlong_as_double(bits);
                 }
                 for (int k = done; k <= c; k++) {
-                    const double l = -col[k * NR + c + 2];
+                    const double l = -col[k * NR + c + 3];
 #pragma unroll
                     for (int g = 0; g < G; g++) v[g] = fma(col[k * NR + 32 * g + lane], l, v[g]);
                 }
 #pragma unroll
-                for (int g = 0; g < G; g++) col[(c + 2) * NR + 32 * g + lane] = v[g];
-                chol_arrive(&f.pre[c + 2]);
+                for (int g = 0; g < G; g++) col[(c + 3) * NR + 32 * g + lane] = v[g];
+                chol_arrive(&f.pre[c + 3]);
                 continue;
             }
             for (int k = done; k <= c; k++) {
