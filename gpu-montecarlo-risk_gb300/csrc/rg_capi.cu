@@ -334,15 +334,15 @@ static cudaError_t launch_counting(const Portfolio *p, const rg_query *q, const 
     return launch_plain_small(a, q->rng, sm_count, s);
 }
 
-// Bytes for the block table of a query of the tensor-core or the tiled FP32
-// kernel with enough normals that the table's own launch (about 3 us) pays:
-// a few per cent of a generator that draws 1.2e12 normals a second.
+// Bytes for the block table of a query of the tensor-core kernel with enough
+// normals that the table's own launch (about 3 us) pays: a few per cent of a
+// generator that draws 1.3e12 normals a second.  (The tiled FP32 kernel takes
+// none: see its generator.)
 static size_t table_bytes(const Portfolio *p, const rg_query *q)
 {
     const bool tensor = q->precision == RG_PREC_BF16X3 || q->precision == RG_PREC_FP16X3;
-    const bool tiled = !tensor && q->rng == RG_RNG_PHILOX && p->n > fused_max_n();
     const int days = q->draw_mode == RG_DRAWS_AGGREGATED ? 1 : q->horizon;
-    if (!(tensor || tiled) || (double)q->n_paths * p->n * days < 1e8) return 0;
+    if (!tensor || (double)q->n_paths * p->n * days < 1e8) return 0;
     return sizeof(PhiloxBlock) * philox_table_len(p->n, days, q->path_offset, q->n_paths);
 }
 

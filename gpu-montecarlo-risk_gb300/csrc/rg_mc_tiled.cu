@@ -4,7 +4,7 @@
 // at its definition: the pipelined mc_tiled_pipe_kernel (default), the
 // phase-serial mc_tiled_kernel it is built from (RG_PLAIN_KERNEL=serial) and
 // the warp-specialised mc_tiled_ws_kernel (RG_PLAIN_KERNEL=ws).  At N = 600,
-// H = 10, 1e7 paths: 111.6, 136.6 and 170 ms with daily draws; 83.2, 94.1
+// H = 10, 1e7 paths: 112.3, 136.6 and 170 ms with daily draws; 82.8, 94.1
 // and 149 ms with aggregated draws.
 //
 // Phase-serial form: a CTA owns a tile of 64 paths at a time (grid-stride
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kWsThreadsT, 1) mc_tiled_ws_kernel(const Tiled
 //              range r.
 //   warps 8-15 normals of the next tile, range by range from the top
 //              (waiting on RELEASE[r], then arriving on FILLED[r]); two quads
-//              at a time with their Philox rounds interleaved (rg_philox2).
+//              at a time with their Philox rounds interleaved (rg_philox2_from).
 // At N = 600 the bottom range, released last, is needed only at the end of
 // the next tile's top block, so generation and GEMM overlap almost entirely.
 // The GEMM is the phase-serial kernel's (4-path x 8-asset FFMA2 tiles,
@@ -553,7 +553,6 @@ __global__ void __launch_bounds__(kPipeThreads, 1) mc_tiled_pipe_kernel(const Ti
         const int gt = tid - kPipeHalf;
         const int p = gt & (kTP - 1), r4 = gt >> 6; // 4 threads per path
         const int days = t.aggregated ? 1 : a.horizon;
-        const uint4 *blocks = reinterpret_cast<const uint4 *>(a.blocks);
         for (long long j = 0; j < my_tiles; j++) {
             const long long p0 = ((long long)blockIdx.x + j * gridDim.x) * kTP;
             const unsigned long long path = a.path0 + (unsigned long long)(p0 + p);
@@ -581,23 +580,26 @@ __global__ void __launch_bounds__(kPipeThreads, 1) mc_tiled_pipe_kernel(const Ti
                         y.z += y2;
                         y.w += y3;
                     };
-                    // both quads real: rounds 1-2 from the block table (N = 600,
-                    // H = 10, 5e5 paths 5.77 -> 5.69 ms; two or three days side
-                    // by side 5.71 and 5.70)
-                    if (blocks && q2 < nq) {
-                        for (int d = 0; d < days; d++) {
-                            uint4 wa, wb;
-                            rg_philox2_from(__ldg(blocks + (size_t)d * nq + q), __ldg(blocks + (size_t)d * nq + q2), pc,
-                                            a.keys, wa, wb);
-                            add(wa, wb);
-                        }
-                    } else {
-                        for (int d = 0; d < days; d++) {
-                            uint4 wa = make_uint4((uint32_t)(d * nq + q), 0u, plo, phi);
-                            uint4 wb = make_uint4((uint32_t)(d * nq + q2), 0u, plo, phi);
-                            rg_philox2(wa, wb, a.keys);
-                            add(wa, wb);
-                        }
+                    // The path's part of Philox rounds 1-2 once a tile, two days
+                    // a turn.  FP32, before (neither) -> now, ms: N = 67, H = 20,
+                    // 463,001 paths 0.977 -> 0.850; N = 130, H = 10, 1e6 paths
+                    // 2.223 -> 2.103; N = 300, 6e5 paths 2.643 -> 2.592; N = 600,
+                    // 2e5 paths 2.345 -> 2.324; N = 67, H = 2, 4e6 paths 2.129 ->
+                    // 2.085.  One of the two alone: two days a turn 0.891, 2.134,
+                    // 2.602, 2.332, 2.090; the path's part 0.960, 2.235, 2.654,
+                    // 2.346, 2.120.  Four days a turn: 0.829, 2.089, 2.577, 2.325,
+                    // but 2.166 with two days.  The block's part from a table
+                    // (as in rg_mc_tc.cu), one day a turn: 0.985, 2.306, 2.669,
+                    // 2.330, 2.180 (its loads share this kernel's shared-memory
+                    // bandwidth).
+#pragma unroll 2
+                    for (int d = 0; d < days; d++) {
+                        const PhiloxBlock ba = philox_block((uint32_t)(d * nq + q), phi, a.keys);
+                        const PhiloxBlock bb = philox_block((uint32_t)(d * nq + q2), phi, a.keys);
+                        uint4 wa, wb;
+                        rg_philox2_from(make_uint4(ba.x, ba.y, ba.z, 0u), make_uint4(bb.x, bb.y, bb.z, 0u), pc, a.keys,
+                                        wa, wb);
+                        add(wa, wb);
                     }
                     z.x *= t.zscale;
                     z.y *= t.zscale;
@@ -796,12 +798,6 @@ cudaError_t launch_tiled(const PlainArgs &a, const float *Lt, bool aggregated, i
                             : kt == 16 ? mc_tiled_pipe_kernel<false, 16> : mc_tiled_pipe_kernel<false, 8>);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        if (a.blocks) {
-            const size_t len = philox_table_len(a.n, aggregated ? 1 : a.horizon, a.path0, a.n_paths);
-            if (len) e = launch_philox_table(a.blocks, len, a.path0, a.keys, s);
-            else t.a.blocks = nullptr;
-            if (e != cudaSuccess) return e;
-        }
         long long tiles = (a.n_paths + kTP - 1) / kTP;
         long long grid = sm_count;
         if (tiles < grid) grid = tiles;
