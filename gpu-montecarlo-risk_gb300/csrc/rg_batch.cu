@@ -290,7 +290,9 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     }
     for (int i = 0; i < count; i++) b->queries.push_back(items[i].query);
     b->total_tiles = tile;
-    e = cudaMemcpy(b->d_items, host.data(), host.size(), cudaMemcpyHostToDevice);
+    // on one stream: a copy from pageable memory may return once it is staged,
+    // and cap_stream does not wait for the legacy stream
+    e = cudaMemcpyAsync(b->d_items, host.data(), host.size(), cudaMemcpyHostToDevice, b->cap_stream);
     if (e == cudaSuccess && blocks) e = launch_batch_tables(b->d_items, count, b->cap_stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->cap_stream);
     if (e != cudaSuccess) {

@@ -1,0 +1,41 @@
+"""Host side of batches on the fake runtime: the order of the runtime calls that
+set a batch up."""
+import numpy as np
+import pytest
+
+import host_engine
+import riskgpu
+
+
+@pytest.fixture(scope="module")
+def linked(tmp_path_factory):
+    return host_engine.link(str(tmp_path_factory.mktemp("linked")))
+
+
+@pytest.fixture
+def fake(linked, tmp_path, monkeypatch):
+    monkeypatch.setenv("RG_TUNE_CACHE", str(tmp_path / "tune.json"))
+    with host_engine.engine(linked, str(tmp_path)) as f:
+        yield f
+
+
+def _items(sizes, horizon=8, paths=20_000, **more):
+    more = dict(dict(precision=riskgpu.PREC_BF16X3), **more)
+    return [(riskgpu.Portfolio(np.zeros(n), np.eye(n), np.full(n, 1.0 / n)),
+             riskgpu.make_query(paths, 7 + i, horizon=horizon, **more)) for i, n in enumerate(sizes)]
+
+
+def test_item_table_is_on_the_device_before_the_table_kernel_reads_it(fake):
+    """The upload and the kernel share a stream, or something between them
+    waits: a copy from pageable memory on another stream may return before its
+    data has arrived."""
+    items = _items([10, 80, 300])
+    fake.reset()
+    batch = riskgpu.Batch(items)
+    log = fake.log()
+    at = next(i for i, (name, _, d) in enumerate(log) if name == "launch" and "batch_tables" in d)
+    up = max(i for i in range(at) if log[i][0].startswith("cudaMemcpy") and log[i][2].startswith("H2D"))
+    waited = any(name == "cudaStreamSynchronize" and s == log[up][1] or name == "cudaDeviceSynchronize"
+                 for name, s, _ in log[up + 1:at])
+    assert log[up][1] == log[at][1] or waited, (log[up], log[at])
+    batch.close()
