@@ -479,7 +479,9 @@ __global__ void __launch_bounds__(kCholCta, 1) chol_small_kernel(
 // ------------------------------------------------------------ blocked form
 // Start of a kernel launched programmatically behind the previous one: let
 // the next one be scheduled, then wait until the previous one's writes are
-// visible.
+// visible.  Such a kernel runs while its predecessor still writes L, dinv and
+// info, so none of its pointers is __restrict__: that (with const, the
+// read-only cache too) would let a load be placed before the wait.
 __device__ __forceinline__ void pdl_enter()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -529,8 +531,7 @@ __global__ void chol_prep_kernel(const double *__restrict__ A, long long lda, in
 // r0 = k0 + kb, beside CTA 0, which factors the 32 x 32 diagonal block at r0
 // (the panel's kernel has brought it up to date) and leaves its reciprocal
 // pivots in dinv.
-__global__ void __launch_bounds__(kCholCta, 1) chol_step_kernel(double *__restrict__ L, int n, int k0, int kb,
-                                                                    double *__restrict__ dinv, int *__restrict__ info)
+__global__ void __launch_bounds__(kCholCta, 1) chol_step_kernel(double *L, int n, int k0, int kb, double *dinv, int *info)
 {
     __shared__ double P[kCholTile][kCholNb + 1];
     __shared__ double col[kCholNb * kCholNb];
@@ -609,8 +610,7 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(32 * kPanelWarps)
-    chol_panel_kernel(double *__restrict__ L, int n, int k0, const double *__restrict__ dinv,
-                      const int *__restrict__ info)
+    chol_panel_kernel(double *L, int n, int k0, const double *dinv, const int *info)
 {
     __shared__ double lp[kCholNb][kCholNb + 1];
     __shared__ double X[kCholNb][kCholNb + 1]; // cluster 0: the rows of the next diagonal block
@@ -664,8 +664,7 @@ __global__ void __cluster_dims__(kPanelCluster, 1, 1) __launch_bounds__(32 * kPa
 }
 
 // Packed FP32 rows, and the moment sums in a fixed order (one CTA reduces).
-__global__ void chol_finish_kernel(const double *__restrict__ L, int n, float *__restrict__ Lp,
-                                   double *__restrict__ aux, const int *__restrict__ info)
+__global__ void chol_finish_kernel(const double *L, int n, float *Lp, double *aux, const int *info)
 {
     __shared__ double red[33];
     pdl_enter();
