@@ -709,15 +709,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) mc_tc_kernel(const __grid_const
 //                per generator thread)
 //   zempty[z]    MMA -> generator: the MMAs that read slot z are complete (one
 //                arrival per issuer)
-//   full/empty   Lhat ring (copy completion, MMA completion)
+//   full/empty   Lhat ring (copy completion, MMA completion); SPLIT: a ring of
+//                its own for each issuer
 //   acc_full[m]  MMA -> epilogue: row tile m of the tile accumulated
 //   acc_free[m]  epilogue -> MMA: row tile m read (one arrival per warp)
-//   slot_free[s] epilogue -> first generator warp: the tile in slot s is finished
+//   slot_free[s] epilogue (and, SPLIT, each issuer) -> first generator warp:
+//                the tile in slot s is finished
 // The K-tile number g, use counts per row tile and per tile slot (the same
 // on both sides of each barrier) give the phase parities, since items of a
-// batch differ in size.  The tile index is read after tile_pub, never after
-// zfull[0]: slot s is republished only after the epilogue finished the tile
-// that used it, so no waiter can fall a whole phase behind.
+// batch differ in size.  A parity wait is sound only for a waiter that sees
+// every phase: a barrier's next phase may end only after all its waiters have
+// seen the last.  The tile index is read after tile_pub, never after zfull[0],
+// and slot s is republished only after the epilogue finished the tile that
+// used it, which takes the work of the generator, of the copy warp and of the
+// issuers that own a row tile; an issuer that owns none (SPLIT, N <= 127) is
+// held to it by its own arrival on slot_free.  A stage of the Lhat ring serves
+// one issuer, which so sees all its phases; in one ring for both, each would
+// have to wait for the other's pairs too (copies complete in any order), which
+// took 2010 us where this takes 1842 (N = 487, aggregated, 2e6 paths).
 static constexpr int kWsThreads = 1024;
 static constexpr int kWsEpiWarps = 4;
 static constexpr unsigned kWsTileSlots = 3; // path tiles published: generated, multiplied or read back, next
@@ -805,6 +814,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     constexpr int kWsGenWarp0 = SPLIT ? 7 : 5;
     constexpr int kIssuers = SPLIT ? 2 : 1;
     constexpr int kWsGenThreads = kWsThreads - 32 * kWsGenWarp0;
+    constexpr unsigned kRing0 = SPLIT ? (kStages + 1) / 2 : kStages; // Lhat stages of the first issuer
     // days drawn side by side in the daily form: N = 600, H = 10, 4e6 paths
     // 19.4 -> 18.7 ms (3 days 18.8, 5 days 18.8); the aggregated form draws one
     constexpr int kUnroll = SPLIT ? 1 : 2;
@@ -852,7 +862,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
         }
         for (int s = 0; s < kWsTileSlots; s++) {
             mbar_init(&tile_pub[s], 1);
-            mbar_init(&slot_free[s], 1);
+            mbar_init(&slot_free[s], SPLIT ? 1 + kIssuers : 1);
         }
         for (int i = 0; i < kIssuers; i++) mbar_init(&drain_bar[i], 1);
         tm_abort = 0;
@@ -1019,8 +1029,8 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
     } else if (SPLIT && warp == kWsMmaWarp + 1) {
         // ======================= Lhat producer =======================
         // (the whole warp in step, one elected lane issuing, as the MMA warp)
-        unsigned prod_iter = 0;
-        int skipped = -1; // the stage left unfilled by the fault injection
+        unsigned made[2] = {0, 0}; // copies into each issuer's ring
+        int skipped = -1;          // the stage left unfilled by the fault injection
         auto same = [](int v) -> int { return __shfl_sync(0xffffffffu, v, 0); };
         auto wait = [&](uint64_t *bar, unsigned par) -> bool { return same(mbar_wait(bar, par) ? 1 : 0) != 0; };
         bool dead = false;
@@ -1037,31 +1047,35 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
             for (int kt = 0; kt < n_kt && !dead; kt++) {
                 for (int mt = 0; mt < n_mt; mt++) {
                     if (kt >= tc_kts(mt, n_mt, n_kt)) continue;
-                    const int s = (int)(prod_iter % kStages);
-                    if (same(tm_abort) || !wait(&empty_bar[s], ((prod_iter / kStages) & 1u) ^ 1u)) {
+                    const unsigned me = mt & 1, size = me ? kStages - kRing0 : kRing0;
+                    const unsigned s = (me ? kRing0 : 0u) + made[me] % size;
+                    if (same(tm_abort) || !wait(&empty_bar[s], ((made[me] / size) & 1u) ^ 1u)) {
                         if (lane == 0) atomicOr(b.err, 1u);
                         tm_abort = 1;
                         dead = true;
                         break;
                     }
-                    if (b.inject_stall && prod_iter == 1) { // never filled: the consumer's wait runs out
-                        skipped = (int)prod_iter++;
-                        continue;
-                    }
-                    if (elect_one()) {
+                    if (b.inject_stall && made[0] + made[1] == 1) { // never filled: the consumer's wait runs out
+                        skipped = (int)s;
+                    } else if (elect_one()) {
                         mbar_expect_tx(&full_bar[s], 2 * kTcTileBytes);
                         const unsigned char *src = it.tiles + ((size_t)(mt * n_kt + kt) * 2) * kTcTileBytes;
                         unsigned char *dst = lst + (size_t)s * 2 * kTcTileBytes;
                         bulk_copy(dst, src, kTcTileBytes, &full_bar[s]);
                         bulk_copy(dst + kTcTileBytes, src + kTcTileBytes, kTcTileBytes, &full_bar[s]);
                     }
-                    prod_iter++;
+                    made[me]++;
                 }
             }
         }
         // the copies still in flight land before the kernel ends
-        for (unsigned i = prod_iter > kStages ? prod_iter - kStages : 0; i < prod_iter; i++)
-            if ((int)i != skipped) mbar_wait(&full_bar[i % kStages], (i / kStages) & 1u);
+        for (unsigned me = 0; me < 2; me++) {
+            const unsigned size = me ? kStages - kRing0 : kRing0;
+            for (unsigned i = made[me] > size ? made[me] - size : 0; i < made[me]; i++) {
+                const unsigned s = (me ? kRing0 : 0u) + i % size;
+                if ((int)s != skipped) mbar_wait(&full_bar[s], (i / size) & 1u);
+            }
+        }
         __syncwarp();
     } else if (warp == kWsMmaWarp || (SPLIT && warp == kWsMmaWarp + 2)) {
         // ============ MMA issue (and, unless SPLIT, the Lhat copies) ============
@@ -1143,7 +1157,9 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
         };
 
         unsigned g0 = 0, fpar = 0; // fpar bit m: parity of the uses of row tile m
-        unsigned rs = 0, rph = 0;  // Lhat ring: stage and phase parity of pair ci
+        // this issuer's Lhat ring: first stage, stages, and stage and phase parity of pair ci
+        const unsigned ring0 = me ? kRing0 : 0u, ring = me ? kStages - kRing0 : kRing0;
+        unsigned rs = 0, rph = 0;
         const uint32_t lst_lo = sw128_desc_lo(smem_u32(lst));
         bool dead = false;
         for (unsigned j = 0; !dead && !same(tm_abort); j++) {
@@ -1170,18 +1186,12 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                 for (int mt = 0; mt < n_mt; mt++) {
                     const int kts = tc_kts(mt, n_mt, n_kt);
                     if (kt >= kts) continue;
-                    if (SPLIT && (mt & 1) != me) { // the other issuer's pair
-                        if (++rs == kStages) {
-                            rs = 0;
-                            rph ^= 1u;
-                        }
-                        continue;
-                    }
+                    if (SPLIT && (mt & 1) != me) continue; // the other issuer's pair
                     // the first write to row tile mt: the epilogue has read the previous tile's
                     unsigned bad = 0u;
                     if (kt == 0 && !wait(&acc_free[mt], ((fpar >> mt) & 1u) ^ 1u)) bad = 128u;
                     else if (!SPLIT && !pump(true)) bad = 1u;
-                    else if (!wait(&full_bar[rs], rph)) bad = 2u;
+                    else if (!wait(&full_bar[ring0 + rs], rph)) bad = 2u;
                     if (bad) {
                         give_up(bad);
                         dead = true;
@@ -1189,19 +1199,20 @@ __global__ void __launch_bounds__(kWsThreads, 1) mc_tcws_kernel(const __grid_con
                     }
                     tc_fence_after();
                     if (elect_one()) {
-                        tc_mma_pair(tm + (uint32_t)(mt * P), lst_lo + rs * (2 * kTcTileBytes >> 4), zh_lo, zl_lo, idesc,
-                                    kt > 0 ? 1u : 0u);
-                        tc_commit(&empty_bar[rs]);
+                        tc_mma_pair(tm + (uint32_t)(mt * P), lst_lo + (ring0 + rs) * (2 * kTcTileBytes >> 4), zh_lo, zl_lo,
+                                    idesc, kt > 0 ? 1u : 0u);
+                        tc_commit(&empty_bar[ring0 + rs]);
                         if (kt == kts - 1) tc_commit(&acc_full[mt]); // row tile mt complete
                     }
                     ci++;
-                    if (++rs == kStages) {
+                    if (++rs == ring) {
                         rs = 0;
                         rph ^= 1u;
                     }
                 }
                 if (elect_one()) tc_commit(&zempty[zs]); // the slot may be overwritten once these MMAs complete
             }
+            if (SPLIT && !dead && elect_one()) mbar_arrive(&slot_free[slot]); // this issuer has read the tile's slot
             g0 += (unsigned)n_kt;
             fpar ^= (1u << n_mt) - 1u;
         }
@@ -1518,9 +1529,10 @@ double tc_tile_mma(int n) { return 12.0 * 80.0 * tc_pairs(n); }
 
 // Whether the split form (a copy warp, two MMA warps, 25 generator warps) is
 // the faster one: below about three times as many cycles of normals as of
-// MMAs.  1e6 paths, merged and split, us: N = 600 H = 1 2499 and 1559, H = 5
-// 3093 and 2701, H = 10 4682 and 4933; N = 333 H = 3 1108 and 1029, H = 4 1237
-// and 1278; N = 130 H = 3 489 and 469, H = 4 552 and 561.
+// MMAs.  1e6 paths, merged and split, us: N = 600 H = 1 2529 and 1573, H = 5
+// 3180 and 2746, H = 8 3808 and 4098; N = 333 H = 3 1124 and 1056, H = 4 1259
+// and 1305; N = 130 H = 3 502 and 477, H = 4 563 and 575; N = 64 H = 1 214 and
+// 197.
 bool tc_split_wins(double gen, double mma) { return gen < 3.0 * mma; }
 
 // Paths per tile of a query on sm_count SMs, at most `most`: the multiple of
