@@ -530,7 +530,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     DevCtx *ctx;
     int dev;
     int st = get_ctx(&ctx, &dev);
-    if (st) return finite_inputs() ? RG_ERR_INVALID : get_ctx(&ctx, &dev);
+    if (st) return finite_inputs() ? RG_ERR_INVALID : st; // (a finite input leaves the message as it is)
     const size_t nn = (size_t)n * n;
     const bool want_lt = (parts & kPartLt) && n <= tiled_max_n();
     const bool want_tc[2] = {(parts & kPartTcFp16) && n <= tc_max_n(), (parts & kPartTcBf16) && n <= tc_max_n()};
@@ -538,7 +538,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
                         (want_lt ? (size_t)tiled_kpad(n) * tiled_npad(n) * 4 : 0) +
                         (want_tc[0] ? tc_tile_bytes(n) : 0) + (want_tc[1] ? tc_tile_bytes(n) : 0) + 64;
     st = admit(need);
-    if (st) return finite_inputs() ? RG_ERR_INVALID : admit(need);
+    if (st) return finite_inputs() ? RG_ERR_INVALID : st;
 
     Portfolio *p = new Portfolio();
     p->n = n;

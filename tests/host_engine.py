@@ -9,6 +9,8 @@ import os
 import shutil
 import subprocess
 
+import pytest
+
 import riskgpu
 from riskgpu import build
 
@@ -75,3 +77,16 @@ def engine(linked, folder):
             if isinstance(o, (riskgpu.Portfolio, riskgpu.Batch, riskgpu.Server)):
                 o._h = ctypes.c_void_p()
         riskgpu.LIB_PATH, riskgpu._lib = was
+
+
+# ---- fixtures (imported by the test files)
+@pytest.fixture(scope="session")
+def linked(tmp_path_factory):
+    return link(str(tmp_path_factory.mktemp("linked")))
+
+
+@pytest.fixture
+def fake(linked, tmp_path, monkeypatch):
+    monkeypatch.setenv("RG_TUNE_CACHE", str(tmp_path / "tune.json"))
+    with engine(linked, str(tmp_path)) as f:
+        yield f

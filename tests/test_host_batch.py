@@ -1,22 +1,9 @@
 """Host side of batches on the fake runtime: the order of the runtime calls that
 set a batch up."""
 import numpy as np
-import pytest
 
-import host_engine
 import riskgpu
-
-
-@pytest.fixture(scope="module")
-def linked(tmp_path_factory):
-    return host_engine.link(str(tmp_path_factory.mktemp("linked")))
-
-
-@pytest.fixture
-def fake(linked, tmp_path, monkeypatch):
-    monkeypatch.setenv("RG_TUNE_CACHE", str(tmp_path / "tune.json"))
-    with host_engine.engine(linked, str(tmp_path)) as f:
-        yield f
+from host_engine import fake, linked  # noqa: F401
 
 
 def _items(sizes, horizon=8, paths=20_000, **more):
