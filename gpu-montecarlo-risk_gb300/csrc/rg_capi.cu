@@ -58,13 +58,15 @@ struct QueryRes {
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
 // alone: 228 us, of which about 190).  `idle` keeps the resources of a few
-// calls for the next ones.
+// calls for the next ones.  `held`: blocks of destroyed portfolios that wait
+// for the device (block_release).
 struct DevCtx {
     bool ready = false;
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;
     std::vector<QueryRes> idle;
+    std::vector<void *> held;
 };
 
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
@@ -224,9 +226,38 @@ static int admit(size_t need)
     return RG_OK;
 }
 
+// Waits for all work of the current device, also on streams of the caller's.
+// False where the wait is refused, as it is while a stream of the device is
+// being captured: nothing has been waited for then.
+static bool device_wait()
+{
+    if (cudaDeviceSynchronize() == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// A block of the current device goes back to the pool once no work can use it.
+// Where the wait is refused it is held, with those before it, until a later
+// call of this function (at the next destruction or creation) gets one.
+static void block_release(DevCtx *c, void *block)
+{
+    std::vector<void *> done;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        done.swap(c->held);
+    }
+    if (block) done.push_back(block);
+    if (done.empty()) return;
+    if (device_wait()) {
+        for (void *b : done) cudaFreeAsync(b, c->stream);
+        return;
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    c->held.insert(c->held.end(), done.begin(), done.end());
+}
+
 // `quiet`: no work that uses the portfolio is in flight on any stream.
-// Otherwise the device is waited for first, as cudaFree would: a caller may
-// have launched on a stream of its own.
+// Otherwise a caller may have launched on a stream of its own.
 static void portfolio_free(Portfolio *p, bool quiet)
 {
     if (!p) return;
@@ -234,9 +265,11 @@ static void portfolio_free(Portfolio *p, bool quiet)
         int dev = p->device;
         cudaGetDevice(&dev);
         if (dev != p->device) cudaSetDevice(p->device);
-        if (!quiet) cudaDeviceSynchronize();
         DevCtx *c = nullptr;
-        if (get_ctx(&c, nullptr) == RG_OK) cudaFreeAsync(p->d_block, c->stream);
+        if (get_ctx(&c, nullptr) == RG_OK) {
+            if (quiet) cudaFreeAsync(p->d_block, c->stream);
+            else block_release(c, p->d_block);
+        }
         if (dev != p->device) cudaSetDevice(dev);
     }
     delete p;
@@ -531,6 +564,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     int dev;
     int st = get_ctx(&ctx, &dev);
     if (st) return finite_inputs() ? RG_ERR_INVALID : st; // (a finite input leaves the message as it is)
+    block_release(ctx, nullptr);
     const size_t nn = (size_t)n * n;
     const bool want_lt = (parts & kPartLt) && n <= tiled_max_n();
     const bool want_tc[2] = {(parts & kPartTcFp16) && n <= tc_max_n(), (parts & kPartTcBf16) && n <= tc_max_n()};

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import riskgpu
-from host_engine import fake, linked  # noqa: F401
+from host_engine import CAPTURE_REFUSED, fake, linked  # noqa: F401
 
 
 def _create(n=8, bad=None):
@@ -37,3 +37,26 @@ def test_a_missing_device_stays_missing(fake):
     fake.fail("cudaGetDeviceCount", 100)
     st, h, message = _create()
     assert (st, h) == (riskgpu.RG_ERR_NO_DEVICE, None) and "no CUDA device" in message
+
+
+FREES = ("cudaFree", "cudaFreeAsync")
+
+
+def test_a_portfolio_outlives_a_refused_wait(fake):
+    """Destroyed while a stream capture forbids waiting for the device: work
+    launched with it may be in flight, so its memory is not handed on until a
+    wait has succeeded, and is then."""
+    port = riskgpu.Portfolio(np.zeros(70), np.eye(70))
+    before = fake.live()
+    fake.reset()
+    for name in ("cudaDeviceSynchronize", "cudaFree"):
+        fake.fail(name, CAPTURE_REFUSED, count=-1, until="cudaGetErrorString")
+    port.close()
+    assert fake.live() == before and "cudaFreeAsync" not in fake.names()
+    fake.reset()  # the capture has ended
+    other = riskgpu.Portfolio(np.zeros(3), np.eye(3))
+    names = fake.names()
+    free = next(i for i, name in enumerate(names) if name in FREES)
+    assert names[free] == "cudaFree" or "cudaDeviceSynchronize" in names[:free]
+    other.close()
+    assert fake.live() < before
