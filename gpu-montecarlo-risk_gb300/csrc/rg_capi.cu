@@ -58,19 +58,29 @@ struct QueryRes {
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
 // alone: 228 us, of which about 190).  `idle` keeps the resources of a few
-// calls for the next ones.  `held`: blocks of destroyed portfolios that wait
-// for the device (block_release).
+// calls for the next ones.  A resident portfolio has a block from cudaMalloc,
+// since its d_L and d_packed are the caller's to map on a peer or to export to
+// another process, which a pool's memory does not allow.  `spare`: at most
+// kSpareBlocks such blocks, kSpareKeep bytes, of destroyed portfolios, for the
+// next of the same size (creating and destroying one at N = 600: 0.15 ms more
+// with a cudaMalloc and a cudaFree each time); pool_trim frees them.  `held`:
+// those that still wait for the device (block_release).
+struct Block {
+    void *p;
+    size_t bytes;
+};
 struct DevCtx {
     bool ready = false;
     int sm_count = 0;
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;
     std::vector<QueryRes> idle;
-    std::vector<void *> held;
+    std::vector<Block> spare, held;
 };
 
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
 static constexpr size_t kIdleQueries = 8;
+static constexpr size_t kSpareBlocks = 8, kSpareKeep = 32u << 20;
 
 static std::mutex g_mu;
 static DevCtx g_ctx[64];
@@ -134,14 +144,25 @@ int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
     return RG_OK;
 }
 
-// Everything the pool of the current device keeps but does not use goes back
-// to the driver.
+// What the engine keeps on the current device but does not use goes back to
+// the driver.
 void pool_trim()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (g_ctx[dev].pool) cudaMemPoolTrimTo(g_ctx[dev].pool, 0);
+    DevCtx &c = g_ctx[dev];
+    std::vector<Block> spare;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (c.pool) cudaMemPoolTrimTo(c.pool, 0);
+        spare.swap(c.spare);
+    }
+    for (const Block &b : spare)
+        if (cudaFree(b.p) != cudaSuccess) { // refused beside a stream capture
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lk(g_mu);
+            c.held.push_back(b);
+        }
 }
 
 static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
@@ -236,29 +257,65 @@ static bool device_wait()
     return false;
 }
 
-// A block of the current device goes back to the pool once no work can use it.
-// Where the wait is refused it is held, with those before it, until a later
-// call of this function (at the next destruction or creation) gets one.
-static void block_release(DevCtx *c, void *block)
+// A resident portfolio's block becomes a spare one (or is freed) once no work
+// can use it.  Where the wait is refused it is held, with those before it,
+// until a later call of this function (at the next destruction or creation)
+// gets one.
+static void block_release(DevCtx *c, Block block)
 {
-    std::vector<void *> done;
+    std::vector<Block> done;
     {
         std::lock_guard<std::mutex> lk(g_mu);
         done.swap(c->held);
     }
-    if (block) done.push_back(block);
+    if (block.p) done.push_back(block);
     if (done.empty()) return;
-    if (device_wait()) {
-        for (void *b : done) cudaFreeAsync(b, c->stream);
-        return;
+    const bool idle = device_wait();
+    for (const Block &b : done) {
+        {
+            std::lock_guard<std::mutex> lk(g_mu);
+            size_t kept = b.bytes;
+            for (const Block &o : c->spare) kept += o.bytes;
+            const bool room = kept <= kSpareKeep && c->spare.size() < kSpareBlocks;
+            if (!idle || room) {
+                (idle ? c->spare : c->held).push_back(b);
+                continue;
+            }
+        }
+        if (cudaFree(b.p) != cudaSuccess) {
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lk(g_mu);
+            c->held.push_back(b);
+        }
     }
-    std::lock_guard<std::mutex> lk(g_mu);
-    c->held.insert(c->held.end(), done.begin(), done.end());
 }
 
-// `quiet`: no work that uses the portfolio is in flight on any stream.
-// Otherwise a caller may have launched on a stream of its own.
-static void portfolio_free(Portfolio *p, bool quiet)
+// A spare block of just this size, or a new one.
+static cudaError_t block_take(DevCtx *c, size_t bytes, void **p)
+{
+    block_release(c, Block{nullptr, 0});
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        for (size_t i = 0; i < c->spare.size(); i++)
+            if (c->spare[i].bytes == bytes) {
+                *p = c->spare[i].p;
+                c->spare.erase(c->spare.begin() + (long)i);
+                return cudaSuccess;
+            }
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        pool_trim();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+// A pooled portfolio (of one call, or of the plugin cache) goes back to the
+// pool: every call that used it has waited for its work.  A resident one may
+// still be in use on a stream of the caller's.
+static void portfolio_free(Portfolio *p)
 {
     if (!p) return;
     if (p->d_block) {
@@ -267,8 +324,8 @@ static void portfolio_free(Portfolio *p, bool quiet)
         if (dev != p->device) cudaSetDevice(p->device);
         DevCtx *c = nullptr;
         if (get_ctx(&c, nullptr) == RG_OK) {
-            if (quiet) cudaFreeAsync(p->d_block, c->stream);
-            else block_release(c, p->d_block);
+            if (p->pooled) cudaFreeAsync(p->d_block, c->stream);
+            else block_release(c, Block{p->d_block, p->block_bytes});
         }
         if (dev != p->device) cudaSetDevice(dev);
     }
@@ -530,16 +587,16 @@ static unsigned parts_for_query(const rg_query *q, int n)
 }
 
 static int create_portfolio(int32_t n, const double *mu, const double *sigma, int64_t ld, const double *weights,
-                            int32_t flags, unsigned parts, rg_portfolio **out);
+                            int32_t flags, unsigned parts, bool pooled, rg_portfolio **out);
 
 int rg_portfolio_create(int32_t n, const double *mu, const double *sigma, int64_t ld,
                         const double *weights, int32_t flags, rg_portfolio **out)
 {
-    return create_portfolio(n, mu, sigma, ld, weights, flags, kPartAll, out);
+    return create_portfolio(n, mu, sigma, ld, weights, flags, kPartAll, false, out);
 }
 
 static int create_portfolio(int32_t n, const double *mu, const double *sigma, int64_t ld, const double *weights,
-                            int32_t flags, unsigned parts, rg_portfolio **out)
+                            int32_t flags, unsigned parts, bool pooled, rg_portfolio **out)
 {
     if (!out) return set_error(RG_ERR_INVALID, "out is NULL");
     *out = nullptr;
@@ -564,7 +621,6 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     int dev;
     int st = get_ctx(&ctx, &dev);
     if (st) return finite_inputs() ? RG_ERR_INVALID : st; // (a finite input leaves the message as it is)
-    block_release(ctx, nullptr);
     const size_t nn = (size_t)n * n;
     const bool want_lt = (parts & kPartLt) && n <= tiled_max_n();
     const bool want_tc[2] = {(parts & kPartTcFp16) && n <= tc_max_n(), (parts & kPartTcBf16) && n <= tc_max_n()};
@@ -578,6 +634,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     p->n = n;
     p->has_w = weights ? 1 : 0;
     p->device = dev;
+    p->pooled = pooled;
     double *dA = nullptr, *dW = nullptr;
     const double *A = sigma, *W = weights, *MU = mu;
     long long lda = ld;
@@ -596,7 +653,9 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t ow32 = bp.take((size_t)n * sizeof(float));
         const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
-        RG_CUDA_TRY(cudaMallocFromPoolAsync(&p->d_block, bp.total, ctx->pool, s));
+        p->block_bytes = bp.total;
+        if (pooled) RG_CUDA_TRY(cudaMallocFromPoolAsync(&p->d_block, bp.total, ctx->pool, s));
+        else RG_CUDA_TRY(block_take(ctx, bp.total, &p->d_block));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
         p->d_L64 = reinterpret_cast<double *>(blk + oL64);
         p->d_mu64 = reinterpret_cast<double *>(blk + omu);
@@ -689,14 +748,14 @@ fail:
     if (dA) cudaFreeAsync(dA, s);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    portfolio_free(p, true);
+    portfolio_free(p);
     return st;
 }
 
 int rg_portfolio_destroy(rg_portfolio *h)
 {
     if (!h) return RG_OK;
-    portfolio_free(reinterpret_cast<Portfolio *>(h), false);
+    portfolio_free(reinterpret_cast<Portfolio *>(h));
     return RG_OK;
 }
 
@@ -953,10 +1012,10 @@ int rg_run(int32_t n, const double *mu, const double *sigma, int64_t ld, const d
     int st = validate_query(nullptr, q);
     if (st) return st;
     rg_portfolio *h = nullptr;
-    st = create_portfolio(n, mu, sigma, ld, weights, 0, parts_for_query(q, n), &h);
+    st = create_portfolio(n, mu, sigma, ld, weights, 0, parts_for_query(q, n), true, &h);
     if (st) return st;
     st = rg_simulate(h, q, out, nullptr);
-    portfolio_free(reinterpret_cast<Portfolio *>(h), true); // rg_simulate has waited for its work
+    portfolio_free(reinterpret_cast<Portfolio *>(h)); // rg_simulate has waited for its work
     return st;
 }
 
@@ -1019,10 +1078,10 @@ static int plugin_portfolio(int n, const double *mu, const double *sigma, long l
             }
     }
     rg_portfolio *h = nullptr;
-    const int st = create_portfolio(n, mu, sigma, tda, nullptr, 0, parts, &h);
+    const int st = create_portfolio(n, mu, sigma, tda, nullptr, 0, parts, true, &h);
     if (st != RG_OK) return st;
     // every call that held it has waited for its own work
-    PortfolioRef ref(h, [](rg_portfolio *x) { portfolio_free(reinterpret_cast<Portfolio *>(x), true); });
+    PortfolioRef ref(h, [](rg_portfolio *x) { portfolio_free(reinterpret_cast<Portfolio *>(x)); });
     *out = ref;
     if (!use_cache) return RG_OK;
     std::lock_guard<std::mutex> lk(g_plugin_mu);
