@@ -219,9 +219,9 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     std::vector<unsigned char> host((size_t)count * tc_item_bytes());
     cudaError_t e = cudaGetDevice(&b->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, b->device);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_items, host.size());
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_counts, sizeof(unsigned long long) * 2 * (size_t)count);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_work, 2 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = device_alloc(&b->d_items, host.size());
+    if (e == cudaSuccess) e = device_alloc(&b->d_counts, sizeof(unsigned long long) * 2 * (size_t)count);
+    if (e == cudaSuccess) e = device_alloc(&b->d_work, 2 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_counts, sizeof(unsigned long long) * 2 * (size_t)count);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_err, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);

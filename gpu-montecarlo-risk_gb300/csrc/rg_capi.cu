@@ -134,16 +134,6 @@ static int get_ctx(DevCtx **out, int *dev_out)
     return RG_OK;
 }
 
-int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
-{
-    DevCtx *c = nullptr;
-    *err = cudaSuccess;
-    const int st = get_ctx(&c, nullptr);
-    if (st) return st;
-    *err = cudaMallocFromPoolAsync(p, bytes, c->pool, s);
-    return RG_OK;
-}
-
 // What the engine keeps on the current device but does not use goes back to
 // the driver.
 void pool_trim()
@@ -165,6 +155,37 @@ void pool_trim()
         }
 }
 
+// One more try, after pool_trim, for an allocation that failed for want of
+// memory: what the engine keeps for later calls does not fail this one.
+template <class F> static cudaError_t alloc_retry(F alloc)
+{
+    cudaError_t e = alloc();
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    pool_trim();
+    return alloc();
+}
+
+cudaError_t device_alloc(void **p, size_t bytes)
+{
+    return alloc_retry([&] { return cudaMalloc(p, bytes); });
+}
+
+static cudaError_t pool_take(DevCtx *c, void **p, size_t bytes, cudaStream_t s)
+{
+    return alloc_retry([&] { return cudaMallocFromPoolAsync(p, bytes, c->pool, s); });
+}
+
+int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
+{
+    DevCtx *c = nullptr;
+    *err = cudaSuccess;
+    const int st = get_ctx(&c, nullptr);
+    if (st) return st;
+    *err = pool_take(c, p, bytes, s);
+    return RG_OK;
+}
+
 static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
 {
     {
@@ -181,7 +202,7 @@ static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
     cudaError_t e = cudaEventCreate(&r->e0);
     if (e == cudaSuccess) e = cudaEventCreate(&r->e1);
     if (e == cudaSuccess) e = cudaMallocHost(&r->h, sizeof(QueryHead) + QueryRes::kCand * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&r->d, sizeof(QueryHead));
+    if (e == cudaSuccess) e = device_alloc(&r->d, sizeof(QueryHead));
     if (e == cudaSuccess) e = cudaMemsetAsync(r->d, 0, sizeof(QueryHead), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaThreadExchangeStreamCaptureMode(&mode);
@@ -303,13 +324,7 @@ static cudaError_t block_take(DevCtx *c, size_t bytes, void **p)
                 return cudaSuccess;
             }
     }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        pool_trim();
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
+    return device_alloc(p, bytes);
 }
 
 // A pooled portfolio (of one call, or of the plugin cache) goes back to the
@@ -654,7 +669,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
         p->block_bytes = bp.total;
-        if (pooled) RG_CUDA_TRY(cudaMallocFromPoolAsync(&p->d_block, bp.total, ctx->pool, s));
+        if (pooled) RG_CUDA_TRY(pool_take(ctx, &p->d_block, bp.total, s));
         else RG_CUDA_TRY(block_take(ctx, bp.total, &p->d_block));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
         p->d_L64 = reinterpret_cast<double *>(blk + oL64);
@@ -671,7 +686,7 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     if (!dev_in) {
         // Sigma and the weights share one upload buffer
         const size_t a_bytes = (nn * sizeof(double) + 255) & ~(size_t)255;
-        RG_CUDA_TRY(cudaMallocFromPoolAsync((void **)&dA, a_bytes + (weights ? (size_t)n * sizeof(double) : 0), ctx->pool, s));
+        RG_CUDA_TRY(pool_take(ctx, (void **)&dA, a_bytes + (weights ? (size_t)n * sizeof(double) : 0), s));
         if (ld == n)
             RG_CUDA_TRY(cudaMemcpyAsync(dA, sigma, nn * sizeof(double), cudaMemcpyHostToDevice, s));
         else
@@ -886,7 +901,7 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         cudaGetLastError(); // the query runs without the table
         d_table = nullptr;
     }
-    if (cap > QueryRes::kCand) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_cand, 4 * (size_t)cap, ctx->pool, s));
+    if (cap > QueryRes::kCand) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
     a = make_args(p, q, res.d->counts);
     a.err = &res.d->err;
     a.head = res.d;
@@ -916,7 +931,7 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         // mean -+ 12 sd, then a select pass on the bin that holds it (their
         // counts are discarded).
         hist.assign(kVarHistBins + 2, 0ull);
-        RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_hist, hist.size() * 8, ctx->pool, s));
+        RG_CUDA_TRY(pool_take(ctx, &d_hist, hist.size() * 8, s));
         a.var_mode = 2;
         a.sel_bins = kVarHistBins;
         a.sel_lo = (float)(mean - 12.0 * sd);
@@ -944,7 +959,7 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
             if (d_cand) RG_CUDA_TRY(cudaFreeAsync(d_cand, s));
             d_cand = nullptr;
             cap = need;
-            if (cap > QueryRes::kCand) RG_CUDA_TRY(cudaMallocFromPoolAsync(&d_cand, 4 * (size_t)cap, ctx->pool, s));
+            if (cap > QueryRes::kCand) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
             a.cand = d_cand ? static_cast<float *>(d_cand) : res.cand();
         }
         a.var_mode = 1;
@@ -1144,7 +1159,7 @@ int cuda_simulate(MonteCarloParams *params, MonteCarloResult *result)
                               parts_for_query(&q, n), &ref);
     h = ref.get();
     if (st == RG_OK && want_s) {
-        if (cudaMalloc(&d_s, (size_t)params->M * sizeof(int)) != cudaSuccess) {
+        if (device_alloc(&d_s, (size_t)params->M * sizeof(int)) != cudaSuccess) {
             st = set_error(RG_ERR_NOMEM, "cudaMalloc of S_values failed");
         }
         q.d_s_values = d_s;

@@ -379,5 +379,11 @@ int set_error(int status, const char *fmt, ...);
 // allocation's result, or the status of a device that could not be set up.
 int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err);
 void pool_trim();
+// cudaMalloc, tried once more after pool_trim.
+cudaError_t device_alloc(void **p, size_t bytes);
+template <class T> inline cudaError_t device_alloc(T **p, size_t bytes)
+{
+    return device_alloc(reinterpret_cast<void **>(p), bytes);
+}
 
 } // namespace rg

@@ -98,10 +98,10 @@ static int slot_init(Server *sv, Slot &sl)
     const int cap = sv->cfg.max_batch_items;
     const size_t ib = tc_item_bytes();
     cudaError_t e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&sl.d_items, ib * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&sl.d_dyn, 2 * sizeof(long long));
-    if (e == cudaSuccess) e = cudaMalloc(&sl.d_counts, 16 * (size_t)cap);
-    if (e == cudaSuccess) e = cudaMalloc(&sl.d_work, 2 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = device_alloc(&sl.d_items, ib * (size_t)cap);
+    if (e == cudaSuccess) e = device_alloc(&sl.d_dyn, 2 * sizeof(long long));
+    if (e == cudaSuccess) e = device_alloc(&sl.d_counts, 16 * (size_t)cap);
+    if (e == cudaSuccess) e = device_alloc(&sl.d_work, 2 * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMallocHost(&sl.h_items, ib * (size_t)cap);
     if (e == cudaSuccess) e = cudaMallocHost(&sl.h_dyn, 2 * sizeof(long long));
     if (e == cudaSuccess) e = cudaMallocHost(&sl.h_counts, 16 * (size_t)cap);

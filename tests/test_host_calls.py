@@ -112,3 +112,23 @@ def test_spare_portfolio_memory_is_bounded_and_given_back(fake, monkeypatch):
     fake.free_bytes(0, 1 << 40)
     _portfolio(20).close()
     assert [d for name, _, d in fake.log() if name == "cudaFree"] == [str(size)]
+
+
+def _run(**more):
+    return riskgpu.run(np.zeros(20), np.eye(20), np.full(20, 0.05), riskgpu.make_query(1000, 3, **more))
+
+
+@pytest.mark.parametrize("name,call", [
+    ("cudaMallocFromPoolAsync", _run),
+    ("cudaMallocFromPoolAsync", lambda: riskgpu.moments(np.ones((5, 3)))),
+    ("cudaMallocFromPoolAsync", lambda: riskgpu.crash_frequency(np.ones((5, 3)), 0.02, 1)),
+    ("cudaMalloc", lambda: _portfolio(LARGE).close()),
+    ("cudaMalloc", lambda: riskgpu.Batch([(_portfolio(20), riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))])),
+])
+def test_what_the_engine_keeps_does_not_fail_an_allocation(fake, name, call):
+    call()  # (process-wide state exists)
+    for skip in range(4):
+        fake.reset()
+        fake.fail(name, OOM, skip=skip, count=-1, until="cudaMemPoolTrimTo")
+        call()
+        assert skip or "cudaMemPoolTrimTo" in fake.names()
