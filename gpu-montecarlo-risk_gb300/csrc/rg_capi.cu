@@ -43,6 +43,10 @@ int set_error(int status, const char *fmt, ...)
 // pinned buffer that the kernels write the counters and the VaR candidates
 // to.  A 9-asset call has nothing but its kernel between two events in the
 // stream; clearing scratch before and copying it back after took 8 of 34 us.
+// At most kKeptQueries of these are made a device and kept between calls; with
+// more callers than that at once, a call takes stream-ordered memory only (h is
+// null, the counters are cleared and copied), since making and freeing pinned
+// memory waits for the whole device.
 struct QueryRes {
     static constexpr size_t kCand = 65536; // VaR candidates the pinned buffer holds
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -57,8 +61,8 @@ struct QueryRes {
 // driver gets back whatever it keeps beyond kPoolKeep bytes (pool_trim gives
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
-// alone: 228 us, of which about 190).  `idle` keeps the resources of a few
-// calls for the next ones.  A resident portfolio has a block from cudaMalloc,
+// alone: 228 us, of which about 190).  `idle`: those of the `kept` query
+// resources that no call is using.  A resident portfolio has a block from cudaMalloc,
 // since its d_L and d_packed are the caller's to map on a peer or to export to
 // another process, which a pool's memory does not allow.  `spare`: at most
 // kSpareBlocks such blocks, kSpareKeep bytes, of destroyed portfolios, for the
@@ -75,11 +79,12 @@ struct DevCtx {
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;
     std::vector<QueryRes> idle;
+    size_t kept = 0;
     std::vector<Block> spare, held;
 };
 
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
-static constexpr size_t kIdleQueries = 8;
+static constexpr size_t kKeptQueries = 8;
 static constexpr size_t kSpareBlocks = 8, kSpareKeep = 32u << 20;
 
 static std::mutex g_mu;
@@ -186,8 +191,28 @@ int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
     return RG_OK;
 }
 
-static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
+// The calling thread's allocations and frees are allowed beside a stream capture
+// of another thread, as the rest of a call is.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static void query_res_free(QueryRes &r, cudaStream_t s)
 {
+    RelaxedCapture relaxed;
+    if (r.e0) cudaEventDestroy(r.e0);
+    if (r.e1) cudaEventDestroy(r.e1);
+    if (r.d && r.h) cudaFree(r.d);
+    else if (r.d) cudaFreeAsync(r.d, s);
+    if (r.h) cudaFreeHost(r.h);
+    r = QueryRes();
+}
+
+static cudaError_t query_res_take(DevCtx *c, QueryRes *r, cudaStream_t s)
+{
+    bool keep;
     {
         std::lock_guard<std::mutex> lk(g_mu);
         if (!c->idle.empty()) {
@@ -195,35 +220,42 @@ static cudaError_t query_res_take(DevCtx *c, QueryRes *r)
             c->idle.pop_back();
             return cudaSuccess;
         }
+        keep = c->kept < kKeptQueries;
+        if (keep) c->kept++;
     }
-    // (allowed beside a stream capture of another thread, as the rest of a call is)
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    cudaError_t e = cudaEventCreate(&r->e0);
+    RelaxedCapture relaxed;
+    cudaError_t e = cudaSuccess;
+    if (keep && (cudaMallocHost(&r->h, sizeof(QueryHead) + QueryRes::kCand * sizeof(float)) != cudaSuccess ||
+                 device_alloc(&r->d, sizeof(QueryHead)) != cudaSuccess)) { // this call does without
+        cudaGetLastError();
+        if (r->h) cudaFreeHost(r->h);
+        r->h = nullptr;
+        r->d = nullptr;
+        keep = false;
+        std::lock_guard<std::mutex> lk(g_mu);
+        c->kept--;
+    }
+    if (!keep) e = pool_take(c, reinterpret_cast<void **>(&r->d), sizeof(QueryHead), s);
+    if (e == cudaSuccess) e = cudaEventCreate(&r->e0);
     if (e == cudaSuccess) e = cudaEventCreate(&r->e1);
-    if (e == cudaSuccess) e = cudaMallocHost(&r->h, sizeof(QueryHead) + QueryRes::kCand * sizeof(float));
-    if (e == cudaSuccess) e = device_alloc(&r->d, sizeof(QueryHead));
-    if (e == cudaSuccess) e = cudaMemsetAsync(r->d, 0, sizeof(QueryHead), c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) e = cudaMemsetAsync(r->d, 0, sizeof(QueryHead), keep ? c->stream : s);
+    if (e == cudaSuccess && keep) e = cudaStreamSynchronize(c->stream);
     return e;
 }
 
-// Back to the list (the call's work is complete and its kernels have reset
-// the counters: `clean`), or freed when it is full or the call failed.
-static void query_res_give(DevCtx *c, QueryRes &r, bool clean)
+// Kept resources go back to the list, clean (the call's work is complete and
+// its kernels have reset the counters), and are dropped where the call failed.
+static void query_res_give(DevCtx *c, QueryRes &r, cudaStream_t s, bool clean)
 {
-    if (clean) {
+    if (r.h) {
         std::lock_guard<std::mutex> lk(g_mu);
-        if (c->idle.size() < kIdleQueries) {
+        if (clean) {
             c->idle.push_back(r);
             return;
         }
+        c->kept--;
     }
-    if (r.e0) cudaEventDestroy(r.e0);
-    if (r.e1) cudaEventDestroy(r.e1);
-    if (r.h) cudaFreeHost(r.h);
-    if (r.d) cudaFree(r.d);
+    query_res_free(r, s);
 }
 
 #define RG_CUDA_TRY(call)                                                                          \
@@ -887,24 +919,28 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         cudaError_t e = cudaEventRecord(res.e0, s);
         if (e == cudaSuccess) e = launch_counting(p, q, a, ctx->sm_count, s);
         if (e == cudaSuccess) e = cudaEventRecord(res.e1, s);
+        if (e == cudaSuccess && !res.h) {
+            e = cudaMemcpyAsync(&head, res.d, sizeof(head), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaMemsetAsync(res.d, 0, sizeof(head), s);
+        }
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e == cudaSuccess) e = cudaEventElapsedTime(pass_ms, res.e0, res.e1);
-        if (e == cudaSuccess) memcpy(&head, res.h, sizeof(head));
+        if (e == cudaSuccess && res.h) memcpy(&head, res.h, sizeof(head));
         return e;
     };
     unsigned long long counts[2] = {0, 0};
     st = admit(64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2));
     if (st) return st;
-    RG_CUDA_TRY(query_res_take(ctx, &res));
+    RG_CUDA_TRY(query_res_take(ctx, &res, s));
     table = table_bytes(p, q);
     if (table && cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s) != cudaSuccess) {
         cudaGetLastError(); // the query runs without the table
         d_table = nullptr;
     }
-    if (cap > QueryRes::kCand) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
+    if (want_var && (!res.h || cap > QueryRes::kCand)) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
     a = make_args(p, q, res.d->counts);
     a.err = &res.d->err;
-    a.head = res.d;
+    a.head = res.h ? res.d : nullptr;
     a.host = res.h;
     a.blocks = static_cast<PhiloxBlock *>(d_table);
     if (want_var) {
@@ -959,7 +995,7 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
             if (d_cand) RG_CUDA_TRY(cudaFreeAsync(d_cand, s));
             d_cand = nullptr;
             cap = need;
-            if (cap > QueryRes::kCand) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
+            if (!res.h || cap > QueryRes::kCand) RG_CUDA_TRY(pool_take(ctx, &d_cand, 4 * (size_t)cap, s));
             a.cand = d_cand ? static_cast<float *>(d_cand) : res.cand();
         }
         a.var_mode = 1;
@@ -1010,14 +1046,14 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         out->var_passes = passes;
     }
     out->ms_device = ms;
-    query_res_give(ctx, res, true);
+    query_res_give(ctx, res, s, true);
     return RG_OK;
 fail:
     cudaStreamSynchronize(s);
     if (d_table) cudaFreeAsync(d_table, s);
     if (d_hist) cudaFreeAsync(d_hist, s);
     if (d_cand) cudaFreeAsync(d_cand, s);
-    query_res_give(ctx, res, false);
+    query_res_give(ctx, res, s, false);
     return st;
 }
 

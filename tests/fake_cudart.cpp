@@ -4,6 +4,8 @@
 // call succeeds unless a test says otherwise, and the calls whose order or
 // count matters are written to a log, one "name|stream|detail" a line.
 #include <cuda_runtime_api.h>
+#include <chrono>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -26,6 +28,9 @@ std::map<const void *, std::string> &kernels = *new std::map<const void *, std::
 std::map<void *, size_t> live;
 size_t live_bytes = 0, peak_bytes = 0;
 std::vector<size_t> free_list; // answers of cudaMemGetInfo in turn; the last one stays
+std::string gate; // calls of this name wait for each other ...
+int gate_left = 0; // ... until this many have come
+std::condition_variable gate_cv;
 size_t next_handle = 0x1000;
 cudaError_t last = cudaSuccess;
 thread_local struct {
@@ -51,7 +56,11 @@ cudaError_t call(const char *name, cudaStream_t s, const std::string &detail = "
 }
 cudaError_t simple(const char *name, cudaStream_t s = nullptr, const std::string &detail = "")
 {
-    std::lock_guard<std::mutex> lk(mu);
+    std::unique_lock<std::mutex> lk(mu);
+    if (gate_left > 0 && gate == name) {
+        if (--gate_left == 0) gate_cv.notify_all();
+        else gate_cv.wait_for(lk, std::chrono::seconds(10), [] { return gate_left <= 0; });
+    }
     return call(name, s, detail);
 }
 template <class T> cudaError_t handle(const char *name, T *out)
@@ -119,6 +128,13 @@ void fake_free_bytes(const size_t *v, int n)
 {
     std::lock_guard<std::mutex> lk(mu);
     free_list.assign(v, v + n);
+}
+// The next `count` calls of `name` return only once all of them have come.
+void fake_gather(const char *name, int count)
+{
+    std::lock_guard<std::mutex> lk(mu);
+    gate = name;
+    gate_left = count;
 }
 size_t fake_live_bytes() { return live_bytes; }
 size_t fake_peak_bytes() { return peak_bytes; }

@@ -53,6 +53,9 @@ class Fake:
     def fail(self, name, err, skip=0, count=1, until=None):
         self.lib.fake_fail(name.encode(), skip, count, err, until.encode() if until else None)
 
+    def gather(self, name, count):
+        self.lib.fake_gather(name.encode(), count)
+
     def free_bytes(self, *values):
         self.lib.fake_free_bytes((ctypes.c_size_t * len(values))(*values), len(values))
 

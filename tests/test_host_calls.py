@@ -2,6 +2,7 @@
 and the order of runtime calls where memory is short, a call is refused or many
 callers meet."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -132,3 +133,40 @@ def test_what_the_engine_keeps_does_not_fail_an_allocation(fake, name, call):
         fake.fail(name, OOM, skip=skip, count=-1, until="cudaMemPoolTrimTo")
         call()
         assert skip or "cudaMemPoolTrimTo" in fake.names()
+
+
+def test_many_callers_at_once_make_no_device_wide_calls(fake):
+    """Sixteen callers inside rg_simulate together, in waves: beyond the eight
+    kept resources a call uses stream-ordered memory only, and nothing is given
+    back in a way that waits for the device."""
+    port, results = _portfolio(20), []
+
+    def call():
+        results.append(port.simulate(riskgpu.make_query(1000, 3)))
+
+    for wave in range(3):
+        fake.reset()
+        fake.gather("cudaEventRecord", 16)
+        threads = [threading.Thread(target=call) for _ in range(16)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        names = fake.names()
+        made = 8 if wave == 0 else 0
+        assert names.count("cudaHostAlloc") == names.count("cudaMalloc") == made
+        assert not {"cudaFreeHost", "cudaFree", "cudaDeviceSynchronize"} & set(names)
+        assert names.count("cudaMallocFromPoolAsync") == names.count("cudaFreeAsync") == 8
+    assert len(results) == 48 and all(r["n_paths"] == 1000 for r in results)
+
+
+def test_a_query_needs_no_pinned_memory(fake):
+    port = _portfolio(20)
+    fake.fail("cudaHostAlloc", OOM, count=-1)
+    before = fake.live()
+    for _ in range(3):
+        assert port.simulate(riskgpu.make_query(1000, 3))["n_paths"] == 1000
+    assert fake.live() == before
+    fake.reset()
+    port.simulate(riskgpu.make_query(1000, 3))
+    assert "cudaHostAlloc" in fake.names() and "cudaFreeHost" not in fake.names()
