@@ -248,7 +248,7 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
     for (int i = 0; i < count; i++)
         blocks += table_len(reinterpret_cast<const Portfolio *>(items[i].portfolio), items[i].query);
     // the tables are left out beyond 256 MiB, or where there is no room
-    if (blocks > (256ull << 20) / sizeof(PhiloxBlock)) blocks = 0;
+    if (blocks > (256ull << 20) / sizeof(PhiloxBlock) || !admits(blocks * sizeof(PhiloxBlock))) blocks = 0;
     if (blocks && cudaMalloc(&b->d_blocks, blocks * sizeof(PhiloxBlock)) != cudaSuccess) {
         cudaGetLastError();
         b->d_blocks = nullptr;

@@ -278,27 +278,28 @@ static bool all_finite(const double *v, size_t n)
 // Free-memory admission: refuse an allocation of `need` bytes when it would
 // leave less than RG_MEM_HEADROOM_BYTES free.  RG_FAULT_INJECT=alloc makes
 // every engine allocation fail as if cudaMalloc had (host-side injection).
-static int admit(size_t need)
+static int admit(size_t need, bool quiet = false)
 {
+    auto refuse = [&](int st, const char *fmt, auto... args) { return quiet ? st : set_error(st, fmt, args...); };
     if (env_contains("RG_FAULT_INJECT", "alloc"))
-        return set_error(RG_ERR_NOMEM, "injected allocation failure (RG_FAULT_INJECT=alloc)");
+        return refuse(RG_ERR_NOMEM, "injected allocation failure (RG_FAULT_INJECT=alloc)");
     const char *h = getenv("RG_MEM_HEADROOM_BYTES");
     if (h && h[0]) {
         size_t headroom = (size_t)strtoull(h, nullptr, 10);
         size_t fr = 0, tot = 0;
         for (int tries = 0; tries < 2; tries++) {
-            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess)
-                return set_error(RG_ERR_CUDA, "cudaMemGetInfo failed");
+            if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return refuse(RG_ERR_CUDA, "cudaMemGetInfo failed");
             if (fr >= need && fr - need >= headroom) break;
             if (tries == 0) pool_trim(); // what the engine keeps for later calls does not refuse this one
         }
         if (fr < need || fr - need < headroom)
-            return set_error(RG_ERR_ADMISSION,
-                             "admission refused: %zu bytes requested, %zu free, headroom %zu", need,
-                             fr, headroom);
+            return refuse(RG_ERR_ADMISSION, "admission refused: %zu bytes requested, %zu free, headroom %zu", need, fr,
+                          headroom);
     }
     return RG_OK;
 }
+
+bool admits(size_t need) { return admit(need, true) == RG_OK; }
 
 // Waits for all work of the current device, also on streams of the caller's.
 // False where the wait is refused, as it is while a stream of the device is
@@ -844,7 +845,7 @@ int rg_launch_counts(const rg_portfolio *h, const rg_query *q, unsigned long lon
     // the block table lives for this launch, in stream order; a captured
     // launch allocates nothing and goes without
     const size_t table = table_bytes(p, q);
-    if (e == cudaSuccess && table) {
+    if (e == cudaSuccess && table && admits(table)) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
         else if (cap == cudaStreamCaptureStatusNone &&
@@ -929,11 +930,12 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         return e;
     };
     unsigned long long counts[2] = {0, 0};
-    st = admit(64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2));
+    const size_t scratch = 64 + (size_t)cap * 4 + 8 * (kVarHistBins + 2);
+    st = admit(scratch);
     if (st) return st;
     RG_CUDA_TRY(query_res_take(ctx, &res, s));
     table = table_bytes(p, q);
-    if (table && cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s) != cudaSuccess) {
+    if (table && admits(scratch + table) && cudaMallocFromPoolAsync(&d_table, table, ctx->pool, s) != cudaSuccess) {
         cudaGetLastError(); // the query runs without the table
         d_table = nullptr;
     }

@@ -379,6 +379,9 @@ int set_error(int status, const char *fmt, ...);
 // allocation's result, or the status of a device that could not be set up.
 int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err);
 void pool_trim();
+// Whether the free-memory admission check would let `need` bytes through (for
+// memory that a call can do without).
+bool admits(size_t need);
 // cudaMalloc, tried once more after pool_trim.
 cudaError_t device_alloc(void **p, size_t bytes);
 template <class T> inline cudaError_t device_alloc(T **p, size_t bytes)

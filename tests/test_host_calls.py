@@ -170,3 +170,32 @@ def test_a_query_needs_no_pinned_memory(fake):
     fake.reset()
     port.simulate(riskgpu.make_query(1000, 3))
     assert "cudaHostAlloc" in fake.names() and "cudaFreeHost" not in fake.names()
+
+
+def test_block_tables_ask_for_admission(fake, monkeypatch):
+    """A table is memory that a query can do without: where the check would
+    refuse it the call runs without one, and is not refused."""
+    port = _portfolio(640)
+    query = riskgpu.make_query(1_000_000, 3, horizon=20, precision=riskgpu.PREC_BF16X3)
+    table = 640 // 4 * 20 * 16
+
+    def pooled(call):
+        fake.reset()
+        call()
+        return [int(d) for name, _, d in fake.log() if name in ("cudaMallocFromPoolAsync", "cudaMalloc")]
+
+    counts = np.zeros(2, dtype=np.uint64)
+    calls = [lambda: port.simulate(query), lambda: port.launch_counts(query, counts.ctypes.data),
+             lambda: riskgpu.Batch([(port, query)]).close()]
+    for call in calls:
+        assert table in pooled(call)
+    monkeypatch.setenv("RG_MEM_HEADROOM_BYTES", str(1 << 30))
+    for call in calls:
+        assert table in pooled(call)
+    for call in calls:  # room for the rest of the call's memory, not for the table
+        fake.reset()
+        free = (1 << 30) + table - 1
+        fake.free_bytes(free)
+        call()
+        assert table not in [int(d) for name, _, d in fake.log()
+                             if name in ("cudaMallocFromPoolAsync", "cudaMalloc")]
