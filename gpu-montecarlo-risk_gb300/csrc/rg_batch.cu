@@ -67,13 +67,16 @@ static std::string tune_path()
     return (e && e[0]) ? std::string(e) : std::string("riskgpu_tune.json");
 }
 
+// The class of a batch: the two forms of the kernel are tuned apart (the merged
+// form's key has no suffix: files written before the split form took batches
+// hold the merged form's choices).
 static std::string tune_key(const Batch *b)
 {
     long long t = 1;
     while (t < b->total_tiles) t <<= 1;
     char k[96];
     snprintf(k, sizeof k, "tc_batch:nkt=%d:nmt=%d:tiles=%lld:sms=%d", b->n_kt_max, b->n_mt_max, t, b->sm_count);
-    return std::string(k);
+    return std::string(k) + (b->split ? ":split" : "");
 }
 
 // The cache is a flat JSON object {"key": [unit_tiles, ctas_per_sm, ms], ...}.
