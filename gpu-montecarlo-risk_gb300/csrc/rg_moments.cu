@@ -94,9 +94,11 @@ __global__ void center_kernel(double *__restrict__ X, long long T, int n, const 
 }
 
 // Tile blockIdx.x of the lower triangle, rows [seg per, (seg + 1) per) of the
-// centred matrix: part[seg][tile][32 x 32].
+// centred matrix: part[seg][tile][32 x 32], or, with one segment, Sigma itself
+// (the partials of many columns would be half of Sigma once more: N > 1536).
 __global__ void __launch_bounds__(256) cov_tile_kernel(const double *__restrict__ X, long long T, int n,
-                                                       long long per, double *__restrict__ part)
+                                                       long long per, double *__restrict__ part,
+                                                       double *__restrict__ S)
 {
     __shared__ double A[kMomTile][kMomTile + 1], B[kMomTile][kMomTile + 1];
     const int t = blockIdx.x;
@@ -124,6 +126,18 @@ __global__ void __launch_bounds__(256) cov_tile_kernel(const double *__restrict_
             for (int u = 0; u < 4; u++) acc[u] = fma(a, B[tt][cb + u], acc[u]);
         }
         __syncthreads();
+    }
+    if (gridDim.y == 1) {
+        const double inv = 1.0 / (double)(T - 1);
+#pragma unroll
+        for (int u = 0; u < 4; u++) A[r][cb + u] = (0.0 + acc[u]) * inv; // as cov_sum_kernel adds one segment
+        __syncthreads();
+        for (int e = threadIdx.x; e < kMomTile * kMomTile; e += blockDim.x) {
+            const int x = e / kMomTile, y = e % kMomTile;
+            if (i0 + x < n && j0 + y < n) S[(long long)(i0 + x) * n + j0 + y] = A[x][y];
+            if (bi != bj && i0 + y < n && j0 + x < n) S[(long long)(j0 + x) * n + i0 + y] = A[y][x];
+        }
+        return;
     }
     double *out = part + ((size_t)blockIdx.y * gridDim.x + t) * (kMomTile * kMomTile) + r * kMomTile + cb;
 #pragma unroll
@@ -240,7 +254,8 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
     segs = (T + per - 1) / per;
     // one allocation: X, mu, Sigma, column partials, tile partials, flag
     const size_t oX = 0, omu = oX + (size_t)T * n, oS = omu + (size_t)n, ocol = oS + (size_t)n * n,
-                 ocov = ocol + 2 * (size_t)kMomSegs * n, obad = ocov + (size_t)segs * tiles * kMomTile * kMomTile;
+                 ocov = ocol + 2 * (size_t)kMomSegs * n,
+                 obad = ocov + (segs > 1 ? (size_t)segs * tiles * kMomTile * kMomTile : 0);
     double *d = nullptr;
     unsigned long long bad = kAllFinite;
     cudaError_t e = cudaSuccess;
@@ -254,8 +269,8 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
             col_mean_kernel<<<(n + 7) / 8, 256, 0, s>>>(d + ocol, T, n, d + omu);
             const int gy = (int)(T < 256 ? T : 256);
             center_kernel<<<dim3((n + 127) / 128, gy), 128, 0, s>>>(d + oX, T, n, d + omu);
-            cov_tile_kernel<<<dim3(tiles, (unsigned)segs), 256, 0, s>>>(d + oX, T, n, per, d + ocov);
-            cov_sum_kernel<<<tiles, 256, 0, s>>>(d + ocov, (int)segs, T, n, d + oS);
+            cov_tile_kernel<<<dim3(tiles, (unsigned)segs), 256, 0, s>>>(d + oX, T, n, per, d + ocov, d + oS);
+            if (segs > 1) cov_sum_kernel<<<tiles, 256, 0, s>>>(d + ocov, (int)segs, T, n, d + oS);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, dbad, sizeof(bad), cudaMemcpyDeviceToHost, s);
