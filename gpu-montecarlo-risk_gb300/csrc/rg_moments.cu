@@ -282,6 +282,7 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }
     }
+    if (e != cudaSuccess) cudaStreamSynchronize(s); // no copy to or from the caller's memory stays in flight
     if (d) cudaFreeAsync(d, s);
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_moments: %s",
@@ -317,6 +318,7 @@ extern "C" int rg_crash_frequency(const double *returns, int64_t T, int32_t n, i
         if (e == cudaSuccess) e = cudaMemcpyAsync(got, dgot, sizeof(got), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
+    if (e != cudaSuccess) cudaStreamSynchronize(s); // no copy to or from the caller's memory stays in flight
     if (d) cudaFreeAsync(d, s);
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_crash_frequency: %s",

@@ -17,3 +17,22 @@ def test_memory_of_the_moments(fake, days, n):
     tiles = (n + 31) // 32 * ((n + 31) // 32 + 1) // 2
     partials = 0 if tiles >= 8 * 152 or days < 128 else (8 * 152 + tiles) * 32 * 32
     assert fake.peak() <= 8 * (days * n + n * n + 65 * n + partials + 1)
+
+
+CALLS = [lambda X: riskgpu.moments(X), lambda X: riskgpu.crash_frequency(X, 0.02, 1)]
+
+
+@pytest.mark.parametrize("call", CALLS)
+@pytest.mark.parametrize("name,skip", [("launch", 0), ("cudaMemcpyAsync", 1), ("cudaMemcpyAsync", 2),
+                                       ("cudaMemcpyAsync", 3)])
+def test_no_copy_in_flight_when_a_failed_call_returns(fake, call, name, skip):
+    """The caller may free or reuse its arrays: the copies issued are waited for."""
+    fake.reset()
+    fake.fail(name, 700, skip=skip)
+    try:
+        call(np.zeros((40, 3)))
+    except riskgpu.RiskGpuError as e:
+        assert e.status == riskgpu.RG_ERR_CUDA
+    names = fake.names()
+    last_copy = max(i for i, n in enumerate(names) if n == "cudaMemcpyAsync")
+    assert "cudaStreamSynchronize" in names[last_copy:]
