@@ -654,8 +654,8 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
     if (ld < n) return set_error(RG_ERR_INVALID, "leading dimension %lld < N", (long long)ld);
     const bool dev_in = (flags & RG_INPUT_DEVICE) != 0;
     // The factorisation finds entries that are not finite; the host looks at
-    // its arrays only to name the first one, or when no kernel will run (the
-    // scan took 0.1 ms of a call at N = 600).
+    // its arrays only to name the first one, or when the kernels do not run
+    // (the scan took 0.1 ms of a call at N = 600).
     auto finite_inputs = [&]() -> int {
         if (dev_in) return RG_OK;
         if (!all_finite(mu, (size_t)n)) return set_error(RG_ERR_INVALID, "mu has a NaN or Inf");
@@ -797,6 +797,8 @@ fail:
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     portfolio_free(p);
+    // bad input is reported as such also where no kernel could look at it
+    if ((st == RG_ERR_NOMEM || st == RG_ERR_CUDA) && finite_inputs()) st = RG_ERR_INVALID;
     return st;
 }
 

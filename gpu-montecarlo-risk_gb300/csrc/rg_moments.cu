@@ -212,18 +212,24 @@ int check_matrix(const double *X, int64_t T, int32_t n, int64_t ld, int64_t min_
     return RG_OK;
 }
 
-// Without a device the entries are checked here, so that bad input is
-// reported as such on any machine; with one the kernels look for the first
-// that is not finite.
+// The kernels look for the first entry that is not finite.  Where they do not
+// run (no device, no memory, a call that failed) the entries are checked here,
+// so that bad input is reported as such before anything else.
+int check_entries(const double *X, int64_t T, int32_t n, int64_t ld)
+{
+    for (int64_t t = 0; t < T; t++)
+        for (int32_t j = 0; j < n; j++)
+            if (!std::isfinite(X[t * ld + j])) return not_finite(t, j);
+    return RG_OK;
+}
+
 int device_ready(const double *X, int64_t T, int32_t n, int64_t ld)
 {
     int count = 0;
     if (cudaGetDeviceCount(&count) == cudaSuccess && count > 0) return RG_OK;
     cudaGetLastError();
-    for (int64_t t = 0; t < T; t++)
-        for (int32_t j = 0; j < n; j++)
-            if (!std::isfinite(X[t * ld + j])) return not_finite(t, j);
-    return set_error(RG_ERR_NO_DEVICE, "no CUDA device is available");
+    const int st = check_entries(X, T, n, ld);
+    return st ? st : set_error(RG_ERR_NO_DEVICE, "no CUDA device is available");
 }
 
 // Rows packed to width n on the device.
@@ -259,7 +265,8 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
     double *d = nullptr;
     unsigned long long bad = kAllFinite;
     cudaError_t e = cudaSuccess;
-    if ((st = pool_alloc((void **)&d, (obad + 1) * sizeof(double), s, &e)) != RG_OK) return st;
+    if ((st = pool_alloc((void **)&d, (obad + 1) * sizeof(double), s, &e)) != RG_OK)
+        return check_entries(returns, T, n, ld) ? RG_ERR_INVALID : st;
     if (e == cudaSuccess) {
         unsigned long long *dbad = reinterpret_cast<unsigned long long *>(d + obad);
         e = cudaMemsetAsync(dbad, 0xff, sizeof(*dbad), s);
@@ -284,6 +291,7 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
     }
     if (e != cudaSuccess) cudaStreamSynchronize(s); // no copy to or from the caller's memory stays in flight
     if (d) cudaFreeAsync(d, s);
+    if (e != cudaSuccess && (st = check_entries(returns, T, n, ld)) != RG_OK) return st;
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_moments: %s",
                          cudaGetErrorString(e));
@@ -304,7 +312,8 @@ extern "C" int rg_crash_frequency(const double *returns, int64_t T, int32_t n, i
     unsigned char *d = nullptr;
     unsigned long long got[2] = {0, kAllFinite}; // crash days, first entry that is not finite
     cudaError_t e = cudaSuccess;
-    if ((st = pool_alloc((void **)&d, xbytes + sizeof(got), s, &e)) != RG_OK) return st;
+    if ((st = pool_alloc((void **)&d, xbytes + sizeof(got), s, &e)) != RG_OK)
+        return check_entries(returns, T, n, ld) ? RG_ERR_INVALID : st;
     if (e == cudaSuccess) {
         unsigned long long *dgot = reinterpret_cast<unsigned long long *>(d + xbytes);
         e = cudaMemsetAsync(dgot, 0, sizeof(got[0]), s);
@@ -320,6 +329,7 @@ extern "C" int rg_crash_frequency(const double *returns, int64_t T, int32_t n, i
     }
     if (e != cudaSuccess) cudaStreamSynchronize(s); // no copy to or from the caller's memory stays in flight
     if (d) cudaFreeAsync(d, s);
+    if (e != cudaSuccess && (st = check_entries(returns, T, n, ld)) != RG_OK) return st;
     if (e != cudaSuccess)
         return set_error(e == cudaErrorMemoryAllocation ? RG_ERR_NOMEM : RG_ERR_CUDA, "rg_crash_frequency: %s",
                          cudaGetErrorString(e));

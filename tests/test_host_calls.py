@@ -199,3 +199,13 @@ def test_block_tables_ask_for_admission(fake, monkeypatch):
         call()
         assert table not in [int(d) for name, _, d in fake.log()
                              if name in ("cudaMallocFromPoolAsync", "cudaMalloc")]
+
+
+@pytest.mark.parametrize("name,err,status", [("cudaMalloc", OOM, riskgpu.RG_ERR_NOMEM),
+                                             ("cudaMallocFromPoolAsync", OOM, riskgpu.RG_ERR_NOMEM),
+                                             ("launch", 700, riskgpu.RG_ERR_CUDA)])
+def test_bad_input_is_reported_before_a_failed_creation(fake, name, err, status):
+    for bad in (None, 3):
+        fake.fail(name, err, count=-1)
+        assert _create(bad=bad)[:2] == (status if bad is None else riskgpu.RG_ERR_INVALID, None)
+        assert ("row 3" in riskgpu.lib().rg_last_error().decode()) == (bad is not None)

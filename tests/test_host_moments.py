@@ -36,3 +36,19 @@ def test_no_copy_in_flight_when_a_failed_call_returns(fake, call, name, skip):
     names = fake.names()
     last_copy = max(i for i, n in enumerate(names) if n == "cudaMemcpyAsync")
     assert "cudaStreamSynchronize" in names[last_copy:]
+
+
+@pytest.mark.parametrize("call", CALLS)
+@pytest.mark.parametrize("name,err,status", [("cudaGetDeviceCount", 100, riskgpu.RG_ERR_NO_DEVICE),
+                                             ("cudaMallocFromPoolAsync", OOM, riskgpu.RG_ERR_NOMEM),
+                                             ("launch", 700, riskgpu.RG_ERR_CUDA)])
+def test_bad_input_is_reported_before_a_failed_call(fake, call, name, err, status):
+    X = np.zeros((40, 3))
+    for bad in (False, True):
+        if bad:
+            X[17, 2] = np.inf
+        fake.fail(name, err, count=-1)
+        with pytest.raises(riskgpu.RiskGpuError) as e:
+            call(X)
+        assert e.value.status == (riskgpu.RG_ERR_INVALID if bad else status)
+        assert ("returns[17][2]" in str(e.value)) == bad
