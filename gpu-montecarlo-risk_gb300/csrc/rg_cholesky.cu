@@ -38,9 +38,10 @@
 // lane in the panel, 32 x 32 update tiles) and now:
 //   N        9    20    50    64    65   200   333   600   1000   2000
 //   before  34    65   178   249   188   538   924  1578   2810   7246
-//   now     10    18    47    55    66   180   297   528    966   3352
-// Both forms cross at N = 64, the widest block whose columns stay in
-// registers (55 us against about 64 us blocked).
+//   now     12    18    51    59    58   158   260   466    908   3289
+// N = 64 is the widest block whose columns stay in registers.  The blocked form
+// takes 16, 20, 44 and 50 us at N = 9, 20, 50 and 64, but subtracts the products
+// one by one: its error there is larger than that of the form before (FINE).
 // RG_CHOLESKY=single forces cholesky_kernel, one CTA left-looking column by
 // column in place in the row-major output, above N = 64 too (a second
 // implementation that the tests compare).
@@ -52,6 +53,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include "rg_internal.cuh"
 
 namespace rg {
@@ -203,11 +205,17 @@ __device__ __forceinline__ bool finite_bits(double v)
 // y0 (1 + e/2 + 3/8 e^2) to 5/16 e^3 < 2^-61.
 // Largest error over 2e7 arguments, on the CPU with the approximation off by
 // up to 3 ulp: 0.507 ulp (the FP64 form: 0.996).
-__device__ __forceinline__ double pivot_rsqrt(double d)
+// `low`, where wanted: what the rounding to 53 bits left out, so that
+// fma(v, result, v * low) is v / sqrt(d) rounded about once.
+__device__ __forceinline__ double pivot_rsqrt(double d, double *low = nullptr)
 {
     const uint64_t b = (uint64_t)__double_as_longlong(d);
     const int be = (int)(b >> 52); // biased exponent
-    if (be < 64 || be > 1983) return rsqrt(d);
+    if (be < 64 || be > 1983) {
+        const double rs = rsqrt(d), y = d * rs;
+        if (low) *low = 0.5 * rs * fma(-fma(d, rs, -y), rs, fma(-y, rs, 1.0));
+        return rs;
+    }
     const int ex = be - 1023, odd = ex & 1, k = ex >> 1;
     float y0;
     asm("rsqrt.approx.ftz.f32 %0, %1;" // x cut to 24 bits
@@ -220,7 +228,13 @@ __device__ __forceinline__ double pivot_rsqrt(double d)
     const int64_t c = e + ((3 * (int)(((int64_t)es * es) >> 32)) >> 7);                // (e/2 + 3/8 e^2) 2^62
     const int64_t r = ((int64_t)y << 40) + (((int64_t)y * (c >> 2)) >> 20);            // 2^62 / sqrt(x)
     // 53 bits, rounded; a carry out of them raises the exponent
-    return __longlong_as_double((long long)(((uint64_t)(1021 - k) << 52) + ((uint64_t)(r + 256) >> 9)));
+    const uint64_t h = (uint64_t)(r + 256) >> 9;
+    if (low) {
+        const int l = (int)(r - (int64_t)(h << 9)); // times 2^(-62 - k)
+        const uint64_t lb = (uint64_t)__double_as_longlong((double)l);
+        *low = __longlong_as_double(l ? (long long)(lb - ((uint64_t)(62 + k) << 52)) : 0ll);
+    }
+    return __longlong_as_double((long long)(((uint64_t)(1021 - k) << 52) + h));
 }
 
 // The warps that factor a block: the chain warp (0) and six bulk warps (1-3,
@@ -278,17 +292,30 @@ __device__ __forceinline__ bool chol_wait(unsigned long long *bar)
 // had every column before c - 2 applied, applies columns c - 2 and c - 1, forms
 // the pivot and leaves column c final: two FMAs, the reciprocal square root and
 // one multiply a column.  (With column c - 2 left to the bulk warps too, the
-// chain waited for them 280 of 1220 cycles a column of a 32-column block; now
-// 140 of 930, and the bulk warps are busy 0.8 of the time.)  The bulk warps
+// chain waited for them 280 of 1220 cycles a column of a 32-column block
+// instead of 140 of 930.)  The bulk warps
 // (column j in the registers of bulk warp j mod 6, lane = row, two rows a lane
 // for NC > 32) apply each final column c to theirs; the one that owns column
 // c + 3 does that one first, writes it
 // back for the chain warp and catches up with its other columns later
 // (`done`: columns applied so far).  Hand-over by column instead of a CTA
 // barrier a column lets a bulk warp fall behind while the chain goes on.
-template <int NC>
+//
+// FINE (N <= 64) keeps the error of the form before, the left-looking one with
+// sums of their own, a square root and divisions: the quotients are rounded
+// about once (pivot_rsqrt's low part), and the bulk warps sum a column's products
+// from zero in four parts and subtract them from it once.
+// Root-mean-square error of L against extended precision, in 2^-52 of L, over 12
+// factor covariances a size (the form before; with products subtracted one by
+// one and rounded reciprocals; now): N = 9 0.28, 0.37, 0.28; N = 20 0.41, 0.53,
+// 0.43; N = 50 0.90, 0.91, 0.70; N = 64 1.12, 1.07, 0.92.  Device time, without
+// FINE and with it, us: 10.4 and 11.7, 18.0 and 17.9, 47.1 and 50.6, 56.8 and
+// 58.9.  Above 64 the two forms' errors are alike (N = 100 2.02 and 2.07, N = 200
+// 3.68 and 3.67).
+template <int NC, bool FINE>
 __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv, CholFlags &f, int *s_fail)
 {
+    constexpr int STEP = 2;
     constexpr int SL = (NC + kCholBulk - 1) / kCholBulk, G = (NC + 31) / 32, NR = 32 * G;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *failed = s_fail;
@@ -296,95 +323,130 @@ __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv,
         double p[G], q[G]; // the previous column and the one before it
 #pragma unroll
         for (int g = 0; g < G; g++) p[g] = q[g] = 0.0;
-        int c = 0;
-        for (; c < n; c++) {
+        // column c in the 32-row groups from `first` on (rows above the column's
+        // own group hold nothing); false: given up
+        auto column = [&](int c, auto first) -> bool {
+            constexpr int g0 = decltype(first)::value;
             const double lp = -__shfl_sync(0xffffffffu, c >= 32 ? p[G - 1] : p[0], c & 31);
             const double lq = -__shfl_sync(0xffffffffu, c >= 32 ? q[G - 1] : q[0], c & 31);
             if (c >= 3 && !chol_wait(&f.pre[c])) {
                 if (lane == 0) *failed = -1;
-                break;
+                return false;
             }
             double v[G];
 #pragma unroll
-            for (int g = 0; g < G; g++) {
+            for (int g = g0; g < G; g++) {
                 v[g] = fma(p[g], lp, fma(q[g], lq, col[c * NR + 32 * g + lane]));
                 q[g] = p[g];
             }
-            const double d = __shfl_sync(0xffffffffu, c >= 32 ? v[G - 1] : v[0], c & 31);
+            const double d = __shfl_sync(0xffffffffu, v[g0], c & 31);
             if (!good_pivot(d)) { // the same value in every lane
                 if (lane == 0) *failed = c + 1;
-                break;
+                return false;
             }
-            const double rs = pivot_rsqrt(d);
+            double low = 0.0;
+            const double rs = pivot_rsqrt(d, FINE ? &low : nullptr);
 #pragma unroll
-            for (int g = 0; g < G; g++) {
-                p[g] = 32 * g + lane >= c ? v[g] * rs : 0.0; // on the diagonal d / sqrt(d)
+            for (int g = g0; g < G; g++) {
+                const double x = FINE ? fma(v[g], rs, v[g] * low) : v[g] * rs;
+                p[g] = 32 * g + lane >= c ? x : 0.0; // on the diagonal d / sqrt(d)
                 col[c * NR + 32 * g + lane] = p[g];
             }
             if (lane == 0) inv[c] = rs;
             chol_arrive(&f.fin[c]);
-        }
+            return true;
+        };
+        int c = 0;
+        bool ok = true;
+        for (; ok && c < n && c < 32; c += ok) ok = column(c, std::integral_constant<int, 0>());
+        for (; ok && c < n; c += ok) ok = column(c, std::integral_constant<int, G - 1>());
         // after a failure: release the bulk warps from the columns not
         // published (each flag is arrived on once)
         for (; c < n; c++) chol_arrive(&f.fin[c]);
         return;
     }
     const int b = warp < 4 ? warp - 1 : warp - 2; // bulk index
-    double a[SL][G];
+    // FINE: four sums of the columns' products, column k's in sum k mod 4;
+    // else one, the column so far.  (Arrays of their own: chosen from by an
+    // index known only at run time, one array would move to local memory.)
+    double a[SL][G], a1[SL][G], a2[SL][G], a3[SL][G];
 #pragma unroll
     for (int s = 0; s < SL; s++)
 #pragma unroll
         for (int g = 0; g < G; g++) {
             const int j = s * kCholBulk + b;
-            a[s][g] = j < n ? col[j * NR + 32 * g + lane] : 0.0;
+            a[s][g] = !FINE && j < n ? col[j * NR + 32 * g + lane] : 0.0;
+            a1[s][g] = a2[s][g] = a3[s][g] = 0.0;
         }
-    int done = 0;
-    // Unrolled over the slots so that finished columns cost nothing: an FP64
-    // instruction whose predicate is false still takes its 64 cycles.
+    // acc += (FINE) or -= column k's products, for the slots from s0 on
+    auto apply = [&](int k, int s0, double (&acc)[SL][G]) {
+        const double *ck = col + k * NR;
+        double lr[G];
 #pragma unroll
-    for (int s0 = 0; s0 < SL; s0++) {
-        for (int c = s0 * kCholBulk; c < (s0 + 1) * kCholBulk && c + 3 < n; c++) {
+        for (int g = 0; g < G; g++) lr[g] = ck[32 * g + lane];
+#pragma unroll
+        for (int s = 0; s < SL; s++) {
+            if (s < s0) continue;
+            const int j = s * kCholBulk + b;
+            const double l = FINE ? ck[j < NR ? j : 0] : -ck[j < NR ? j : 0];
+            // rows above the column's own 32-row group hold nothing
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                if (g >= s * kCholBulk / 32) acc[s][g] = fma(lr[g], l, acc[s][g]);
+        }
+    };
+    int done = 0;
+    // Unrolled over the slots, two a step, so that finished columns cost little:
+    // an FP64 instruction whose predicate is false still takes its 64 cycles.
+    // One slot a step is more code to fetch (N = 600 478 us instead of 472), three
+    // cost more finished columns (N = 50 52.7 instead of 50.7).
+#pragma unroll
+    for (int s0 = 0; s0 < SL; s0 += STEP) {
+        for (int c = s0 * kCholBulk; c < (s0 + STEP) * kCholBulk && c + 3 < n; c++) {
             if (!chol_wait(&f.fin[c])) {
                 if (lane == 0) *failed = -1;
                 return;
             }
             if (*failed != 0) return;
             if (b == (c + 3) % kCholBulk) {
-                // the owned column by masks: an index known only at run time
-                // would move the array to local memory
-                double v[G];
+                // the owned column by masks, as above; its groups from g0 on
+                const int g0 = (s0 * kCholBulk + 3) / 32;
+                auto owned = [&](const double (&acc)[SL][G], double (&v)[G]) {
 #pragma unroll
-                for (int g = 0; g < G; g++) {
-                    long long bits = 0;
+                    for (int g = g0; g < G; g++) {
+                        long long bits = 0;
 #pragma unroll
-                    for (int s = s0; s < SL; s++)
-                        bits |= __double_as_longlong(a[s][g]) & -(long long)(s == (c + 3) / kCholBulk);
-                    v[g] = __longlong_as_double(bits);
+                        for (int s = s0; s < SL && s <= s0 + STEP; s++)
+                            bits |= __double_as_longlong(acc[s][g]) & -(long long)(s == (c + 3) / kCholBulk);
+                        v[g] = __longlong_as_double(bits);
+                    }
+                };
+                double v[G], v1[G], v2[G], v3[G];
+                owned(a, v);
+                if (FINE) {
+                    owned(a1, v1);
+                    owned(a2, v2);
+                    owned(a3, v3);
                 }
-                for (int k = done; k <= c; k++) {
-                    const double l = -col[k * NR + c + 3];
+                // (the columns before c have been applied: a warp's own columns
+                // are kCholBulk apart; as a loop over the columns left to do
+                // this one step took N = 600 from 472 to 544 us)
+                const double l = FINE ? col[c * NR + c + 3] : -col[c * NR + c + 3];
 #pragma unroll
-                    for (int g = 0; g < G; g++) v[g] = fma(col[k * NR + 32 * g + lane], l, v[g]);
+                for (int g = g0; g < G; g++) v[g] = fma(col[c * NR + 32 * g + lane], l, v[g]);
+#pragma unroll
+                for (int g = g0; g < G; g++) {
+                    double *x = col + (c + 3) * NR + 32 * g + lane;
+                    *x = FINE ? *x - ((v[g] + v1[g]) + (v2[g] + v3[g])) : v[g];
                 }
-#pragma unroll
-                for (int g = 0; g < G; g++) col[(c + 3) * NR + 32 * g + lane] = v[g];
                 chol_arrive(&f.pre[c + 3]);
                 continue;
             }
             for (int k = done; k <= c; k++) {
-                const double *ck = col + k * NR;
-                double lr[G];
-#pragma unroll
-                for (int g = 0; g < G; g++) lr[g] = ck[32 * g + lane];
-#pragma unroll
-                for (int s = s0; s < SL; s++) {
-                    const int j = s * kCholBulk + b;
-                    const double l = -ck[j < NR ? j : 0];
-                    // rows above the column's own 32-row group hold nothing
-#pragma unroll
-                    for (int g = 0; g < G; g++)
-                        if (g >= s * kCholBulk / 32) a[s][g] = fma(lr[g], l, a[s][g]);
-                }
+                if (!FINE || (k & 3) == 0) apply(k, s0, a);
+                else if ((k & 3) == 1) apply(k, s0, a1);
+                else if ((k & 3) == 2) apply(k, s0, a2);
+                else apply(k, s0, a3);
             }
             done = c + 1;
         }
@@ -425,7 +487,7 @@ __global__ void __launch_bounds__(kCholCta, 1) chol_small_kernel(
         if (tid == 0) *info = -1;
         return;
     }
-    if (chol_takes_part()) chol_factor_cta<NC>(n, col, inv, flags, &s_fail);
+    if (chol_takes_part()) chol_factor_cta<NC, true>(n, col, inv, flags, &s_fail);
     __syncthreads();
     if (tid == 0) *info = s_fail < 0 ? kCholTimeout : s_fail;
     if (s_fail) return;
@@ -580,7 +642,7 @@ __global__ void __launch_bounds__(kCholCta, 1) chol_step_kernel(double *L, int n
         col[m * kCholNb + r] = (r < nb && m <= r) ? L[(long long)(r0 + r) * n + r0 + m] : 0.0;
     }
     __syncthreads();
-    if (chol_takes_part()) chol_factor_cta<kCholNb>(nb, col, inv, flags, &s_fail);
+    if (chol_takes_part()) chol_factor_cta<kCholNb, false>(nb, col, inv, flags, &s_fail);
     __syncthreads();
     if (s_fail) {
         if (tid == 0) *info = s_fail < 0 ? kCholTimeout : r0 + s_fail;
