@@ -788,7 +788,7 @@ static cudaError_t launch_cholesky_blocked(const double *A, long long lda, int n
         // While the factoring CTA is the longest, it keeps its SM's FP64 pipe
         // to itself (shared memory for one CTA an SM); with more than about
         // six tiles an SM the trailing update is, and packs the SMs.
-        const size_t alone = tiles <= 6 * 152 ? kCholAlone : 0;
+        const size_t alone = tiles <= 6 * kSms ? kCholAlone : 0;
         e = launch_pdl(chol_step_kernel, 1 + tiles, kCholCta, alone, s, L64, n, k0, kb, dinv, info);
         k0 = r0;
         kb = n - r0 < kCholNb ? n - r0 : kCholNb;

@@ -202,6 +202,10 @@ __host__ __device__ constexpr int packed_row_offset(int i)
 }
 __host__ __device__ constexpr int packed_len(int n) { return packed_row_offset(n); }
 
+// SMs of a GB300, for splits of work whose order of sums must not depend on the
+// device that runs them (launch grids take the device's own count).
+static constexpr int kSms = 152;
+
 // ---------------------------------------------------------------- host
 struct Portfolio {
     int n = 0;

@@ -252,7 +252,7 @@ extern "C" int rg_moments(const double *returns, int64_t T, int32_t n, int64_t l
     cudaStream_t s = (cudaStream_t)stream;
     const int nb = (n + kMomTile - 1) / kMomTile, tiles = nb * (nb + 1) / 2;
     // about eight CTAs an SM, at least 64 rows each
-    int64_t segs = (8 * 152 + tiles - 1) / tiles;
+    int64_t segs = (8 * kSms + tiles - 1) / tiles;
     if (segs > T / 64) segs = T / 64;
     if (segs > 64) segs = 64;
     if (segs < 1) segs = 1;
