@@ -62,13 +62,13 @@ struct QueryRes {
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
 // alone: 228 us, of which about 190).  `idle`: those of the `kept` query
-// resources that no call is using.  A resident portfolio has a block from cudaMalloc,
-// since its d_L and d_packed are the caller's to map on a peer or to export to
-// another process, which a pool's memory does not allow.  `spare`: at most
-// kSpareBlocks such blocks, kSpareKeep bytes, of destroyed portfolios, for the
-// next of the same size (creating and destroying one at N = 600: 0.15 ms more
-// with a cudaMalloc and a cudaFree each time); pool_trim frees them.  `held`:
-// those that still wait for the device (block_release).
+// resources that no call is using.  A resident portfolio has a block from
+// cudaMalloc, since its d_L and d_packed are the caller's to map on a peer or to
+// export to another process, which a pool's memory does not allow.  `spare`: the
+// latest of the destroyed portfolios' blocks, at most kSpareBlocks and kSpareKeep
+// bytes, for the next of the same size (creating and destroying one at N = 600:
+// 0.15 ms more with a cudaMalloc and a cudaFree each time); pool_trim frees them.
+// `held`: those that still wait for the device (block_release).
 struct Block {
     void *p;
     size_t bytes;
@@ -139,6 +139,16 @@ static int get_ctx(DevCtx **out, int *dev_out)
     return RG_OK;
 }
 
+static void blocks_free(DevCtx &c, const std::vector<Block> &blocks)
+{
+    for (const Block &b : blocks)
+        if (cudaFree(b.p) != cudaSuccess) { // refused beside a stream capture
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lk(g_mu);
+            c.held.push_back(b);
+        }
+}
+
 // What the engine keeps on the current device but does not use goes back to
 // the driver.
 void pool_trim()
@@ -152,12 +162,7 @@ void pool_trim()
         if (c.pool) cudaMemPoolTrimTo(c.pool, 0);
         spare.swap(c.spare);
     }
-    for (const Block &b : spare)
-        if (cudaFree(b.p) != cudaSuccess) { // refused beside a stream capture
-            cudaGetLastError();
-            std::lock_guard<std::mutex> lk(g_mu);
-            c.held.push_back(b);
-        }
+    blocks_free(c, spare);
 }
 
 // One more try, after pool_trim, for an allocation that failed for want of
@@ -324,24 +329,24 @@ static void block_release(DevCtx *c, Block block)
     }
     if (block.p) done.push_back(block);
     if (done.empty()) return;
-    const bool idle = device_wait();
-    for (const Block &b : done) {
-        {
-            std::lock_guard<std::mutex> lk(g_mu);
-            size_t kept = b.bytes;
-            for (const Block &o : c->spare) kept += o.bytes;
-            const bool room = kept <= kSpareKeep && c->spare.size() < kSpareBlocks;
-            if (!idle || room) {
-                (idle ? c->spare : c->held).push_back(b);
-                continue;
-            }
-        }
-        if (cudaFree(b.p) != cudaSuccess) {
-            cudaGetLastError();
-            std::lock_guard<std::mutex> lk(g_mu);
-            c->held.push_back(b);
-        }
+    if (!device_wait()) {
+        std::lock_guard<std::mutex> lk(g_mu);
+        c->held.insert(c->held.end(), done.begin(), done.end());
+        return;
     }
+    std::vector<Block> old; // the oldest spare ones make room
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        c->spare.insert(c->spare.end(), done.begin(), done.end());
+        size_t bytes = 0, keep = 0;
+        for (; keep < c->spare.size() && keep < kSpareBlocks; keep++) {
+            bytes += c->spare[c->spare.size() - 1 - keep].bytes;
+            if (bytes > kSpareKeep) break;
+        }
+        old.assign(c->spare.begin(), c->spare.end() - (long)keep);
+        c->spare.erase(c->spare.begin(), c->spare.end() - (long)keep);
+    }
+    blocks_free(*c, old);
 }
 
 // A spare block of just this size, or a new one.

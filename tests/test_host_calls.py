@@ -115,6 +115,14 @@ def test_spare_portfolio_memory_is_bounded_and_given_back(fake, monkeypatch):
     assert [d for name, _, d in fake.log() if name == "cudaFree"] == [str(size)]
 
 
+def test_the_latest_portfolio_memory_is_the_spare_one(fake):
+    for n in list(range(10, 30)) + [70]:
+        _portfolio(n).close()
+    fake.reset()
+    _portfolio(70).close()
+    assert not {"cudaMalloc", "cudaFree"} & set(fake.names())
+
+
 def _run(**more):
     return riskgpu.run(np.zeros(20), np.eye(20), np.full(20, 0.05), riskgpu.make_query(1000, 3, **more))
 
