@@ -62,17 +62,7 @@ struct QueryRes {
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
 // alone: 228 us, of which about 190).  `idle`: those of the `kept` query
-// resources that no call is using.  A resident portfolio has a block from
-// cudaMalloc, since its d_L and d_packed are the caller's to map on a peer or to
-// export to another process, which a pool's memory does not allow.  `spare`: the
-// latest of the destroyed portfolios' blocks, at most kSpareBlocks and kSpareKeep
-// bytes, for the next of the same size (creating and destroying one at N = 600:
-// 0.15 ms more with a cudaMalloc and a cudaFree each time); pool_trim frees them.
-// `held`: those that still wait for the device (block_release).
-struct Block {
-    void *p;
-    size_t bytes;
-};
+// resources that no call is using.
 struct DevCtx {
     bool ready = false;
     int sm_count = 0;
@@ -80,12 +70,10 @@ struct DevCtx {
     cudaMemPool_t pool = nullptr;
     std::vector<QueryRes> idle;
     size_t kept = 0;
-    std::vector<Block> spare, held;
 };
 
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
 static constexpr size_t kKeptQueries = 8;
-static constexpr size_t kSpareBlocks = 8, kSpareKeep = 32u << 20;
 
 static std::mutex g_mu;
 static DevCtx g_ctx[64];
@@ -139,30 +127,14 @@ static int get_ctx(DevCtx **out, int *dev_out)
     return RG_OK;
 }
 
-static void blocks_free(DevCtx &c, const std::vector<Block> &blocks)
-{
-    for (const Block &b : blocks)
-        if (cudaFree(b.p) != cudaSuccess) { // refused beside a stream capture
-            cudaGetLastError();
-            std::lock_guard<std::mutex> lk(g_mu);
-            c.held.push_back(b);
-        }
-}
-
-// What the engine keeps on the current device but does not use goes back to
-// the driver.
+// What the pool of the current device keeps but does not use goes back to the
+// driver.
 void pool_trim()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    DevCtx &c = g_ctx[dev];
-    std::vector<Block> spare;
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        if (c.pool) cudaMemPoolTrimTo(c.pool, 0);
-        spare.swap(c.spare);
-    }
-    blocks_free(c, spare);
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (g_ctx[dev].pool) cudaMemPoolTrimTo(g_ctx[dev].pool, 0);
 }
 
 // One more try, after pool_trim, for an allocation that failed for want of
@@ -306,81 +278,30 @@ static int admit(size_t need, bool quiet = false)
 
 bool admits(size_t need) { return admit(need, true) == RG_OK; }
 
-// Waits for all work of the current device, also on streams of the caller's.
-// False where the wait is refused, as it is while a stream of the device is
-// being captured: nothing has been waited for then.
-static bool device_wait()
-{
-    if (cudaDeviceSynchronize() == cudaSuccess) return true;
-    cudaGetLastError();
-    return false;
-}
-
-// A resident portfolio's block becomes a spare one (or is freed) once no work
-// can use it.  Where the wait is refused it is held, with those before it,
-// until a later call of this function (at the next destruction or creation)
-// gets one.
-static void block_release(DevCtx *c, Block block)
-{
-    std::vector<Block> done;
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        done.swap(c->held);
-    }
-    if (block.p) done.push_back(block);
-    if (done.empty()) return;
-    if (!device_wait()) {
-        std::lock_guard<std::mutex> lk(g_mu);
-        c->held.insert(c->held.end(), done.begin(), done.end());
-        return;
-    }
-    std::vector<Block> old; // the oldest spare ones make room
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        c->spare.insert(c->spare.end(), done.begin(), done.end());
-        size_t bytes = 0, keep = 0;
-        for (; keep < c->spare.size() && keep < kSpareBlocks; keep++) {
-            bytes += c->spare[c->spare.size() - 1 - keep].bytes;
-            if (bytes > kSpareKeep) break;
-        }
-        old.assign(c->spare.begin(), c->spare.end() - (long)keep);
-        c->spare.erase(c->spare.begin(), c->spare.end() - (long)keep);
-    }
-    blocks_free(*c, old);
-}
-
-// A spare block of just this size, or a new one.
-static cudaError_t block_take(DevCtx *c, size_t bytes, void **p)
-{
-    block_release(c, Block{nullptr, 0});
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        for (size_t i = 0; i < c->spare.size(); i++)
-            if (c->spare[i].bytes == bytes) {
-                *p = c->spare[i].p;
-                c->spare.erase(c->spare.begin() + (long)i);
-                return cudaSuccess;
-            }
-    }
-    return device_alloc(p, bytes);
-}
-
+// A resident portfolio has memory from cudaMalloc: its d_L and d_packed are the
+// caller's to map on a peer or to export to another process, which a pool's
+// memory does not allow, and work on streams of the caller's may still read it.
+// cudaFree waits for that work, beside a stream capture too (allowed by the
+// relaxed mode).  A wait for the whole device, before the memory went to a pool
+// or to the next portfolio, is refused there and ends the capture: any thread's,
+// that of a batch being created as well.  Creating and destroying a portfolio at
+// N = 600 takes 725 us so (649 with the memory kept for the next one).
+//
 // A pooled portfolio (of one call, or of the plugin cache) goes back to the
-// pool: every call that used it has waited for its work.  A resident one may
-// still be in use on a stream of the caller's.
+// pool: every call that used it has waited for its work.
 static void portfolio_free(Portfolio *p)
 {
     if (!p) return;
-    if (p->d_block) {
+    if (p->d_block && p->pooled) {
         int dev = p->device;
         cudaGetDevice(&dev);
         if (dev != p->device) cudaSetDevice(p->device);
         DevCtx *c = nullptr;
-        if (get_ctx(&c, nullptr) == RG_OK) {
-            if (p->pooled) cudaFreeAsync(p->d_block, c->stream);
-            else block_release(c, Block{p->d_block, p->block_bytes});
-        }
+        if (get_ctx(&c, nullptr) == RG_OK) cudaFreeAsync(p->d_block, c->stream);
         if (dev != p->device) cudaSetDevice(dev);
+    } else if (p->d_block) {
+        RelaxedCapture relaxed;
+        cudaFree(p->d_block);
     }
     delete p;
 }
@@ -706,9 +627,8 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t ow32 = bp.take((size_t)n * sizeof(float));
         const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
-        p->block_bytes = bp.total;
         if (pooled) RG_CUDA_TRY(pool_take(ctx, &p->d_block, bp.total, s));
-        else RG_CUDA_TRY(block_take(ctx, bp.total, &p->d_block));
+        else RG_CUDA_TRY(device_alloc(&p->d_block, bp.total));
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
         p->d_L64 = reinterpret_cast<double *>(blk + oL64);
         p->d_mu64 = reinterpret_cast<double *>(blk + omu);

@@ -212,7 +212,6 @@ struct Portfolio {
     int has_w = 0;
     int device = 0;
     bool pooled = false;       // d_block is from the engine's pool (else from cudaMalloc)
-    size_t block_bytes = 0;
     void *d_block = nullptr;   // one allocation holding every device buffer below
     double *d_L64 = nullptr;   // n x n row-major, zero upper
     double *d_mu64 = nullptr;  // n

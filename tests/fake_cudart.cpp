@@ -260,7 +260,12 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return
 cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) { return handle("cudaStreamEndCapture", g); }
 cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m)
 {
-    return simple("cudaThreadExchangeStreamCaptureMode", nullptr, *m == cudaStreamCaptureModeRelaxed ? "relaxed" : "other");
+    static thread_local cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+    const cudaStreamCaptureMode was = mode;
+    mode = *m;
+    *m = was;
+    return simple("cudaThreadExchangeStreamCaptureMode", nullptr,
+                  mode == cudaStreamCaptureModeRelaxed ? "relaxed" : "other");
 }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *g, cudaGraph_t, unsigned long long)
 {

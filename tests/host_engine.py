@@ -15,8 +15,7 @@ import riskgpu
 from riskgpu import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-OOM = 2                 # cudaErrorMemoryAllocation
-CAPTURE_REFUSED = 900   # cudaErrorStreamCaptureUnsupported
+OOM = 2  # cudaErrorMemoryAllocation
 
 
 def link(folder):

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import riskgpu
-from host_engine import CAPTURE_REFUSED, OOM, fake, linked  # noqa: F401
+from host_engine import OOM, fake, linked  # noqa: F401
 
 
 def _create(n=8, bad=None):
@@ -40,87 +40,30 @@ def test_a_missing_device_stays_missing(fake):
     assert (st, h) == (riskgpu.RG_ERR_NO_DEVICE, None) and "no CUDA device" in message
 
 
-FREES = ("cudaFree", "cudaFreeAsync")
-LARGE = 2100  # a portfolio whose memory is not kept for the next one
-
-
 def _portfolio(n):
     return riskgpu.Portfolio(np.zeros(n), np.eye(n))
 
 
-@pytest.mark.parametrize("n", [70, LARGE])
-def test_a_portfolio_outlives_a_refused_wait(fake, n):
-    """Destroyed while a stream capture forbids waiting for the device: work
-    launched with it may be in flight, so its memory is not handed on until a
-    wait has succeeded, and is then."""
-    port = _portfolio(n)
-    one = fake.live()
-    fake.reset()
-    for name in ("cudaDeviceSynchronize", "cudaFree"):
-        fake.fail(name, CAPTURE_REFUSED, count=-1, until="cudaGetErrorString")
-    port.close()
-    assert fake.live() == one and "cudaFreeAsync" not in fake.names()
-    second = _portfolio(n)
-    assert fake.live() == 2 * one
-    fake.reset()  # the capture has ended
-    third = _portfolio(n)
-    names = fake.names()
-    free = [i for i, name in enumerate(names) if name in FREES and name != "cudaFreeAsync"]
-    assert "cudaDeviceSynchronize" in names[:free[0] if free else None]
-    assert fake.live() == 2 * one
-    second.close()
-    third.close()
-
-
-def test_resident_portfolios_own_plain_device_memory(fake):
+@pytest.mark.parametrize("n", [3, 70, 700])
+def test_resident_portfolios_own_plain_device_memory(fake, n):
     """d_L and d_packed are the caller's to map on a peer or to export to
-    another process, which memory of a pool does not allow."""
-    port = _portfolio(LARGE)
+    another process, which memory of a pool does not allow; work that reads
+    them may be in flight, which cudaFree waits for.  A wait for the whole
+    device would end a stream capture of any thread."""
+    port = _portfolio(n)
     size = max(int(d) for name, _, d in fake.log() if name == "cudaMalloc")
-    assert size >= LARGE * LARGE * 8
+    assert size >= n * n * 8
     fake.reset()
     port.close()
-    assert ("cudaFree", "0", str(size)) in fake.log() and fake.live() == 0
+    log = fake.log()
+    assert [d for name, _, d in log if name in ("cudaFree", "cudaFreeAsync")] == [str(size)] and fake.live() == 0
+    assert "cudaDeviceSynchronize" not in fake.names()
+    modes = [d for name, _, d in log[:fake.names().index("cudaFree")] if name == "cudaThreadExchangeStreamCaptureMode"]
+    assert modes == ["relaxed"]
     # a call's own portfolio is the engine's business
     fake.reset()
     riskgpu.run(np.zeros(70), np.eye(70), None, riskgpu.make_query(1000, 3))
     assert not [d for name, _, d in fake.log() if name == "cudaMalloc" and int(d) >= 70 * 70 * 8]
-
-
-def test_spare_portfolio_memory_is_bounded_and_given_back(fake, monkeypatch):
-    ports = [_portfolio(70) for _ in range(20)]
-    one = fake.live() // 20
-    for p in ports:
-        p.close()
-    assert fake.live() == 8 * one
-    fake.reset()
-    again = _portfolio(70)
-    assert "cudaMalloc" not in fake.names()
-    ports = [_portfolio(900 + 100 * i) for i in range(5)]
-    for p in ports + [again]:
-        p.close()
-    assert fake.live() <= 32 << 20
-    # an allocation that fails gets what is kept
-    fake.reset()
-    fake.fail("cudaMalloc", OOM, count=-1, until="cudaFree")
-    port = _portfolio(33)
-    size = fake.live()
-    port.close()
-    assert size < one
-    # and so does an admission check that would refuse
-    monkeypatch.setenv("RG_MEM_HEADROOM_BYTES", "1000")
-    fake.reset()
-    fake.free_bytes(0, 1 << 40)
-    _portfolio(20).close()
-    assert [d for name, _, d in fake.log() if name == "cudaFree"] == [str(size)]
-
-
-def test_the_latest_portfolio_memory_is_the_spare_one(fake):
-    for n in list(range(10, 30)) + [70]:
-        _portfolio(n).close()
-    fake.reset()
-    _portfolio(70).close()
-    assert not {"cudaMalloc", "cudaFree"} & set(fake.names())
 
 
 def _run(**more):
@@ -131,7 +74,7 @@ def _run(**more):
     ("cudaMallocFromPoolAsync", _run),
     ("cudaMallocFromPoolAsync", lambda: riskgpu.moments(np.ones((5, 3)))),
     ("cudaMallocFromPoolAsync", lambda: riskgpu.crash_frequency(np.ones((5, 3)), 0.02, 1)),
-    ("cudaMalloc", lambda: _portfolio(LARGE).close()),
+    ("cudaMalloc", lambda: _portfolio(20).close()),
     ("cudaMalloc", lambda: riskgpu.Batch([(_portfolio(20), riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))])),
 ])
 def test_what_the_engine_keeps_does_not_fail_an_allocation(fake, name, call):
