@@ -291,7 +291,10 @@ int rg_batch_create(const rg_batch_item *items, int32_t count, int32_t flags, rg
                            q.draw_mode == RG_DRAWS_AGGREGATED, p->wmu, tile);
         tile += tc_tiles_of(q.n_paths, paths);
     }
-    for (int i = 0; i < count; i++) b->queries.push_back(items[i].query);
+    for (int i = 0; i < count; i++) {
+        b->queries.push_back(items[i].query);
+        reinterpret_cast<const Portfolio *>(items[i].portfolio)->shared = true;
+    }
     b->total_tiles = tile;
     // on one stream: a copy from pageable memory may return once it is staged,
     // and cap_stream does not wait for the legacy stream

@@ -62,7 +62,13 @@ struct QueryRes {
 // back the rest).  From the device's default pool, which keeps nothing, every
 // call after a device synchronisation mapped its scratch anew (a 9-asset call
 // alone: 228 us, of which about 190).  `idle`: those of the `kept` query
-// resources that no call is using.
+// resources that no call is using.  `spare`: the latest blocks of resident
+// portfolios that were destroyed unshared (portfolio_free), at most kSpareBlocks
+// and kSpareKeep bytes, for the next of the same size.
+struct Block {
+    void *p;
+    size_t bytes;
+};
 struct DevCtx {
     bool ready = false;
     int sm_count = 0;
@@ -70,10 +76,12 @@ struct DevCtx {
     cudaMemPool_t pool = nullptr;
     std::vector<QueryRes> idle;
     size_t kept = 0;
+    std::vector<Block> spare;
 };
 
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
 static constexpr size_t kKeptQueries = 8;
+static constexpr size_t kSpareBlocks = 8, kSpareKeep = 32u << 20;
 
 static std::mutex g_mu;
 static DevCtx g_ctx[64];
@@ -127,14 +135,34 @@ static int get_ctx(DevCtx **out, int *dev_out)
     return RG_OK;
 }
 
-// What the pool of the current device keeps but does not use goes back to the
-// driver.
+// The calling thread's allocations and frees are allowed beside a stream capture
+// of another thread, as the rest of a call is.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static void blocks_free(const std::vector<Block> &blocks)
+{
+    if (blocks.empty()) return;
+    RelaxedCapture relaxed;
+    for (const Block &b : blocks) cudaFree(b.p);
+}
+
+// What the engine keeps on the current device but does not use goes back to
+// the driver.
 void pool_trim()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (g_ctx[dev].pool) cudaMemPoolTrimTo(g_ctx[dev].pool, 0);
+    std::vector<Block> spare;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (g_ctx[dev].pool) cudaMemPoolTrimTo(g_ctx[dev].pool, 0);
+        spare.swap(g_ctx[dev].spare);
+    }
+    blocks_free(spare);
 }
 
 // One more try, after pool_trim, for an allocation that failed for want of
@@ -167,14 +195,6 @@ int pool_alloc(void **p, size_t bytes, cudaStream_t s, cudaError_t *err)
     *err = pool_take(c, p, bytes, s);
     return RG_OK;
 }
-
-// The calling thread's allocations and frees are allowed beside a stream capture
-// of another thread, as the rest of a call is.
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 static void query_res_free(QueryRes &r, cudaStream_t s)
 {
@@ -284,8 +304,10 @@ bool admits(size_t need) { return admit(need, true) == RG_OK; }
 // cudaFree waits for that work, beside a stream capture too (allowed by the
 // relaxed mode).  A wait for the whole device, before the memory went to a pool
 // or to the next portfolio, is refused there and ends the capture: any thread's,
-// that of a batch being created as well.  Creating and destroying a portfolio at
-// N = 600 takes 725 us so (649 with the memory kept for the next one).
+// that of a batch being created as well.  Where no such work can be (`shared` is
+// not set: every call that used the portfolio has waited for its own) the block
+// is kept for the next portfolio of its size: create and destroy at N = 9 82 us
+// and at N = 600 570 us, shared 270 and 725.
 //
 // A pooled portfolio (of one call, or of the plugin cache) goes back to the
 // pool: every call that used it has waited for its work.
@@ -300,10 +322,37 @@ static void portfolio_free(Portfolio *p)
         if (get_ctx(&c, nullptr) == RG_OK) cudaFreeAsync(p->d_block, c->stream);
         if (dev != p->device) cudaSetDevice(dev);
     } else if (p->d_block) {
-        RelaxedCapture relaxed;
-        cudaFree(p->d_block);
+        std::vector<Block> out{Block{p->d_block, p->block_bytes}};
+        if (!p->shared) {
+            std::lock_guard<std::mutex> lk(g_mu);
+            std::vector<Block> &spare = g_ctx[p->device].spare;
+            spare.push_back(out[0]);
+            size_t keep = 0, bytes = 0; // the latest; the oldest make room
+            for (; keep < spare.size() && keep < kSpareBlocks; keep++) {
+                bytes += spare[spare.size() - 1 - keep].bytes;
+                if (bytes > kSpareKeep) break;
+            }
+            out.assign(spare.begin(), spare.end() - (long)keep);
+            spare.erase(spare.begin(), spare.end() - (long)keep);
+        }
+        blocks_free(out);
     }
     delete p;
+}
+
+// A spare block of just this size, or a new one.
+static cudaError_t block_take(DevCtx *c, size_t bytes, void **p)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        for (size_t i = 0; i < c->spare.size(); i++)
+            if (c->spare[i].bytes == bytes) {
+                *p = c->spare[i].p;
+                c->spare.erase(c->spare.begin() + (long)i);
+                return cudaSuccess;
+            }
+    }
+    return device_alloc(p, bytes);
 }
 
 // Offsets of a portfolio's device buffers inside its one allocation, each
@@ -628,7 +677,8 @@ static int create_portfolio(int32_t n, const double *mu, const double *sigma, in
         const size_t oaux = bp.take((cholesky_aux_len(n) + tc_scratch_len(n)) * sizeof(double)); // moments, scratch
         const size_t oinfo = bp.take(sizeof(int));
         if (pooled) RG_CUDA_TRY(pool_take(ctx, &p->d_block, bp.total, s));
-        else RG_CUDA_TRY(device_alloc(&p->d_block, bp.total));
+        else RG_CUDA_TRY(block_take(ctx, bp.total, &p->d_block));
+        p->block_bytes = bp.total;
         unsigned char *blk = static_cast<unsigned char *>(p->d_block);
         p->d_L64 = reinterpret_cast<double *>(blk + oL64);
         p->d_mu64 = reinterpret_cast<double *>(blk + omu);
@@ -738,6 +788,7 @@ int rg_portfolio_info_get(const rg_portfolio *h, rg_portfolio_info *out)
 {
     if (!h || !out) return set_error(RG_ERR_INVALID, "NULL argument");
     const Portfolio *p = reinterpret_cast<const Portfolio *>(h);
+    p->shared = true; // with the pointers below
     out->n_assets = p->n;
     out->has_weights = p->has_w;
     out->d_L = p->d_L64;
@@ -767,6 +818,7 @@ int rg_launch_counts(const rg_portfolio *h, const rg_query *q, unsigned long lon
     st = get_ctx(&ctx, nullptr);
     if (st) return st;
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+    p->shared = true; // not waited for
     cudaError_t e = cudaMemsetAsync(d_counts, 0, 2 * sizeof(unsigned long long), s);
     PlainArgs a = make_args(p, q, d_counts);
     // the block table lives for this launch, in stream order; a captured

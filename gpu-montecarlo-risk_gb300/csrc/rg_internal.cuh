@@ -16,6 +16,7 @@
 #pragma once
 
 #include <cstdint>
+#include <atomic>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -212,6 +213,11 @@ struct Portfolio {
     int has_w = 0;
     int device = 0;
     bool pooled = false;       // d_block is from the engine's pool (else from cudaMalloc)
+    size_t block_bytes = 0;
+    // Work that no call of the engine waits for may read d_block: a launch on a
+    // caller's stream, a batch or a server, or the caller's own (its pointers
+    // were handed out).  Set by every entry point that lets that happen.
+    mutable std::atomic<bool> shared{false};
     void *d_block = nullptr;   // one allocation holding every device buffer below
     double *d_L64 = nullptr;   // n x n row-major, zero upper
     double *d_mu64 = nullptr;  // n

@@ -181,8 +181,10 @@ using namespace rg;
 #define NA_TRY(call)                                                                               \
     do {                                                                                           \
         cudaError_t e_ = (call);                                                                   \
-        if (e_ != cudaSuccess)                                                                     \
+        if (e_ != cudaSuccess) {                                                                   \
+            p->shared = true; /* returns without waiting for its launches */                       \
             return set_error(RG_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_));         \
+        }                                                                                          \
     } while (0)
 
 extern "C" int rg_simulate_noalloc(const rg_portfolio *h, const rg_query *q, rg_result *out, void *stream)

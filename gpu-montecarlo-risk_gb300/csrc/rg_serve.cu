@@ -344,6 +344,7 @@ int rg_server_register(rg_server *h, int32_t portfolio_id, const rg_portfolio *p
     if (pp->n > max_n || tc_row_tiles_of(pp->n) > kServedMaxRowTiles || !pp->d_tc[0] || !pp->d_tc[1])
         return set_error(RG_ERR_UNSUPPORTED, "served portfolios are limited to N <= %d", max_n);
     std::lock_guard<std::mutex> lk(sv->mu);
+    pp->shared = true;
     sv->portfolios[portfolio_id] = pp;
     return RG_OK;
 }

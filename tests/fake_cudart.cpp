@@ -108,6 +108,7 @@ void fake_reset()
     std::lock_guard<std::mutex> lk(mu);
     text.clear();
     fails.clear();
+    last = cudaSuccess;
     free_list.clear();
     peak_bytes = live_bytes;
 }

@@ -53,6 +53,7 @@ def test_resident_portfolios_own_plain_device_memory(fake, n):
     port = _portfolio(n)
     size = max(int(d) for name, _, d in fake.log() if name == "cudaMalloc")
     assert size >= n * n * 8
+    port.info()
     fake.reset()
     port.close()
     log = fake.log()
@@ -66,6 +67,81 @@ def test_resident_portfolios_own_plain_device_memory(fake, n):
     assert not [d for name, _, d in fake.log() if name == "cudaMalloc" and int(d) >= 70 * 70 * 8]
 
 
+def _noalloc(port):
+    return riskgpu.lib().rg_simulate_noalloc(port.handle, ctypes.byref(riskgpu.make_query(1000, 3)),
+                                             ctypes.byref(riskgpu.Result()), None)
+
+
+SHARING = {
+    "info": lambda port: port.info(),
+    "launch_counts": lambda port: port.launch_counts(riskgpu.make_query(1000, 3), np.zeros(2).ctypes.data),
+    "noalloc": lambda port: _noalloc(port),
+    "batch": lambda port: riskgpu.Batch([(port, riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))]).close(),
+    "server": lambda port: riskgpu.lib().rg_server_register(SERVER[0]._h, 1, port.handle),
+}
+SERVER = []
+
+
+@pytest.mark.parametrize("how", SHARING)
+def test_memory_that_others_may_read_is_not_handed_on(fake, how):
+    """Work that no call waits for may still read a portfolio after these
+    calls: its memory is freed, which waits, and not kept for the next one."""
+    if how == "server":
+        SERVER.append(riskgpu.Server())
+    port = _portfolio(70)
+    if how == "noalloc":  # one that fails
+        fake.fail("cudaStreamSynchronize", 700)
+    SHARING[how](port)
+    fake.reset()
+    port.close()
+    assert "cudaFree" in fake.names()
+    fake.reset()
+    _portfolio(70)
+    assert "cudaMalloc" in fake.names()
+    while SERVER:
+        SERVER.pop().close()
+
+
+def test_spare_memory_is_bounded_and_given_back(fake, monkeypatch):
+    """Portfolios whose every call has waited leave their memory for the next
+    ones: the latest blocks, at most eight and 32 MiB."""
+    def use(n):
+        port = _portfolio(n)
+        port.factor()
+        if n <= 768:
+            port.simulate(riskgpu.make_query(1000, 3))
+            assert _noalloc(port) == riskgpu.RG_OK
+        return port
+
+    use(40).close()
+    rest = fake.live()  # and the kept query resources
+    fake.reset()
+    use(40).close()
+    assert not {"cudaMalloc", "cudaFree", "cudaDeviceSynchronize"} & set(fake.names())
+    ports = [use(70) for _ in range(20)]
+    one = (fake.live() - rest) // 20
+    for p in ports:
+        p.close()
+    assert fake.live() <= rest + 8 * one
+    for n in list(range(10, 30)) + [70]:
+        use(n).close()
+    fake.reset()
+    use(70).close()
+    assert not {"cudaMalloc", "cudaFree"} & set(fake.names())
+    for n in range(900, 1400, 100):
+        use(n).close()
+    assert fake.live() <= rest + (32 << 20)
+    # an allocation that fails, or an admission check that would refuse, gets them
+    fake.fail("cudaMalloc", OOM, count=-1, until="cudaFree")
+    use(33).close()
+    assert fake.live() < rest + one
+    monkeypatch.setenv("RG_MEM_HEADROOM_BYTES", "1000")
+    fake.reset()
+    fake.free_bytes(0, 1 << 40)
+    _portfolio(20)
+    assert "cudaFree" in fake.names()
+
+
 def _run(**more):
     return riskgpu.run(np.zeros(20), np.eye(20), np.full(20, 0.05), riskgpu.make_query(1000, 3, **more))
 
@@ -74,7 +150,7 @@ def _run(**more):
     ("cudaMallocFromPoolAsync", _run),
     ("cudaMallocFromPoolAsync", lambda: riskgpu.moments(np.ones((5, 3)))),
     ("cudaMallocFromPoolAsync", lambda: riskgpu.crash_frequency(np.ones((5, 3)), 0.02, 1)),
-    ("cudaMalloc", lambda: _portfolio(20).close()),
+    ("cudaMalloc", lambda: _portfolio(20).info()),
     ("cudaMalloc", lambda: riskgpu.Batch([(_portfolio(20), riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))])),
 ])
 def test_what_the_engine_keeps_does_not_fail_an_allocation(fake, name, call):
