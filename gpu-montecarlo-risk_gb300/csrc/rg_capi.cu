@@ -29,8 +29,11 @@ namespace rg {
 
 static thread_local char g_err[512] = "";
 
+// A runtime call's error is taken from the runtime as well: it keeps the last
+// one until it is asked, and the check after the next launch would find it.
 int set_error(int status, const char *fmt, ...)
 {
+    if (status == RG_ERR_CUDA || status == RG_ERR_NOMEM) cudaGetLastError();
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_err, sizeof(g_err), fmt, ap);

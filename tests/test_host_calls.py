@@ -236,3 +236,26 @@ def test_bad_input_is_reported_before_a_failed_creation(fake, name, err, status)
         fake.fail(name, err, count=-1)
         assert _create(bad=bad)[:2] == (status if bad is None else riskgpu.RG_ERR_INVALID, None)
         assert ("row 3" in riskgpu.lib().rg_last_error().decode()) == (bad is not None)
+
+
+@pytest.mark.parametrize("name,call", [
+    ("cudaMallocFromPoolAsync", _run),
+    ("cudaMalloc", lambda: _portfolio(20).info()),
+    ("cudaStreamSynchronize", _run),
+    ("cudaMallocFromPoolAsync", lambda: riskgpu.moments(np.ones((5, 3)))),
+    ("cudaMalloc", lambda: riskgpu.Batch([(_portfolio(20), riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))])),
+    ("cudaGraphInstantiate", lambda: riskgpu.Batch([(_portfolio(20),
+                                                     riskgpu.make_query(1000, 3, precision=riskgpu.PREC_FP16X3))])),
+])
+def test_a_failed_call_does_not_fail_the_next(fake, name, call):
+    """The runtime keeps the last error until it is asked for; the check after
+    the next launch must not find this one's."""
+    call()
+    for _ in range(2):
+        if "Malloc" in name:
+            fake.fail(name, OOM, count=2)  # and the second try
+        else:
+            fake.fail(name, 700)
+        with pytest.raises(riskgpu.RiskGpuError):
+            call()
+        call()
