@@ -4,7 +4,6 @@ device memory reads as zeros."""
 import contextlib
 import ctypes
 import gc
-import glob
 import os
 import shutil
 import subprocess
@@ -25,9 +24,9 @@ def link(folder):
     if not os.path.exists(os.path.join(include, "cuda_runtime_api.h")):
         include = "/usr/local/cuda/include"
     out = os.path.join(folder, "libriskgpu_host.so")
+    objects = [os.path.join(build.OUT, os.path.basename(c)[:-3] + ".o") for c in build._sources()[0]]
     subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I" + include, "-o", out,
-                    os.path.join(HERE, "fake_cudart.cpp")] + sorted(glob.glob(os.path.join(build.OUT, "*.o"))),
-                   check=True)
+                    os.path.join(HERE, "fake_cudart.cpp")] + objects, check=True)
     return out
 
 
