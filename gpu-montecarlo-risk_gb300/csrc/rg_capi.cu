@@ -873,9 +873,9 @@ int rg_simulate(const rg_portfolio *h, const rg_query *q, rg_result *out, void *
         const double se = std::sqrt(alpha * (1.0 - alpha) / (double)M) / dens;
         // standard errors either side: six with a thousand paths on both sides
         // of the quantile (a miss, answered by two more passes, once in 5e8
-        // queries), ten otherwise, where the order statistic is not yet normal.  The host sorts
-        // through the band: 1e6 paths at level 0.99, 2043 candidates and 67 us
-        // a call with ten, 1250 and 59 us with six
+        // queries), ten otherwise, where the order statistic is not yet normal.
+        // The host sorts through the band: 1e6 paths at level 0.99, 2043
+        // candidates and 67 us a call with ten, 1250 and 59 us with six
         const double half = (std::min(T, M - T) >= 1000 ? 6.0 : 10.0) * se + 1e-3 * sd;
         // RG_FAULT_INJECT=varband displaces the band by 5 sd (host-side
         // injection that exercises the histogram fallback)

@@ -291,7 +291,7 @@ __device__ __forceinline__ bool chol_wait(unsigned long long *bar)
 // Right-looking.  The chain warp, once column c - 1 is final and column c has
 // had every column before c - 2 applied, applies columns c - 2 and c - 1, forms
 // the pivot and leaves column c final: two FMAs, the reciprocal square root and
-// one multiply a column.  (With column c - 2 left to the bulk warps too, the
+// one multiply (FINE: and an FMA) a column.  (With column c - 2 left to the bulk warps too, the
 // chain waited for them 280 of 1220 cycles a column of a 32-column block
 // instead of 140 of 930.)  The bulk warps
 // (column j in the registers of bulk warp j mod 6, lane = row, two rows a lane
@@ -453,7 +453,7 @@ __device__ __forceinline__ void chol_factor_cta(int n, double *col, double *inv,
     }
 }
 
-// N <= 64: everything in one CTA (NC = 32 or 64).
+// N <= 64: everything in one CTA (NC = 16, 32, 48 or 64).
 template <int NC>
 __global__ void __launch_bounds__(kCholCta, 1) chol_small_kernel(
     const double *__restrict__ A, long long lda, int n, const double *__restrict__ w,
